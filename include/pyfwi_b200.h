@@ -138,7 +138,12 @@ typedef struct pyfwi_options {
                                kernels (many steps per launch, a grid barrier between steps)
                                where the layout allows: exact checkpoints holding every step in
                                FP32, the tile kernels (variants 0..2), the reference adjoint;
-                               otherwise (and inside a caller's stream capture) one launch per step */
+                               otherwise (and inside a caller's stream capture) one launch per step.
+                               2: resident time loops, one cooperative launch per run of steps
+                               and few shots with the wavefield kept on chip, where checkpoint
+                               segments hold difference sets in FP32 (store_diffs), no overlap is
+                               on, every source lies in the update domain and the grid fits on
+                               the SMs (up to about 600,000 cells); the step kernels otherwise */
     int32_t overlap;        /* 1: exact checkpoints in FP32 with recompute segments: recompute
                                segment m-1 on a second stream of the plan while the adjoint of
                                segment m runs (two segment buffers in the workspace) */
@@ -273,15 +278,17 @@ int pyfwi_launch_count(const pyfwi_plan *plan, int64_t *count);
 /* What the plan made of the options that apply only where its layout
  * allows: *flags bit 0 persistent time loops (options.persist), bit 1
  * recompute beside the adjoint (options.overlap), bit 2 difference sets in the
- * checkpoint segments (options.store_diffs).  No reference counterpart. */
+ * checkpoint segments (options.store_diffs), bit 3 resident time loops
+ * (options.persist 2).  No reference counterpart. */
 int pyfwi_plan_flags(const pyfwi_plan *plan, int32_t *flags);
 
 /* Read and clear the workspace's device error word after the work queued on
  * `stream` (synchronises that stream).  *code: 0 none, 1 a streaming kernel
  * gave up waiting (one second) for a row copy and left its rows unwritten,
  * 2 a streaming kernel found its shared memory misaligned for copies, 3 a
- * persistent kernel gave up waiting (one second) at a grid barrier and left
- * its remaining steps undone.
+ * persistent kernel gave up waiting (one second) at a grid barrier, or a
+ * resident one for a neighbour's halo, and left its remaining steps undone (a
+ * resident one leaves NaN in its results).
  * Returns PYFWI_E_TIMEOUT when *code != 0.  The reference has no device-side
  * waits and no counterpart. */
 int pyfwi_device_error(pyfwi_plan *plan, void *workspace, size_t bytes, int32_t *code, void *stream);

@@ -10,11 +10,11 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libpyfwi_b200.so")
-SOURCES = [os.path.join(HERE, "csrc", f) for f in ("pyfwi_b200.cu", "static_scratch.cu", "lowpass.cu")]
+SOURCES = [os.path.join(HERE, "csrc", f) for f in ("pyfwi_b200.cu", "static_scratch.cu", "lowpass.cu", "resident.cu", "resident8.cu")]
 DEPS = SOURCES + [os.path.join(HERE, "csrc", f) for f in os.listdir(os.path.join(HERE, "csrc"))] + \
     [os.path.join(ROOT, "include", "pyfwi_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC,-O3", "-shared", "-I" + os.path.join(ROOT, "include"),
+              "-Xcompiler", "-fPIC,-O3", "-shared", "-t", "4", "-I" + os.path.join(ROOT, "include"),
               "-I" + os.path.join(HERE, "csrc")]
 
 

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(NTHREADS) adj_persist(const __grid_constant__ 
 // Failure-path self test of the grid barrier: the CTAs of this launch wait
 // for one CTA more than there are, so the wait runs out after `limit_ns` and
 // sets the error word to 3, as a persistent kernel's would.
-__global__ void barrier_selftest_kernel(unsigned *bar, int *err, unsigned long long limit_ns)
+static __global__ void barrier_selftest_kernel(unsigned *bar, int *err, unsigned long long limit_ns)
 {
     grid_sync(bar, gridDim.x + 1, err, limit_ns);
 }

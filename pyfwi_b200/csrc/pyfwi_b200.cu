@@ -8,6 +8,7 @@
 #include "pyfwi_b200.h"
 #include "kernels.cuh"
 #include "persist_kernels.cuh"
+#include "resident.h"
 #include "stream_kernels.cuh"
 #include "tile_tma.cuh"
 
@@ -103,6 +104,9 @@ struct pyfwi_plan {
     int R, tz, st_w, ftma, atz, ast_w, ans, apf, chunk_opt, nacc, G, ngroups, seg, M, n_inj;  // a*: adjoint step variant
     bool exact_adj = false;  // PYFWI_ADJOINT_EXACT
     bool persist = false;    // time loops as persistent kernels (options.persist, where the layout allows)
+    bool resident = false;   // time loops with the wavefield on chip (options.persist 2, where it fits)
+    int sms = 0;             // SMs of the device the resident launches run on (0: not asked yet)
+    unsigned tag = 1;        // next unused tag of the exchange buffer in this call
     bool overlap = false;    // recompute of segment m-1 on a second stream beside the adjoint of segment m
     int qd = 0;              // the segment store holds the imaging's differences of each state (options.store_diffs):
                              // 1 in FP32, 2 in 24 bits (FP24 snapshots); 0 the states
@@ -111,7 +115,7 @@ struct pyfwi_plan {
     int fwd_cap = 0, adj_cap = 0;  // co-resident CTAs of the persistent kernels on this device
     long long state;  // floats per state (5 planes)
     // workspace offsets in bytes
-    size_t o_hdr, o_src, o_red, o_mat, o_dampx, o_dampz, o_work, o_adj, o_gacc, o_store, o_store16, o_store8, total;
+    size_t o_hdr, o_src, o_red, o_mat, o_dampx, o_dampz, o_work, o_adj, o_gacc, o_store, o_store16, o_store8, o_xch, total;
     long long launches = 0;
     bool model_set = false, fwd_valid = false;
     // per-kernel event timing (pyfwi_profile_enable)
@@ -820,11 +824,196 @@ int last_diffs(pyfwi_plan *p, void *ws, int m, int t_hi, int n, cudaStream_t st)
     return PYFWI_OK;
 }
 
+// ---- resident time loops -----------------------------------------------------
+// This call's time loops run with the wavefield on chip: the plan allows it,
+// the device has the SMs, and the stream is not being captured by the caller
+// (cooperative launches stay out of the caller's graphs).
+bool use_resident(pyfwi_plan *p, cudaStream_t st)
+{
+    if (!p->resident) return false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+    if (!p->sms) {
+        int dev = 0, sms = 0, coop = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return false;
+        p->sms = coop ? std::min(sms, RES_MAX_CTAS) : 1;
+    }
+    ResTiles tl;
+    return resident_tiles(p->g, p->R, p->lines, p->G, p->sms, false, &tl) &&
+           resident_tiles(p->g, p->R, p->lines, p->G, p->sms, true, &tl);
+}
+
+// A call's first use of the exchange buffer: no word holds a tag of this call.
+int clear_exchange(pyfwi_plan *p, void *ws, cudaStream_t st)
+{
+    CK(cudaMemsetAsync(at<char>(ws, p->o_xch), 0, RES_XCH_BYTES, st));
+    p->tag = 1;
+    return PYFWI_OK;
+}
+
+Buf slot_of(const Buf &b, int slot) { return {b.base + slot * b.stride, b.stride}; }
+
+// Forward steps [t0, t1) of slots c0 .. c0 + n - 1 of the group starting at
+// shot s0, from state `in` (slot 0's) to `out`; sets: their difference sets
+// (null: none), the first of which is that of step q_t0.  Several launches
+// when more source samples than travel with one are not zero.
+int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl, int t0, int t1, const Buf &in,
+                     const Buf &out, float *traces, const Buf *sets, int q_t0, cudaStream_t st)
+{
+    const pyfwi_geometry &G = p->geom;
+    FwdResArgs fa;
+    memset(&fa, 0, sizeof fa);
+    fa.a = base_step(p, ws);
+    fa.a.shot0 = s0 + c0;
+    fa.a.traces = traces;
+    fa.tl = tl;
+    fa.xch = at<uint4>(ws, p->o_xch);
+    fa.state = p->state;
+    fa.dt_scale = G.dt_scale;
+    fa.nt_ext = G.nt_ext;
+    fa.record = traces != nullptr;
+    fa.q_t0 = q_t0;
+    if (sets) {
+        fa.q = slot_of(*sets, c0).base;
+        fa.a.q_stride = sets->stride;
+    }
+    fa.err = at<int>(ws, ERR_OFF);
+    fa.limit_ns = BARRIER_WAIT_NS;
+    int last = (int)(p->src_vals.size() / 4) - 1;  // the last sample that adds anything
+    while (last >= 0 && !src_adds(src_at(p, last))) --last;
+    Buf from = in;
+    for (int t = t0; t < t1;) {
+        fa.k0 = t / G.dt_scale;
+        const int left = std::min(last, (t1 - 1) / G.dt_scale) - fa.k0 + 1;
+        fa.nk = std::max(0, std::min(left, RES_MAX_SAMPLES));
+        const int te = left > RES_MAX_SAMPLES ? (fa.k0 + RES_MAX_SAMPLES) * G.dt_scale : t1;
+        for (int q = 0; q < fa.nk; ++q) fa.wav[q] = src_at(p, fa.k0 + q);
+        const Buf to = te == t1 ? out : slot_of(work_state(p, ws, te & 1), c0);
+        fa.t0 = t;
+        fa.t1 = te;
+        fa.a.in = from.base;
+        fa.a.in_stride = from.stride;
+        fa.a.out = to.base;
+        fa.a.out_stride = to.stride;
+        fa.tag0 = p->tag;
+        p->tag += (unsigned)(te - t) + 1;
+        ProfileScope prof(p, st, 0, tl.nslots * (te - t));
+        cudaError_t e = launch_fwd_resident(fa, p->R, st);
+        if (e != cudaSuccess) return fail(PYFWI_E_CUDA, "resident forward launch: %s", cudaGetErrorString(e));
+        p->launches++;
+        from = to;
+        t = te;
+    }
+    return PYFWI_OK;
+}
+
+// Adjoint steps t_hi - 1 .. t_lo of a whole group with the sets of segment m,
+// from adjoint state `ping` to the other one.
+int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, int m, int t_hi, int t_lo, int &ping,
+                     float *adj, cudaStream_t st)
+{
+    const pyfwi_geometry &G = p->geom;
+    if (t_hi - 1 < t_lo) return PYFWI_OK;
+    AdjArgs a = base;
+    a.in = adj + (long long)ping * p->state;
+    a.in_stride = a.out_stride = 2 * p->state;
+    if (t_hi == G.nt) {  // later steps' residuals are added by the step before
+        a.inj_row = inj_row_of(p, G.nt - 1);
+        int rc = launch_inject(p, a, n, st);
+        if (rc) return rc;
+    }
+    const Buf sets = seg_state(p, ws, m, 0);
+    AdjResArgs r;
+    memset(&r, 0, sizeof r);
+    r.state = p->state;
+    r.t_hi = t_hi;
+    r.t_lo = t_lo;
+    r.nt = G.nt;
+    r.nt_ext = G.nt_ext;
+    r.dt_scale = G.dt_scale;
+    r.q_t0 = m * p->seg;
+    r.err = at<int>(ws, ERR_OFF);
+    r.limit_ns = BARRIER_WAIT_NS;
+    ResTiles tl;
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, true, &tl))
+        return fail(PYFWI_E_INVALID, "the adjoint does not fit on chip");
+    const int conc = tl.nslots;
+    for (int c0 = 0; c0 < n; c0 += conc) {
+        tl.nslots = std::min(conc, n - c0);
+        r.tl = tl;
+        r.a = a;
+        r.a.shot0 = base.shot0 + c0;
+        r.a.in = a.in + (long long)c0 * 2 * p->state;
+        r.a.out = adj + (long long)(1 - ping) * p->state + (long long)c0 * 2 * p->state;
+        r.a.gacc = base.gacc + c0 * base.gacc_stride;
+        r.a.fwd_stride = sets.stride;
+        r.q = slot_of(sets, c0).base;
+        r.xch = at<uint4>(ws, p->o_xch);
+        r.tag0 = p->tag;
+        p->tag += (unsigned)(t_hi - t_lo) + 1;
+        ProfileScope prof(p, st, 1, tl.nslots * (t_hi - t_lo));
+        cudaError_t e = launch_adj_resident(r, p->R, st);
+        if (e != cudaSuccess) return fail(PYFWI_E_CUDA, "resident adjoint launch: %s", cudaGetErrorString(e));
+        p->launches++;
+    }
+    ping = 1 - ping;
+    return PYFWI_OK;
+}
+
+// The forward pass of a group on chip: restart states, and the difference
+// sets of the last segment.
+int resident_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
+{
+    const int nt = p->geom.nt;
+    ResTiles tl;
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, false, &tl))
+        return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
+    int rc = clear_exchange(p, ws, st);
+    if (rc) return rc;
+    const int conc = tl.nslots;
+    const Buf sets = seg_state(p, ws, p->M - 1, 0);
+    for (int c0 = 0; c0 < n; c0 += conc) {
+        tl.nslots = std::min(conc, n - c0);
+        for (int m = 0; m < p->M; ++m) {
+            const int t0 = m * p->seg, t1 = std::min(t0 + p->seg, nt);
+            const bool last = m == p->M - 1;
+            const Buf in = slot_of(exact_state(p, ws, t0), c0);
+            const Buf out = slot_of(last ? work_state(p, ws, nt & 1) : exact_state(p, ws, t1), c0);
+            rc = resident_forward(p, ws, s0, c0, tl, t0, t1, in, out, traces, last ? &sets : nullptr, t0, st);
+            if (rc) return rc;
+        }
+    }
+    return last_diffs(p, ws, p->M - 1, nt, n, st);
+}
+
+// Recompute of segment m on chip: its difference sets.
+int resident_recompute(pyfwi_plan *p, void *ws, int s0, int n, int m, cudaStream_t st)
+{
+    const int t0 = m * p->seg, t1 = std::min(t0 + p->seg, p->geom.nt);
+    ResTiles tl;
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, false, &tl))
+        return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
+    const int conc = tl.nslots;
+    const Buf sets = seg_state(p, ws, m, 0);
+    Range range("pyfwi recompute segment");
+    for (int c0 = 0; c0 < n; c0 += conc) {
+        tl.nslots = std::min(conc, n - c0);
+        int rc = resident_forward(p, ws, s0, c0, tl, t0, t1, slot_of(exact_state(p, ws, t0), c0),
+                                  slot_of(work_state(p, ws, t1 & 1), c0), nullptr, &sets, t0, st);
+        if (rc) return rc;
+    }
+    return last_diffs(p, ws, m, t1, n, st);
+}
+
 int exact_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
 {
     Buf z = exact_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(z.base + q * z.stride, 0, p->state * sizeof(float), st));
     if (use_persist(p, st)) return persist_pass(p, ws, s0, n, traces, st);
+    if (use_resident(p, st)) return resident_pass(p, ws, s0, n, traces, st);
     StepArgs a = base_step(p, ws);
     a.shot0 = s0;
     a.traces = traces;
@@ -1213,6 +1402,19 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
         } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && p->overlap) {
             rc = overlap_backward(p, ws, a, s0, n, t_src, ping, adj, st);
             if (rc) return rc;
+        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && use_resident(p, st)) {
+            rc = clear_exchange(p, ws, st);
+            if (rc) return rc;
+            for (int m = p->M - 1; m >= 0; --m) {
+                const int t_lo = m * p->seg, t_hi = std::min((m + 1) * p->seg, G.nt);
+                if (m < p->M - 1) {
+                    rc = resident_recompute(p, ws, s0, n, m, st);
+                    if (rc) return rc;
+                }
+                Range range("pyfwi adjoint segment");
+                rc = resident_adjoint(p, ws, a, n, m, t_hi, std::max(t_lo, 1), ping, adj, st);
+                if (rc) return rc;
+            }
         } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT) {
             StepArgs f = base_step(p, ws);
             f.shot0 = s0;
@@ -1519,7 +1721,7 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     p->n_inj = (G.nt + G.dt_scale - 1) / G.dt_scale;
     // persistent time loops: every step stored in FP32 (one segment), tile
     // kernels with one shot per adjoint CTA, the reference adjoint
-    p->persist = opt->persist && opt->checkpoint == PYFWI_CKPT_EXACT && p->M == 1 &&
+    p->persist = opt->persist && opt->persist != 2 && opt->checkpoint == PYFWI_CKPT_EXACT && p->M == 1 &&
                  opt->snapshot == PYFWI_SNAP_FP32 && !p->exact_adj && !p->st_w && !p->ftma && !p->ast_w &&
                  p->ans == 1;
     if (p->persist) p->opt.graph = 0;  // a few launches per call: nothing to replay
@@ -1534,6 +1736,15 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
                     p->nacc == 3 && !p->persist && !p->st_w && !p->ftma && !p->ast_w && p->ans == 1 && !p->apf &&
                     G.npml + p->R >= 4;  // whole 4-column groups are written: the imaged columns end 3 short of tnx
     p->qd = qd ? (opt->snapshot == PYFWI_SNAP_FP24 ? 2 : 1) : 0;
+    // resident time loops: difference sets on one stream, tiles that fit on chip
+    ResTiles tl;
+    bool src_in = true;  // every source inside the update domain
+    for (int s = 0; s < G.ns; ++s)
+        src_in = src_in && srcz[s] >= p->R && srcz[s] <= tnz - p->R && srcx[s] >= p->R && srcx[s] <= tnx - p->R;
+    p->resident = opt->persist == 2 && p->qd == 1 && !p->overlap && src_in &&
+                  resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, false, &tl) &&
+                  resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, true, &tl);
+    if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
 
     const size_t pf = (size_t)p->g.plane * sizeof(float), sb = (size_t)p->state * sizeof(float);
     // regions holding planes start on a row of the workspace (a multiple of
@@ -1575,6 +1786,8 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     if (bf16_snaps(p)) o += up((size_t)p->seg * p->state * sizeof(__nv_bfloat16) * p->G);
     p->o_store8 = o;
     if (fp24_snaps(p)) o += up((size_t)p->seg * p->state * p->G);
+    p->o_xch = o;
+    if (p->resident) o += up(RES_XCH_BYTES);
     p->total = o;
     *out = p;
     return PYFWI_OK;
@@ -1646,7 +1859,7 @@ int pyfwi_launch_count(const pyfwi_plan *p, int64_t *count)
 int pyfwi_plan_flags(const pyfwi_plan *p, int32_t *flags)
 {
     if (!p || !flags) return fail(PYFWI_E_INVALID, "NULL argument");
-    *flags = (p->persist ? 1 : 0) | (p->overlap ? 2 : 0) | (p->qd ? 4 : 0);
+    *flags = (p->persist ? 1 : 0) | (p->overlap ? 2 : 0) | (p->qd ? 4 : 0) | (p->resident ? 8 : 0);
     return PYFWI_OK;
 }
 

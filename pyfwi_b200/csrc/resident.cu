@@ -1,0 +1,85 @@
+// Tilings of the resident time loops, and those of the fourth-order stencils
+// (resident8.cu has the eighth-order ones).
+#include "resident_launch.cuh"
+
+#include <algorithm>
+
+namespace pyfwi {
+
+template cudaError_t launch_fwd_resident_r<2>(FwdResArgs &a, cudaStream_t s);
+template cudaError_t launch_adj_resident_r<2>(AdjResArgs &a, cudaStream_t s);
+extern template cudaError_t launch_fwd_resident_r<4>(FwdResArgs &a, cudaStream_t s);
+extern template cudaError_t launch_adj_resident_r<4>(AdjResArgs &a, cudaStream_t s);
+
+namespace {
+
+constexpr size_t MAX_FLOATS = (232448 - 1024) / sizeof(float);  // 227 KB per CTA less the static words
+
+template <int R>
+bool fits(int th, int nq, int rb, int ctas, const Lines &lines, bool adjoint)
+{
+    using S = ResShape<R>;
+    const int halo = (th + 4 * R) * (nq + 2 * S::HG) - th * nq, slots = res_slots(R, lines, th, nq);
+    return th <= S::TH && nq <= S::NQ && (th / rb) * nq <= RES_THREADS && halo <= RES_HALO &&
+           ctas * frame_count(th, nq, 2 * R, S::HG) <= RES_MAX_STRIPS && slots <= RES_MAX_SLOTS &&
+           (!adjoint || ADJ_RES_FLOATS<R> + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
+}
+
+static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_FLOATS, "the forward loop fits on an SM");
+
+}  // namespace
+
+// The tiling with the least modelled time of `shots` shots, in launches of c
+// shots each on sms / c tiles.  Few rows per block make a step short but a
+// launch small; many let one launch hold four times the cells.  The model of a
+// step (us) is a fit to launches of both orders on grids of 140 x 140 to 560 x
+// 1060 cells, each run with 1, 2 and 3 rows and 1 to 8 shots per launch; it is
+// within 10 % of all 36.  Measured, forward / adjoint, per step of all shots:
+// 8 shots of 240 x 440 take 19.2 / 25.8 us with 1 row one after another, 13.8
+// / 19.1 with 2 rows two at a time, 10.7 / 18.9 with 3 rows four at a time; 8
+// of 140 x 140 in one launch 3.10 / 3.88 with 1 row, 4.25 / 7.33 with 3.
+bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms, bool adjoint, ResTiles *out)
+{
+    struct Cost {
+        double step, row, warp_row, ring, row3;  // fixed; per row; per warp of blocks and row; per warp of ring items; with 3 rows
+    };
+    constexpr Cost COST[2][2] = {{{1.48, 0.64, 0.072, 0.021, 0.0}, {0.26, 0.35, 0.0, 1.02, 2.54}},
+                                 {{2.62, 0.96, 0.0, 0.15, 0.0}, {4.73, 0.0, 0.139, 0.0, 4.80}}};
+    const Cost &k = COST[R > 2][adjoint];
+    const int ncg = (g.tnx + 3) / 4, hg = R <= 2 ? 1 : 2;
+    double best = 0;
+    if (g.tnz < 4 * R || g.tnx < 4 * R) return false;
+    for (int rb = 1; rb <= 3; ++rb) {
+        const int nbz = (g.tnz + rb - 1) / rb;
+        for (int c = 1; c <= std::min(shots, sms); ++c) {
+            const int most = sms / c, waves = (shots + c - 1) / c;
+            if (c > 1 && (shots + c - 2) / (c - 1) == waves) continue;  // as many launches with fewer shots each
+            for (int gz = 1; gz <= most && (gz == 1 || nbz / gz * rb >= 2 * R); ++gz) {
+                const int gx = std::min(most / gz, std::max(1, ncg / hg));
+                const int bz = (nbz + gz - 1) / gz, nq = (ncg + gx - 1) / gx, th = rb * bz;
+                if (!(R == 2 ? fits<2>(th, nq, rb, c * gz * gx, lines, adjoint) : fits<4>(th, nq, rb, c * gz * gx, lines, adjoint)))
+                    continue;
+                const double ring = (double)(th + 2 * R) * (nq + 2) - (double)th * nq;
+                const double cost = waves * (k.step + rb * (k.row + k.warp_row * bz * nq / 32.0) + k.ring * ring / 32.0 +
+                                             (rb == 3 ? k.row3 : 0.0));
+                if (best == 0 || cost < best) {
+                    best = cost;
+                    *out = {gz, gx, c, rb, nbz, ncg, bz, nq};
+                }
+            }
+        }
+    }
+    return best > 0;
+}
+
+cudaError_t launch_fwd_resident(FwdResArgs &a, int R, cudaStream_t s)
+{
+    return R == 2 ? launch_fwd_resident_r<2>(a, s) : launch_fwd_resident_r<4>(a, s);
+}
+
+cudaError_t launch_adj_resident(AdjResArgs &a, int R, cudaStream_t s)
+{
+    return R == 2 ? launch_adj_resident_r<2>(a, s) : launch_adj_resident_r<4>(a, s);
+}
+
+}  // namespace pyfwi

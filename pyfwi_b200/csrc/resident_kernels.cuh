@@ -1,0 +1,1304 @@
+// Time loops with the wavefield resident on chip.
+//
+// A step kernel reads and writes every field of every cell from memory once
+// per time step (40 bytes and more per cell and shot), and a small survey's
+// step is a few microseconds of launch and latency.  Here one cooperative
+// launch runs a whole run of consecutive steps of a few shots: the grid of
+// each shot is cut into gz x gx tiles, one CTA per SM owns one tile for all
+// steps, and each of its computing threads owns a block of RB rows x 4
+// columns of it.  A thread keeps its block's fields (and forward the
+// materials) in registers; shared memory holds the copies that neighbouring
+// blocks difference.  Per step a CTA
+//   * computes the ring of cells around its tile that its neighbours also
+//     compute (the velocity ring forward, the stress ring backward), so one
+//     halo exchange per step is enough: the outermost 2R rows and columns of
+//     three stress planes forward, of the two velocity products backward;
+//   * writes those strips to a global exchange buffer (two alternate by step
+//     parity) in 16-byte words of three values and the step's tag;
+//   * reads its up to eight neighbours' words until their tags match and puts
+//     the values into its halo (a few words per thread: a warp or two of their
+//     own took 4000 to 9000 cycles a step for a tile of 81 x 52 cells).
+// The tag travels with the data (one 16-byte access is a single transaction),
+// so there is neither a flag nor a fence: a release of a flag word waits until
+// everything the SM has written is in L2, the difference sets included, which
+// measured 4000 (100 x 100 survey) to 11000 cycles a step (500 x 1000).
+// What is left of the memory traffic is the imaging's difference sets (20
+// bytes per imaged cell, written forward, read backward).
+//
+// Measured, forward / adjoint per step of all shots, against one launch per
+// step: 500 x 1000 cells and 4 shots 50.8 / 59.2 -> 23.0 / 44.4 us; whole
+// gradients of 100 x 100 cells, 4 shots, 500 steps 7.1 -> 2.9 ms, and of 200 x
+// 400 cells, 10 shots, 400 steps 24 -> 13.7 ms.
+//
+// The arithmetic is that of fwd_step / adj_step, operation for operation:
+// the results are the step kernels' bits, whatever the tiling.
+//
+// Every wait is bounded by p.limit_ns of the global timer: a CTA that gives
+// up sets the workspace error word to 3 and stops, and so does every CTA that
+// finds the word set when it starts or while it waits.  A CTA that stops
+// leaves NaN in its states, its remaining samples and its gradient
+// accumulators, so that no caller mistakes the results for good ones.
+#pragma once
+
+#include "persist_kernels.cuh"
+
+namespace pyfwi {
+
+// Threads of a CTA, a block each: 12 warps leave 168 registers a thread.
+constexpr int RES_THREADS = 384;
+constexpr int RES_HALO = RES_THREADS; // halo groups of a tile, at most: one thread fetches at most a group's words
+constexpr int RES_MAX_CTAS = 148;     // CTAs of a launch: the SMs of a B200
+constexpr int RES_MAX_STRIPS = 65536; // strip groups of all CTAs (a word's index takes 18 bits)
+constexpr int RES_PAD = 8;            // floats before the first plane: edge groups read past a row's start
+// Every shared plane has the same row stride and size, known when compiling:
+// a thread addresses its neighbours in all of them by one register and
+// immediate offsets.
+constexpr int RES_W = 60, RES_ROWS = 92, RES_PLANE = RES_W * RES_ROWS;
+constexpr int RES_NAN = 0x7fc00000;    // what a loop that gave up leaves
+constexpr int RES_MAX_SLOTS = 1000;   // 4-cell groups with receivers of a CTA (10 bits)
+constexpr size_t RES_XCH_BYTES = 2ull * RES_MAX_STRIPS * 64;  // exchange buffer of a workspace
+constexpr int RES_MAX_SAMPLES = 1024; // source samples that travel as launch parameters
+
+// Tiles of a resident launch.  Rows are dealt out in blocks of rb; the last
+// block may reach past the grid, where nothing moves.
+struct ResTiles {
+    int gz, gx, nslots;  // tiles per shot down and across; shots of the launch (gz * gx * nslots CTAs)
+    int rb;              // rows of a thread's block
+    int nbz, ncg;        // block rows and 4-column groups of the grid
+    int bz, nq;          // block rows and groups of the largest tile
+};
+
+template <int R>
+struct ResShape {
+    static constexpr int HG = R <= 2 ? 1 : 2;  // halo groups (2R columns rounded up to 4)
+    static constexpr int HX = 4 * HG;
+    static constexpr int NQ = (RES_W - 2 * HX) / 4;  // most groups across a tile
+    static constexpr int TH = RES_ROWS - 4 * R;      // most rows
+    static constexpr int RING = 2 * R * (NQ + 2) + 2 * TH;  // most items of its ring
+    static constexpr int OW = 4 * NQ, OPLANE = OW * TH;     // planes of the tile alone
+    // every region of shared memory starts on a float4
+    static_assert(RES_W % 4 == 0 && RES_ROWS % 4 == 0 && RING % 4 == 0 && RES_PLANE % 4 == 0 && OPLANE % 4 == 0 &&
+                      RES_PAD % 4 == 0,
+                  "aligned regions");
+};
+
+// A rectangle of H x W items split into a frame (bz rows, bx columns thick)
+// and the inside; a rectangle with no inside is all frame.
+__host__ __device__ inline int frame_count(int H, int W, int bz, int bx)
+{
+    return H <= 2 * bz || W <= 2 * bx ? H * W : H * W - (H - 2 * bz) * (W - 2 * bx);
+}
+
+__device__ __forceinline__ void frame_item(int e, int H, int W, int bz, int bx, int &r, int &q)
+{
+    if (H <= 2 * bz || W <= 2 * bx) {
+        r = e / W;
+        q = e - r * W;
+        return;
+    }
+    const int band = bz * W;
+    if (e < 2 * band) {
+        r = e / W;
+        q = e - r * W;
+        if (e >= band) r += H - 2 * bz;
+        return;
+    }
+    e -= 2 * band;
+    r = bz + e / (2 * bx);
+    q = e % (2 * bx);
+    if (q >= bx) q += W - 2 * bx;
+}
+
+__device__ __forceinline__ void inner_item(int e, int W, int bz, int bx, int &r, int &q)
+{
+    const int w = W - 2 * bx;
+    r = bz + e / w;
+    q = bx + e % w;
+}
+
+__device__ __forceinline__ int frame_index(int r, int q, int H, int W, int bz, int bx)
+{
+    if (H <= 2 * bz || W <= 2 * bx) return r * W + q;
+    if (r < bz) return r * W + q;
+    if (r >= H - bz) return (r - H + 2 * bz) * W + q;
+    return 2 * bz * W + (r - bz) * 2 * bx + (q < bx ? q : q - W + 2 * bx);
+}
+
+constexpr unsigned ITEM_DAMP = 1u << 30;  // an item with damping on one of its cells
+__device__ __forceinline__ unsigned pack_item(int r, int q) { return (unsigned)r << 12 | (unsigned)q; }
+__device__ __forceinline__ int item_row(unsigned e) { return (int)((e >> 12) & 0xFFFu); }
+__device__ __forceinline__ int item_col(unsigned e) { return (int)(e & 0xFFFu); }
+
+struct FwdResArgs {
+    StepArgs a;        // constant fields; in / out: the states at t0 and t1
+    ResTiles tl;
+    uint4 *xch;        // exchange buffer: [parity][CTA][frame][4] words
+    unsigned tag0;     // tag of the strips of state s: tag0 + s - t0 (new to the buffer in every launch)
+    long long state;   // floats per state
+    int t0, t1;
+    int dt_scale, nt_ext, record;
+    float *q;          // difference sets of slot 0 (a.q_stride apart): the set of S_{t+1} at q + (t - q_t0) * state
+    int q_t0;
+    int *err;
+    unsigned long long limit_ns;
+    int k0, nk;        // samples k0 .. k0 + nk - 1 are in wav, the others are zero
+    float4 wav[RES_MAX_SAMPLES];
+};
+
+struct AdjResArgs {
+    AdjArgs a;         // constant fields; in / out: the adjoint states before step t_hi - 1 and after step t_lo
+    ResTiles tl;
+    uint4 *xch;
+    unsigned tag0;     // tag of the strips that step t reads: tag0 + t_hi - 1 - t
+    long long state;
+    int t_hi, t_lo;    // steps t_hi - 1 .. t_lo (t_lo >= 1)
+    int nt, nt_ext, dt_scale;
+    const float *q;    // the set of S_{t+1} at q + (t - q_t0) * state, slots a.fwd_stride apart
+    int q_t0;
+    int slots;         // 4-cell groups with receivers whose residuals a CTA stages
+    int *err;
+    unsigned long long limit_ns;
+};
+
+// Shared memory in floats.
+template <int R, int RB>
+constexpr int FWD_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 6 * ResShape<R>::RING + 2 * RES_ROWS + 2 * RES_W + 8 +
+                               4 * RES_MAX_SAMPLES + 4 * RES_THREADS;
+template <int R>
+constexpr int ADJ_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 5 * ResShape<R>::OPLANE + 22 * ResShape<R>::RING + 2 * RES_ROWS +
+                               3 * RES_W + 3 * RES_THREADS;
+constexpr int RES_SLOT_FLOATS = 44;  // and per slot of staged residuals (adjoint)
+
+// 16-byte words that are written and read as one transaction.
+__device__ __forceinline__ void st_word(uint4 *p, float a, float b, float c, unsigned tag)
+{
+    const unsigned long long lo = (unsigned long long)__float_as_uint(b) << 32 | __float_as_uint(a),
+                             hi = (unsigned long long)tag << 32 | __float_as_uint(c);
+    asm volatile("{\n.reg .b128 w;\nmov.b128 w, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], w;\n}\n" ::"l"(p), "l"(lo),
+                 "l"(hi)
+                 : "memory");
+}
+
+__device__ __forceinline__ uint4 ld_word(const uint4 *p)
+{
+    unsigned long long lo, hi;
+    asm volatile("{\n.reg .b128 w;\nld.relaxed.gpu.global.b128 w, [%2];\nmov.b128 {%0, %1}, w;\n}\n"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p)
+                 : "memory");
+    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+
+// Where a halo group of tile (tz, tx) comes from: the strip group of the CTA
+// that owns it, or ~0u outside the grid (where the halo stays zero).
+template <int R>
+__device__ __forceinline__ unsigned halo_source(const Grid &g, const ResTiles &tl, int frame, int slot, int tz, int tx,
+                                                int i0, int th, int q0, int nq, int gi, int gq)
+{
+    if (gi < 0 || gi >= g.tnz || gq < 0 || gq >= tl.ncg) return ~0u;
+    const int z = gi < i0 ? tz - 1 : gi >= i0 + th ? tz + 1 : tz, x = gq < q0 ? tx - 1 : gq >= q0 + nq ? tx + 1 : tx;
+    const int oi = tl.rb * (tl.nbz * z / tl.gz), oh = tl.rb * (tl.nbz * (z + 1) / tl.gz) - oi;
+    const int oq = tl.ncg * x / tl.gx, ow = tl.ncg * (x + 1) / tl.gx - oq;
+    return (unsigned)(((slot * tl.gz + z) * tl.gx + x) * frame + frame_index(gi - oi, gq - oq, oh, ow, 2 * R, ResShape<R>::HG));
+}
+
+// A thread's halo words (W in all: a group has W): where each lies in the
+// exchange buffer (18 bits) and where its values go (14 bits); ~0u: none.
+template <int R, int W>
+__device__ __forceinline__ void halo_words(unsigned *word, const Grid &g, const ResTiles &tl, int frame, int slot, int tz, int tx,
+                                           int i0, int th, int q0, int nq)
+{
+    constexpr int HG = ResShape<R>::HG;
+    const int n = W * ((th + 4 * R) * (nq + 2 * HG) - th * nq);
+#pragma unroll 1
+    for (int u = threadIdx.x; u < W * RES_THREADS; u += RES_THREADS) {
+        word[u] = ~0u;
+        if (u >= n) continue;
+        int r, q;
+        frame_item(u / W, th + 4 * R, nq + 2 * HG, 2 * R, HG, r, q);
+        const unsigned src = halo_source<R>(g, tl, frame, slot, tz, tx, i0, th, q0, nq, i0 - 2 * R + r, q0 - HG + q);
+        if (src != ~0u) word[u] = (4 * src + u % W) << 14 | (unsigned)(r * RES_W + 4 * q);
+    }
+}
+
+// Each of the words read until its tag is `tag`, then handed to put(offset,
+// word of the group, value).  False when the wait gave up (error word set,
+// here or by another CTA).
+template <int W, class Put>
+__device__ __forceinline__ bool fetch_halo(const uint4 *buf, unsigned tag, const unsigned *words, int *err,
+                                           unsigned long long limit_ns, Put put)
+{
+    unsigned long long t0 = 0;
+    unsigned open = 0, word[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        word[k] = words[k * RES_THREADS + threadIdx.x];
+        if (word[k] != ~0u) open |= 1u << k;
+    }
+    for (unsigned n = 1; open; ++n) {
+        uint4 v[W];
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if (open >> k & 1) v[k] = ld_word(buf + (word[k] >> 14));
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if ((open >> k & 1) && v[k].w == tag) {
+                open &= ~(1u << k);
+                put((int)(word[k] & 0x3FFFu), (int)(word[k] >> 14 & 3u), v[k]);
+            }
+        if (open && (n & 63u) == 0) {
+            if (ld_relaxed_gpu(err) != 0) return false;
+            if (!t0) {
+                t0 = global_ns();
+            } else if (global_ns() - t0 > limit_ns) {
+                atomicCAS(err, 0, 3);
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
+// A row of 4 own columns `c` with its neighbours in shared memory, in row12's
+// places (v[4 + k] is column k of the group at `row`): what forward (backward)
+// differences of the four read.
+template <int R, bool FWD>
+__device__ __forceinline__ void xrow(float (&v)[12], const float4 &c, const float *row)
+{
+    v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+    if constexpr (R == 2) {
+        v[0] = v[1] = v[10] = v[11] = 0.f;
+        if (FWD) {
+            const float2 r = *reinterpret_cast<const float2 *>(row + 4);
+            v[2] = 0.f;
+            v[3] = row[-1];
+            v[8] = r.x; v[9] = r.y;
+        } else {
+            const float2 l = *reinterpret_cast<const float2 *>(row - 2);
+            v[2] = l.x; v[3] = l.y;
+            v[8] = row[4];
+            v[9] = 0.f;
+        }
+    } else {
+        const float4 l = ld4s(row - 4), r = ld4s(row + 4);
+        v[0] = l.x; v[1] = l.y; v[2] = l.z; v[3] = l.w;
+        v[8] = r.x; v[9] = r.y; v[10] = r.z; v[11] = r.w;
+    }
+}
+
+// Rows of a window around the RB own rows of a plane that backward (FWD:
+// forward) z differences read: own(r) for row r of the block, the rows above
+// and below from shared memory (row 0 of the block at p, rows W apart).
+template <int R, int RB, bool FWD>
+struct ZWindow {
+    static constexpr int UP = FWD ? R - 1 : R, N = RB + 2 * R - 1;
+    float4 w[N];
+    template <class Own>
+    __device__ __forceinline__ ZWindow(Own own, const float *p)
+    {
+#pragma unroll
+        for (int m = 0; m < N; ++m) {
+            const int row = m - UP;
+            if (row >= 0 && row < RB)
+                w[m] = own(row);
+            else
+                w[m] = ld4s(p + row * RES_W);
+        }
+    }
+    // The difference at row r, column k, in the operation order of zbwd / zfwd.
+    __device__ __forceinline__ float at(int r, int k, const float *c) const
+    {
+        const int o = r + UP;
+        float s = FWD ? c[0] * (f4(w[o + 1], k) - f4(w[o], k)) : c[0] * (f4(w[o], k) - f4(w[o - 1], k));
+#pragma unroll
+        for (int q = 1; q < R; ++q)
+            s = FWD ? fmaf(c[q], f4(w[o + q + 1], k) - f4(w[o - q], k), s) : fmaf(c[q], f4(w[o + q], k) - f4(w[o - q - 1], k), s);
+        return s;
+    }
+};
+
+// The same window moving down row by row: the 2R rows that the difference at
+// the current row reads.
+template <int R, bool FWD>
+struct ZSlide {
+    static constexpr int UP = FWD ? R - 1 : R, DN = FWD ? R : R - 1;
+    float4 w[2 * R];
+    template <class Row>
+    __device__ __forceinline__ ZSlide(Row row)
+    {
+#pragma unroll
+        for (int m = 1; m < 2 * R; ++m) w[m] = row(m - 1 - UP);
+    }
+    __device__ __forceinline__ void next(const float4 &v)
+    {
+#pragma unroll
+        for (int m = 1; m < 2 * R; ++m) w[m - 1] = w[m];
+        w[2 * R - 1] = v;
+    }
+    __device__ __forceinline__ const float4 &centre() const { return w[UP]; }
+    __device__ __forceinline__ float at(int k, const float *c) const
+    {
+        float s = FWD ? c[0] * (f4(w[UP + 1], k) - f4(w[UP], k)) : c[0] * (f4(w[UP], k) - f4(w[UP - 1], k));
+#pragma unroll
+        for (int q = 1; q < R; ++q)
+            s = FWD ? fmaf(c[q], f4(w[UP + q + 1], k) - f4(w[UP - q], k), s)
+                    : fmaf(c[q], f4(w[UP + q], k) - f4(w[UP - q - 1], k), s);
+        return s;
+    }
+};
+
+// Difference values are written once and read once: streaming accesses.
+__device__ __forceinline__ void qst4s(float *q, float4 v) { __stcs(reinterpret_cast<float4 *>(q), v); }
+__device__ __forceinline__ float4 qld4s(const float *q)
+{
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(q));
+    return v;
+}
+__device__ __forceinline__ void qprefetch4(const float *q) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q)); }
+__device__ __forceinline__ float4 mk4(const float (&v)[4]) { return make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ float4 times4(const float4 &u, const float4 &v)
+{
+    return make_float4(u.x * v.x, u.y * v.y, u.z * v.z, u.w * v.w);
+}
+
+// Receivers k0 .. k0 + n - 1 of line l on rows [r0, r1), columns [c0, c1).
+__device__ __forceinline__ void line_range(const Lines &L, int l, int r0, int r1, int c0, int c1, int &k0, int &n)
+{
+    int lo, hi;  // first and one past the last receiver
+    if (L.drow[l] == 0) {
+        const int d = L.dcol[l];
+        lo = c0 > L.col0[l] ? (c0 - L.col0[l] + d - 1) / d : 0;
+        hi = c1 > L.col0[l] ? (c1 - 1 - L.col0[l]) / d + 1 : 0;
+        if (L.row0[l] < r0 || L.row0[l] >= r1) hi = lo;
+    } else {
+        const int d = L.drow[l];
+        lo = r0 > L.row0[l] ? (r0 - L.row0[l] + d - 1) / d : 0;
+        hi = r1 > L.row0[l] ? (r1 - 1 - L.row0[l]) / d + 1 : 0;
+        if (L.col0[l] < c0 || L.col0[l] >= c1) hi = lo;
+    }
+    if (hi > L.count[l]) hi = L.count[l];
+    k0 = lo;
+    n = hi > lo ? hi - lo : 0;
+}
+
+// The tile of this CTA.
+struct ResTile {
+    int slot, tz, tx, i0, th, q0, nq, j0;
+    int nblk, nin;  // blocks; the first nin reach neither the halo nor the strips
+};
+
+template <int R, int RB>
+__device__ __forceinline__ ResTile res_tile(const ResTiles &tl)
+{
+    constexpr int HG = ResShape<R>::HG, BZ = (2 * R + RB - 1) / RB;  // block rows that hold the strips
+    ResTile t;
+    const int per = tl.gz * tl.gx, tile = blockIdx.x % per;
+    t.slot = blockIdx.x / per;
+    t.tz = tile / tl.gx;
+    t.tx = tile - t.tz * tl.gx;
+    const int b0 = tl.nbz * t.tz / tl.gz, b1 = tl.nbz * (t.tz + 1) / tl.gz;
+    t.i0 = RB * b0;
+    t.th = RB * (b1 - b0);
+    t.q0 = tl.ncg * t.tx / tl.gx;
+    t.nq = tl.ncg * (t.tx + 1) / tl.gx - t.q0;
+    t.j0 = 4 * t.q0;
+    t.nblk = (b1 - b0) * t.nq;
+    t.nin = t.nblk - frame_count(b1 - b0, t.nq, BZ, HG);
+    return t;
+}
+
+// Block row and group of block e: the inside first, then the frame.
+template <int R, int RB>
+__device__ __forceinline__ void res_block(const ResTile &t, int e, int &bz, int &q)
+{
+    constexpr int BZ = (2 * R + RB - 1) / RB, HG = ResShape<R>::HG;
+    if (e < t.nin)
+        inner_item(e, t.nq, BZ, HG, bz, q);
+    else
+        frame_item(e - t.nin, t.th / RB, t.nq, BZ, HG, bz, q);
+}
+
+// ---------------------------------------------------------------------------
+// forward steps t0 .. t1 - 1 (fwd_step's arithmetic)
+// ---------------------------------------------------------------------------
+template <int R, int RB, int QD>
+__global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_constant__ FwdResArgs p)
+{
+    constexpr int NT = RES_THREADS, HX = ResShape<R>::HX, HG = ResShape<R>::HG;
+    extern __shared__ float4 smem4[];
+    __shared__ int s_stop, s_line[3][4];
+    const StepArgs &a = p.a;
+    const Grid &g = a.g;
+    const long long P = g.plane;
+    const int tid = threadIdx.x;
+    const ResTile T = res_tile<R, RB>(p.tl);
+    const int i0 = T.i0, j0 = T.j0, th = T.th, nq = T.nq;
+    constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING;
+    float *const sm = reinterpret_cast<float *>(smem4) + RES_PAD;
+    // Cell (r, c) of the tile lies at (r + 2R) * W + HX + c of every plane.
+    float *const s_txx = sm, *const s_tzz = sm + PL, *const s_txz = sm + 2 * PL, *const s_vx = sm + 3 * PL, *const s_vz = sm + 4 * PL;
+    float *const s_rb = sm + 5 * PL;                              // buoyancy of the ring's items
+    float *const s_dx = s_rb + 4 * RING, *const s_dz = s_dx + W;  // damping of columns j0 - HX .., rows i0 - 2R ..
+    float *const s_org = s_dz + RES_ROWS;                         // the source cell's stresses before the add
+    float4 *const s_wav = reinterpret_cast<float4 *>(s_org + 4);
+    unsigned *const t_ring = reinterpret_cast<unsigned *>(s_wav + RES_MAX_SAMPLES);
+    unsigned *const t_word = t_ring + RING;                       // the threads' halo words
+    const int frame = frame_count(RB * p.tl.bz, p.tl.nq, 2 * R, HG);  // strip groups of the largest tile
+    const int nring = (th + 2 * R) * (nq + 2) - th * nq;
+    const int shot = a.shot0 + T.slot;
+    const float dt = a.k.dt;
+    const float *in = a.in + T.slot * a.in_stride;
+    const int xpar = 4 * gridDim.x * frame;  // words per parity
+    uint4 *const strip = p.xch + 4 * blockIdx.x * frame;
+
+    // the tile with its halo, the ring's table and buoyancy, the damping
+    if (tid == 0) s_stop = ld_relaxed_gpu(p.err) != 0;
+    for (int e = tid; e < (th + 4 * R) * (nq + 2 * HG); e += NT) {
+        const int r = e / (nq + 2 * HG), q = e - r * (nq + 2 * HG), o = r * W + 4 * q;
+        const int gi = i0 - 2 * R + r, gj = j0 - HX + 4 * q;
+        cp4(s_txx + o, in + TXX * P, g, gi, gj);
+        cp4(s_tzz + o, in + TZZ * P, g, gi, gj);
+        cp4(s_txz + o, in + TXZ * P, g, gi, gj);
+        cp4(s_vx + o, in + VX * P, g, gi, gj);
+        cp4(s_vz + o, in + VZ * P, g, gi, gj);
+    }
+    for (int e = tid; e < p.nk; e += NT) s_wav[e] = p.wav[e];
+    // Outside the update domain nothing moves: zero materials there leave every
+    // field as it is (x + dt * (0 * y) = x; no source sits there).
+    auto masked = [&](const float *plane, int gi, int gj) {
+        float4 v = ld4(plane, g, gi, gj);
+        if (!in_domain(g, R, gi, gj)) v.x = 0.f;
+        if (!in_domain(g, R, gi, gj + 1)) v.y = 0.f;
+        if (!in_domain(g, R, gi, gj + 2)) v.z = 0.f;
+        if (!in_domain(g, R, gi, gj + 3)) v.w = 0.f;
+        return v;
+    };
+    auto row_damp = [&](int gi) { return gi + ZO >= 0 && gi + ZO < g.rows ? __ldg(a.dampz + gi + ZO) : 0.f; };
+    auto damped = [&](int gi, int gj) {
+        const float4 x = damp4(a.dampx, g, gj);
+        return row_damp(gi) != 0.f || x.x != 0.f || x.y != 0.f || x.z != 0.f || x.w != 0.f;
+    };
+    for (int e = tid; e < nring; e += NT) {
+        int r, q;
+        frame_item(e, th + 2 * R, nq + 2, R, 1, r, q);
+        t_ring[e] = pack_item(r, q) | (damped(i0 - R + r, j0 - 4 + 4 * q) ? ITEM_DAMP : 0u);
+        st4s(s_rb + 4 * e, masked(a.mat + 2 * P, i0 - R + r, j0 - 4 + 4 * q));
+    }
+    for (int e = tid; e < 4 * nq + 2 * HX; e += NT) {
+        const int c = j0 - HX + e + XO;
+        s_dx[e] = c >= 0 && c < g.pitch ? __ldg(a.dampx + c) : 0.f;
+    }
+    for (int e = tid; e < th + 4 * R; e += NT) s_dz[e] = row_damp(i0 - 2 * R + e);
+    if (tid < a.lines.n) {
+        // receivers of the tile, per line: how many, the first one's place and the stride in the
+        // planes, its trace column
+        const Lines &L = a.lines;
+        int k0, n;
+        line_range(L, tid, i0, min(i0 + th, g.tnz), j0, min(j0 + 4 * nq, g.tnx), k0, n);
+        const int r = L.row0[tid] + k0 * L.drow[tid] - i0, c = L.col0[tid] + k0 * L.dcol[tid] - j0;
+        s_line[tid][0] = n;
+        s_line[tid][1] = (r + 2 * R) * W + c + HX;
+        s_line[tid][2] = L.drow[tid] * W + L.dcol[tid];
+        s_line[tid][3] = shot * a.nr + L.slot0[tid] + k0;
+    }
+    cp_wait_all();
+    __syncthreads();
+
+    halo_words<R, 4>(t_word, g, p.tl, frame, T.slot, T.tz, T.tx, i0, th, T.q0, nq);
+    auto put = [&](int o, int c, const uint4 &w) {
+        s_txx[o + c] = __uint_as_float(w.x);
+        s_tzz[o + c] = __uint_as_float(w.y);
+        s_txz[o + c] = __uint_as_float(w.z);
+    };
+
+    // this thread's block
+    const bool mine = tid < T.nblk, inside = tid < T.nin;
+    int bz = 0, bq = 0;
+    if (mine) res_block<R, RB>(T, tid, bz, bq);
+    const int br = bz * RB;                                // its first row in the tile
+    const int ot = (br + 2 * R) * W + HX + 4 * bq;         // and its place in the planes
+    const int gi0 = i0 + br, gj0 = j0 + 4 * bq;
+    const int co = (gi0 + ZO) * g.pitch + gj0 + XO;        // its first cell in a plane
+    float4 vx[RB], vz[RB], sxx[RB], szz[RB], sxz[RB];
+    float4 b[RB], lam[RB], mu[RB];
+    bool damp = false;
+    unsigned img = 0;                                      // rows with imaged cells
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        vx[r] = vz[r] = sxx[r] = szz[r] = sxz[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        b[r] = lam[r] = mu[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!mine) continue;
+        const int gi = gi0 + r;
+        vx[r] = ld4s(s_vx + ot + r * W);
+        vz[r] = ld4s(s_vz + ot + r * W);
+        sxx[r] = ld4s(s_txx + ot + r * W);
+        szz[r] = ld4s(s_tzz + ot + r * W);
+        sxz[r] = ld4s(s_txz + ot + r * W);
+        b[r] = masked(a.mat + 2 * P, gi, gj0);
+        lam[r] = masked(a.mat, gi, gj0);
+        mu[r] = masked(a.mat + P, gi, gj0);
+        damp = damp || damped(gi, gj0);
+        if (QD && gi >= a.qlo && gi <= a.qhi_z && gj0 + 3 >= a.qlo && gj0 <= a.qhi_x) img |= 1u << r;
+    }
+
+    // The strip group of row r of the tile in this thread's column, -1: none.
+    auto strip_group = [&](int r) {
+        return r < 2 * R || r >= th - 2 * R || bq < HG || bq >= nq - HG ? frame_index(r, bq, th, nq, 2 * R, HG) : -1;
+    };
+
+    // the source cell: in the tile, or in its halo
+    const int si = __ldg(a.srcz + shot), sj = __ldg(a.srcx + shot);
+    const int s_r = si - i0 + 2 * R, s_c = sj - j0 + HX, so = s_r * W + s_c;
+    const bool src_t = s_r >= 0 && s_r < th + 4 * R && s_c >= 0 && s_c < 4 * nq + 2 * HX;
+    const bool src_own = si >= i0 && si < i0 + th && sj >= j0 && sj < j0 + 4 * nq;
+    const bool my_src = mine && si >= gi0 && si < gi0 + RB && sj >= gj0 && sj < gj0 + 4;
+
+    // This thread's receiver (a tile has fewer than there are threads): its place in the planes and its
+    // trace column.
+    int rec_o = -1;
+    bool rec_vzx = false;
+    float *rec_tr = a.traces;
+    for (int l = 0, e = tid; p.record && l < a.lines.n; e -= s_line[l++][0])
+        if (e >= 0 && e < s_line[l][0]) {
+            rec_o = s_line[l][1] + e * s_line[l][2];
+            rec_vzx = a.lines.vzx[l];
+            rec_tr += s_line[l][3] + e;
+        }
+    const int rec_row = a.ns * a.nr;
+    // Its traces of row `row`: the velocities (as soon as they are there), the stresses (before the next source).
+    auto record_v = [&](int row) {
+        float *tr = rec_tr + (long long)row * rec_row;
+        tr[0] = s_vx[rec_o];
+        tr[a.trace_plane] = rec_vzx ? s_vx[rec_o] : s_vz[rec_o];
+    };
+    auto record_t = [&](int row) {
+        float *tr = rec_tr + (long long)row * rec_row;
+        tr[2 * a.trace_plane] = s_txx[rec_o];
+        tr[3 * a.trace_plane] = s_tzz[rec_o];
+        tr[4 * a.trace_plane] = s_txz[rec_o];
+    };
+
+    // New velocities of the block; qi: the difference set of the input state (null: none).
+    auto velocity = [&](float *qi) {
+        {
+            const ZWindow<R, RB, false> z([&](int r) { return sxz[r]; }, s_txz + ot);  // Dz- txz
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                float x[12], s[4], n[4];
+                xrow<R, false>(x, sxx[r], s_txx + ot + r * W);  // Dx- txx
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    s[k] = xbwd<R>(x, k, a.k.cx) + z.at(r, k, a.k.cz);
+                    n[k] = f4(vx[r], k) + dt * (f4(b[r], k) * s[k]);
+                }
+                if (QD && qi && (img >> r & 1)) qst4s(qi + Q_TXS * P + co + r * g.pitch, mk4(s));
+                vx[r] = mk4(n);
+            }
+        }
+        {
+            const ZWindow<R, RB, true> z([&](int r) { return szz[r]; }, s_tzz + ot);  // Dz+ tzz
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                float x[12], s[4], n[4];
+                xrow<R, true>(x, sxz[r], s_txz + ot + r * W);  // Dx+ txz
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    s[k] = z.at(r, k, a.k.cz) + xfwd<R>(x, k, a.k.cx);
+                    n[k] = f4(vz[r], k) + dt * (f4(b[r], k) * s[k]);
+                }
+                if (QD && qi && (img >> r & 1)) qst4s(qi + Q_TZS * P + co + r * g.pitch, mk4(s));
+                vz[r] = mk4(n);
+            }
+        }
+        if (damp) {
+            const float4 dx = ld4s(s_dx + HX + 4 * bq);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const float dr = s_dz[br + r + 2 * R];
+                float nx[4], nz[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float d = f4(dx, k) + dr;
+                    nx[k] = f4(vx[r], k) + dt * (-d * f4(vx[r], k));
+                    nz[k] = f4(vz[r], k) + dt * (-d * f4(vz[r], k));
+                }
+                vx[r] = mk4(nx);
+                vz[r] = mk4(nz);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            st4s(s_vx + ot + r * W, vx[r]);
+            st4s(s_vz + ot + r * W, vz[r]);
+        }
+    };
+
+    // New velocities of ring item e.
+    auto ring = [&](int e) {
+        const unsigned item = t_ring[e];
+        const int r = item_row(item), q = item_col(item), c = (r + R) * W + HX - 4 + 4 * q;
+        const float4 ovx = ld4s(s_vx + c), ovz = ld4s(s_vz + c), bb = ld4s(s_rb + 4 * e), cxz = ld4s(s_txz + c);
+        float x[12], nx[4], nz[4];
+        const ZWindow<R, 1, false> zx([&](int) { return cxz; }, s_txz + c);
+        xrow<R, false>(x, ld4s(s_txx + c), s_txx + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) nx[k] = f4(ovx, k) + dt * (f4(bb, k) * (xbwd<R>(x, k, a.k.cx) + zx.at(0, k, a.k.cz)));
+        const ZWindow<R, 1, true> zz([&](int) { return ld4s(s_tzz + c); }, s_tzz + c);
+        xrow<R, true>(x, cxz, s_txz + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) nz[k] = f4(ovz, k) + dt * (f4(bb, k) * (zz.at(0, k, a.k.cz) + xfwd<R>(x, k, a.k.cx)));
+        if (item & ITEM_DAMP) {
+            const float4 dx = ld4s(s_dx + HX - 4 + 4 * q);
+            const float dr = s_dz[r + R];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float d = f4(dx, k) + dr;
+                nx[k] = nx[k] + dt * (-d * nx[k]);
+                nz[k] = nz[k] + dt * (-d * nz[k]);
+            }
+        }
+        st4s(s_vx + c, mk4(nx));
+        st4s(s_vz + c, mk4(nz));
+    };
+
+    // New stresses of the block; its strips to xo, the velocity differences to qo.
+    auto stress = [&](uint4 *xo, unsigned tag, float *qo) {
+        float4 hx[RB];  // Dx- vz
+        {               // normal stresses: Dx+ vx, Dz- vz (and, imaged, Dz+ vz)
+            const ZWindow<R, RB, false> zz([&](int r) { return vz[r]; }, s_vz + ot);
+            const ZWindow<R, RB, true> zi([&](int r) { return vz[r]; }, s_vz + ot);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                float x[12], ex[4], ez[4], h[4], oxx[4], ozz[4];
+                xrow<R, true>(x, vx[r], s_vx + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) ex[k] = xfwd<R>(x, k, a.k.cx);
+                xrow<R, false>(x, vz[r], s_vz + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    h[k] = xbwd<R>(x, k, a.k.cx);
+                    ez[k] = zz.at(r, k, a.k.cz);
+                }
+                hx[r] = mk4(h);
+                if (QD && (img >> r & 1)) {
+                    float *q = qo + co + r * g.pitch, s[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[k] = zi.at(r, k, a.k.cz) + h[k];
+                    qst4s(q + Q_DXP_VX * P, mk4(ex));
+                    qst4s(q + Q_DZM_VZ * P, mk4(ez));
+                    qst4s(q + Q_VZS * P, mk4(s));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {  // normal_pair_fwd, the damping apart
+                    const float l = f4(lam[r], k), m = f4(mu[r], k), l2m = l + 2.f * m;
+                    oxx[k] = __fmaf_rn(dt, __fmaf_rn(l2m, ex[k], __fmul_rn(l, ez[k])), f4(sxx[r], k));
+                    ozz[k] = __fmaf_rn(dt, __fmaf_rn(l, ex[k], __fmul_rn(l2m, ez[k])), f4(szz[r], k));
+                }
+                sxx[r] = mk4(oxx);
+                szz[r] = mk4(ozz);
+            }
+        }
+        const ZWindow<R, RB, true> zx([&](int r) { return vx[r]; }, s_vx + ot);  // Dz+ vx
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            float oxz[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) oxz[k] = f4(sxz[r], k) + dt * (f4(mu[r], k) * (f4(hx[r], k) + zx.at(r, k, a.k.cz)));
+            if (damp) {
+                const float4 dx = ld4s(s_dx + HX + 4 * bq);
+                const float dr = s_dz[br + r + 2 * R];
+                float oxx[4], ozz[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float d = f4(dx, k) + dr;
+                    oxx[k] = __fmaf_rn(dt, __fmul_rn(-d, f4(sxx[r], k)), f4(sxx[r], k));
+                    ozz[k] = __fmaf_rn(dt, __fmul_rn(-d, f4(szz[r], k)), f4(szz[r], k));
+                    oxz[k] = oxz[k] + dt * (-d * oxz[k]);
+                }
+                sxx[r] = mk4(oxx);
+                szz[r] = mk4(ozz);
+            }
+            sxz[r] = mk4(oxz);
+            if (!inside) {
+                const int s = strip_group(br + r);
+                if (s >= 0) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) st_word(xo + 4 * s + k, f4(sxx[r], k), f4(szz[r], k), oxz[k], tag);
+                }
+            }
+            st4s(s_txx + ot + r * W, sxx[r]);
+            st4s(s_tzz + ot + r * W, szz[r]);
+            st4s(s_txz + ot + r * W, sxz[r]);
+        }
+    };
+
+    int k = p.t0 / p.dt_scale, sub = p.t0 - k * p.dt_scale;  // sample index and position inside it
+    if (rec_o >= 0 && sub == 0 && k < p.nt_ext) record_v(k);
+    __syncthreads();
+    // ring items go to the threads without a block first, then to those inside
+    const int rank = tid >= T.nblk ? tid - T.nblk : tid + NT - T.nblk;
+    bool stop = s_stop;
+    for (int t = p.t0; t < p.t1 && !stop; ++t) {
+        if (rec_o >= 0 && sub == 0 && k < p.nt_ext) record_t(k);
+        // this step's source sample, where it reaches the tile (uniform over the CTA)
+        float4 src = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (src_t && sub == 0 && k >= p.k0 && k - p.k0 < p.nk) src = s_wav[k - p.k0];
+        const bool add = src.x != 0.f || src.y != 0.f || src.z != 0.f || src.w != 0.f;
+        float *qi = nullptr, *qo = nullptr;
+        if constexpr (QD) {
+            qo = p.q + (long long)(t - p.q_t0) * p.state + T.slot * a.q_stride;
+            if (t > p.q_t0) qi = qo - p.state;
+        }
+        if (add) {
+            __syncthreads();
+            if (tid == 0) {
+                if (src_own) {
+                    s_org[0] = s_txx[so];
+                    s_org[1] = s_tzz[so];
+                    s_txx[so] += src.z;
+                    s_tzz[so] += src.w;
+                }
+                s_vx[so] += src.x;  // outside the ring: not read
+                s_vz[so] += src.y;
+            }
+            __syncthreads();
+            if (my_src) {  // the block's own copies
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    vx[r] = ld4s(s_vx + ot + r * W);
+                    vz[r] = ld4s(s_vz + ot + r * W);
+                    sxx[r] = ld4s(s_txx + ot + r * W);
+                    szz[r] = ld4s(s_tzz + ot + r * W);
+                }
+            }
+        }
+        // velocities: the blocks inside, then, with the halo, the others
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 1) {
+                if (t > p.t0) {  // the neighbours' strips of S_t
+                    if (!fetch_halo<4>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t - p.t0), t_word, p.err, p.limit_ns, put))
+                        s_stop = 1;
+                    __syncthreads();
+                    stop = s_stop;
+                    if (stop) break;
+                }
+                if (add && !src_own) {
+                    if (t == p.t0) __syncthreads();
+                    if (tid == 0) {
+                        s_org[0] = s_txx[so];
+                        s_org[1] = s_tzz[so];
+                        s_txx[so] += src.z;
+                        s_tzz[so] += src.w;
+                    }
+                    __syncthreads();
+                }
+            }
+            if (mine && inside == (pass == 0)) velocity(qi);
+        }
+        if (stop) break;
+        for (int e = rank; e < nring; e += NT) ring(e);
+        if constexpr (QD) {
+            // the stress differences near the source cell again, without this
+            // step's source (see fwd_step)
+            if (qi && add) {
+                __syncthreads();
+                if (tid < 4 * R) {
+                    const int gi = tid < 2 * R ? si : si - R + (tid - 2 * R), gj = tid < 2 * R ? sj - R + 1 + tid : sj;
+                    if (gi >= i0 && gi < i0 + th && gi < g.tnz && gj >= j0 && gj < j0 + 4 * nq && gj < g.tnx) {
+                        const long long sc = so;
+                        const float oxx = s_org[0], ozz = s_org[1];
+                        auto lxx = [&](long long m) { return m == sc ? oxx : s_txx[m]; };
+                        auto lzz = [&](long long m) { return m == sc ? ozz : s_tzz[m]; };
+                        auto lxz = [&](long long m) { return s_txz[m]; };
+                        const long long c = (gi - i0 + 2 * R) * W + gj - j0 + HX;
+                        const long long o = cell_off(g, gi, gj);
+                        qi[Q_TXS * P + o] = lbwd<R>(lxx, c, 1, a.k.cx) + lbwd<R>(lxz, c, W, a.k.cz);
+                        qi[Q_TZS * P + o] = lfwd<R>(lzz, c, W, a.k.cz) + lfwd<R>(lxz, c, 1, a.k.cx);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (mine) stress(strip + ((t + 1) & 1) * xpar, p.tag0 + (unsigned)(t + 1 - p.t0), qo);
+        if (rec_o >= 0 && t + 1 < p.t1 && sub + 1 == p.dt_scale && k + 1 < p.nt_ext) record_v(k + 1);
+        if (++sub == p.dt_scale) {
+            sub = 0;
+            ++k;
+        }
+        __syncthreads();
+    }
+    if (stop && rec_o >= 0)
+        for (; k < p.nt_ext; ++k)
+            for (int f = 0; f < 5; ++f)
+                rec_tr[f * a.trace_plane + (long long)k * a.ns * a.nr] = __int_as_float(RES_NAN);
+    if (!mine) return;
+    const float nan = __int_as_float(RES_NAN);
+    float *out = a.out + T.slot * a.out_stride;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        if (gi0 + r >= g.tnz) break;
+        if (stop) vx[r] = vz[r] = sxx[r] = szz[r] = sxz[r] = make_float4(nan, nan, nan, nan);
+        float *o = out + co + r * g.pitch;
+        *reinterpret_cast<float4 *>(o + VX * P) = vx[r];
+        *reinterpret_cast<float4 *>(o + VZ * P) = vz[r];
+        *reinterpret_cast<float4 *>(o + TXX * P) = sxx[r];
+        *reinterpret_cast<float4 *>(o + TZZ * P) = szz[r];
+        *reinterpret_cast<float4 *>(o + TXZ * P) = sxz[r];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// adjoint steps t_hi - 1 .. t_lo with imaging (adj_step's arithmetic)
+// ---------------------------------------------------------------------------
+// Each thread keeps its block's velocities and stresses in registers.  Shared memory holds what neighbouring blocks difference (b * Av
+// on the tile and its 2R halo; the sums of adj_sums and mu * Atxz on the tile
+// and its ring), the block's lam and mu and its three accumulators, and the
+// ring's stresses and materials.
+template <int R, int RB>
+__global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_constant__ AdjResArgs p)
+{
+    constexpr int NT = RES_THREADS, HX = ResShape<R>::HX, HG = ResShape<R>::HG;
+    extern __shared__ float4 smem4[];
+    __shared__ int s_stop, s_nslot, s_line[4][6];
+    const AdjArgs &a = p.a;
+    const Grid &g = a.g;
+    const long long P = g.plane;
+    const int tid = threadIdx.x;
+    const ResTile T = res_tile<R, RB>(p.tl);
+    const int i0 = T.i0, j0 = T.j0, th = T.th, nq = T.nq;
+    constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING, OW = ResShape<R>::OW, OP = ResShape<R>::OPLANE;
+    float *const sm = reinterpret_cast<float *>(smem4) + RES_PAD;
+    // Cell (r, c) of the tile lies at (r + 2R) * W + HX + c of the first five planes, at r * OW + c of the others.
+    float *const s_pvx = sm, *const s_pvz = sm + PL, *const s_px = sm + 2 * PL, *const s_pz = sm + 3 * PL, *const s_pxz = sm + 4 * PL;
+    float *const s_lam = sm + 5 * PL, *const s_mu = s_lam + OP, *const s_g = s_mu + OP;  // s_g: three planes
+    float *const s_ring = s_g + 3 * OP;              // [ring item][5][4]: its stresses, lam, mu
+    float *const s_dx = s_ring + 20 * RING, *const s_mx = s_dx + W, *const s_dz = s_mx + W;  // damping; -dt on the domain's columns
+    unsigned *const t_ring = reinterpret_cast<unsigned *>(s_dz + RES_ROWS);
+    int *const t_rslot = reinterpret_cast<int *>(t_ring + RING);  // slots of the ring's items
+    unsigned *const t_word = reinterpret_cast<unsigned *>(t_rslot + RING);  // the threads' halo words
+    float *const s_res = reinterpret_cast<float *>(t_word + 3 * RES_THREADS);  // [2][5][slots][4] staged residuals
+    int *const t_dst = reinterpret_cast<int *>(s_res + 40 * p.slots);  // [4 slots] where a receiver's residual goes
+    const int nring = (th + 2 * R) * (nq + 2) - th * nq;
+    const float dt = a.k.dt;
+    const float *in = a.in + T.slot * a.in_stride;
+    const int frame = frame_count(RB * p.tl.bz, p.tl.nq, 2 * R, HG);
+    const int xpar = 4 * gridDim.x * frame;
+    uint4 *const strip = p.xch + 4 * blockIdx.x * frame;
+    const int shot = a.shot0 + T.slot;
+    const int glo = a.npml + R, ghi_z = g.tnz - R - a.npml, ghi_x = g.tnx - R - a.npml;
+
+    // receivers of the tile and its ring, per line: how many, the first one's
+    // index, trace column and staged entry; [3]: all of them
+    if (tid < 32) {
+        int k0 = 0, n = 0;
+        const Lines &L = a.lines;
+        if (tid < L.n) line_range(L, tid, i0 - R, i0 + th + R, j0 - 4, j0 + 4 * nq + 4, k0, n);
+        const int n0 = __shfl_sync(0xffffffffu, n, 0), n1 = __shfl_sync(0xffffffffu, n, 1), n2 = __shfl_sync(0xffffffffu, n, 2);
+        if (tid < L.n) {
+            s_line[tid][0] = n;
+            s_line[tid][1] = k0;
+            s_line[tid][2] = shot * a.nr + L.slot0[tid] + k0;
+            s_line[tid][3] = tid == 0 ? 0 : tid == 1 ? n0 : n0 + n1;
+        }
+        if (tid == 0) {
+            s_line[3][0] = n0 + n1 + n2;
+            s_nslot = 0;
+            s_stop = ld_relaxed_gpu(p.err) != 0;
+        }
+    }
+    for (int e = tid; e < 40 * p.slots; e += NT) s_res[e] = 0.f;
+    __syncthreads();
+    const int nrec = s_line[3][0];
+    // A slot of staged residuals for each line with receivers on the four cells from (gi, gj): 10 bits
+    // a line, slot + 1.
+    auto slots_of = [&](int gi, int gj) {
+        int w = 0;
+        for (int l = 0; nrec && l < a.lines.n; ++l) {
+            int slot = 0;
+            for (int c = 0; c < 4; ++c) {
+                const int ks = line_slot(a.lines, l, gi, gj + c);
+                if (ks < 0) continue;
+                if (!slot) slot = atomicAdd(&s_nslot, 1) + 1;
+                t_dst[s_line[l][3] + ks - s_line[l][1]] = 4 * (slot - 1) + c;
+            }
+            w |= slot << 10 * l;
+        }
+        return w;
+    };
+    for (int e = tid; e < (th + 4 * R) * (nq + 2 * HG); e += NT) {
+        const int r = e / (nq + 2 * HG), q = e - r * (nq + 2 * HG), o = r * W + 4 * q;
+        const int gi = i0 - 2 * R + r, gj = j0 - HX + 4 * q;
+        const float4 b = ld4(a.mat + 2 * P, g, gi, gj);
+        st4s(s_pvx + o, times4(ld4(in + VX * P, g, gi, gj), b));
+        st4s(s_pvz + o, times4(ld4(in + VZ * P, g, gi, gj), b));
+    }
+    for (int e = tid; e < nring; e += NT) {
+        int r, q;
+        frame_item(e, th + 2 * R, nq + 2, R, 1, r, q);
+        t_ring[e] = pack_item(r, q);
+        const int gi = i0 - R + r, gj = j0 - 4 + 4 * q;
+        t_rslot[e] = slots_of(gi, gj);
+        float *s = s_ring + 20 * e;
+        st4s(s, ld4(in + TXX * P, g, gi, gj));
+        st4s(s + 4, ld4(in + TZZ * P, g, gi, gj));
+        st4s(s + 8, ld4(in + TXZ * P, g, gi, gj));
+        st4s(s + 12, ld4(a.mat, g, gi, gj));
+        st4s(s + 16, ld4(a.mat + P, g, gi, gj));
+    }
+    for (int e = tid; e < 4 * nq + 2 * HX; e += NT) {
+        const int c = j0 - HX + e + XO;
+        s_dx[e] = c >= 0 && c < g.pitch ? __ldg(a.dampx + c) : 0.f;
+        s_mx[e] = in_domain(g, R, R, j0 - HX + e) ? -dt : 0.f;
+    }
+    for (int e = tid; e < th + 4 * R; e += NT) {
+        const int i = i0 - 2 * R + e + ZO;
+        s_dz[e] = i >= 0 && i < g.rows ? __ldg(a.dampz + i) : 0.f;
+    }
+
+    // this thread's block
+    const bool mine = tid < T.nblk, inside = tid < T.nin;
+    int bz = 0, bq = 0;
+    if (mine) res_block<R, RB>(T, tid, bz, bq);
+    const int br = bz * RB;
+    const int ot = (br + 2 * R) * W + HX + 4 * bq, og = br * OW + 4 * bq;
+    const int gi0 = i0 + br, gj0 = j0 + 4 * bq;
+    const int co = (gi0 + ZO) * g.pitch + gj0 + XO;
+    float4 vx[RB], vz[RB], ax[RB], az[RB], axz[RB];
+    const float *const gb = a.mat + 2 * P + co;  // its buoyancy, read where it is used (L1)
+    int rs[RB];         // its slots of staged residuals
+    unsigned img = 0;   // rows with imaged cells
+    float *const G = a.gacc + T.slot * a.gacc_stride;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        vx[r] = vz[r] = ax[r] = az[r] = axz[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        rs[r] = 0;
+        if (!mine) continue;
+        const int gi = gi0 + r;
+        vx[r] = ld4(in + VX * P, g, gi, gj0);
+        vz[r] = ld4(in + VZ * P, g, gi, gj0);
+        ax[r] = ld4(in + TXX * P, g, gi, gj0);
+        az[r] = ld4(in + TZZ * P, g, gi, gj0);
+        axz[r] = ld4(in + TXZ * P, g, gi, gj0);
+        st4s(s_lam + og + r * OW, ld4(a.mat, g, gi, gj0));
+        st4s(s_mu + og + r * OW, ld4(a.mat + P, g, gi, gj0));
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            st4s(s_g + f * OP + og + r * OW,
+                 gi < g.tnz ? *reinterpret_cast<const float4 *>(G + f * P + co + r * g.pitch) : make_float4(0.f, 0.f, 0.f, 0.f));
+        rs[r] = slots_of(gi, gj0);
+        if (gi >= glo && gi <= ghi_z && gj0 + 3 >= glo && gj0 <= ghi_x) img |= 1u << r;
+    }
+    __syncthreads();
+
+    const bool res_v = nrec && (a.res[VX] || a.res[VZ]), res_s = nrec && (a.res[TXX] || a.res[TZZ] || a.res[TXZ]);
+    // This thread's receiver (the tile and its ring have fewer than there are threads): where its residuals
+    // go and its trace column.
+    int rec_d = -1, rec_c = 0;
+    for (int l = 0, e = tid; l < a.lines.n; e -= s_line[l++][0])
+        if (e >= 0 && e < s_line[l][0]) {
+            rec_d = t_dst[s_line[l][3] + e];
+            rec_c = s_line[l][2] + e;
+        }
+    // Its residuals of row `row`, step t, into buffer t & 1.
+    auto stage = [&](int row, int t) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(s_res + (t & 1) * 20 * p.slots + rec_d);
+        const long long o = (long long)row * a.ns * a.nr + rec_c;
+#pragma unroll
+        for (int f = 0; f < 5; ++f)
+            if (a.res[f])
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + f * 16 * p.slots), "l"(a.res[f] + o) : "memory");
+    };
+    // Adds the staged residuals of field f, step t, of the slots in w to a group, one receiver line after
+    // another (the cells of a slot without a receiver hold zero).
+    auto inject = [&](float4 &v, int t, int f, int w) {
+        const float *d = s_res + ((t & 1) * 5 + f) * 4 * p.slots;
+        for (; w; w = (int)((unsigned)w >> 10)) {
+            const int s = w & 1023;
+            if (!s) continue;
+            const float4 x = ld4s(d + 4 * (s - 1));
+            v.x += x.x;
+            v.y += x.y;
+            v.z += x.z;
+            v.w += x.w;
+        }
+    };
+    const int t_first = p.t_hi - 1;
+    // word w of a group holds values 3 w .. of its 4 vx and 4 vz products
+    halo_words<R, 3>(t_word, g, p.tl, frame, T.slot, T.tz, T.tx, i0, th, T.q0, nq);
+    auto put = [&](int o, int w, const uint4 &v) {
+        const int f = 3 * w;
+        (f < 4 ? s_pvx + o + f : s_pvz + o + f - 4)[0] = __uint_as_float(v.x);
+        (f + 1 < 4 ? s_pvx + o + f + 1 : s_pvz + o + f - 3)[0] = __uint_as_float(v.y);
+        if (w < 2) (w == 0 ? s_pvx + o + 2 : s_pvz + o + 1)[0] = __uint_as_float(v.z);
+    };
+    // A step injects where its t mod dt_scale is 0 (step 0 never runs); kept by counting down: that of t, and
+    // the residual row of the next injecting step below t.
+    int sub_t = t_first % p.dt_scale;
+    int row = inj_row_dev((t_first - 1) / p.dt_scale * p.dt_scale, p.nt, p.nt_ext, p.dt_scale);
+
+    // What the adjoint velocities difference, from new stresses.
+    auto sums = [&](const float4 &l, const float4 &m, const float4 &x, const float4 &z, const float4 &xz, int o) {
+        float4 sx, sz;
+        adj_sums(l.x, m.x, x.x, z.x, sx.x, sz.x);
+        adj_sums(l.y, m.y, x.y, z.y, sx.y, sz.y);
+        adj_sums(l.z, m.z, x.z, z.z, sx.z, sz.z);
+        adj_sums(l.w, m.w, x.w, z.w, sx.w, sz.w);
+        st4s(s_px + o, sx);
+        st4s(s_pz + o, sz);
+        st4s(s_pxz + o, times4(m, xz));
+    };
+    // -dt on the cells of a row that are updated, else zero (x + 0 * y = x).
+    auto step4 = [&](int gi, int c) { return gi >= R && gi <= g.tnz - R ? ld4s(s_mx + c) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    // New stresses of four cells from their differences Dx+ (b vx), Dz- (b vz), Dz+ (b vx) + Dx- (b vz).
+    auto update = [&](float4 &x, float4 &z, float4 &xz, const float4 &dx, float dz, const float4 &md, const float (&ex)[4],
+                      const float (&ez)[4], const float (&exz)[4]) {
+        float ox[4], oz[4], oxz[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ox[k] = f4(x, k) + f4(md, k) * (f4(dx, k) * f4(x, k) + ex[k]);
+            oz[k] = f4(z, k) + f4(md, k) * (dz * f4(z, k) + ez[k]);
+            oxz[k] = f4(xz, k) + f4(md, k) * ((f4(dx, k) + dz) * f4(xz, k) + exz[k]);
+        }
+        x = mk4(ox);
+        z = mk4(oz);
+        xz = mk4(oxz);
+    };
+
+    // The strip group of row r of the tile in this thread's column, -1: none.
+    auto strip_group = [&](int r) {
+        return r < 2 * R || r >= th - 2 * R || bq < HG || bq >= nq - HG ? frame_index(r, bq, th, nq, 2 * R, HG) : -1;
+    };
+
+    // New stresses of the block.
+    auto stress = [&]() {
+        const float4 dx = ld4s(s_dx + HX + 4 * bq);
+        {
+            auto row = [&](int r) { return ld4s(s_pvx + ot + r * W); };
+            ZSlide<R, true> zx(row);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const float4 md = step4(gi0 + r, HX + 4 * bq);
+                const float dz = s_dz[br + r + 2 * R];
+                float x[12], ox[4], oxz[4];
+                zx.next(row(r + R));
+                xrow<R, true>(x, zx.centre(), s_pvx + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) ox[k] = f4(ax[r], k) + f4(md, k) * (f4(dx, k) * f4(ax[r], k) + xfwd<R>(x, k, a.k.cx));
+                xrow<R, false>(x, ld4s(s_pvz + ot + r * W), s_pvz + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    oxz[k] = f4(axz[r], k) + f4(md, k) * ((f4(dx, k) + dz) * f4(axz[r], k) +
+                                                         (zx.at(k, a.k.cz) + xbwd<R>(x, k, a.k.cx)));
+                ax[r] = mk4(ox);
+                axz[r] = mk4(oxz);
+            }
+        }
+        auto row = [&](int r) { return ld4s(s_pvz + ot + r * W); };
+        ZSlide<R, false> zz(row);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            const float4 md = step4(gi0 + r, HX + 4 * bq);
+            const float dz = s_dz[br + r + 2 * R];
+            zz.next(row(r + R - 1));
+            float oz[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) oz[k] = f4(az[r], k) + f4(md, k) * (dz * f4(az[r], k) + zz.at(k, a.k.cz));
+            az[r] = mk4(oz);
+            sums(ld4s(s_lam + og + r * OW), ld4s(s_mu + og + r * OW), ax[r], az[r], axz[r], ot + r * W);
+        }
+    };
+    // New stresses of ring item e, first, where it is due, what the residual of step t adds to them.
+    auto ring = [&](int e, int t, bool due) {
+        const int r = item_row(t_ring[e]), q = item_col(t_ring[e]), c = (r + R) * W + HX - 4 + 4 * q;
+        float *s = s_ring + 20 * e;
+        float4 x4 = ld4s(s), z4 = ld4s(s + 4), xz4 = ld4s(s + 8);
+        const int w = t_rslot[e];
+        if (due && w) {
+            if (a.res[TXX]) inject(x4, t, TXX, w);
+            if (a.res[TZZ]) inject(z4, t, TZZ, w);
+            if (a.res[TXZ]) inject(xz4, t, TXZ, w);
+        }
+        const ZWindow<R, 1, true> zx([&](int) { return ld4s(s_pvx + c); }, s_pvx + c);
+        const ZWindow<R, 1, false> zz([&](int) { return ld4s(s_pvz + c); }, s_pvz + c);
+        float x[12], ex[4], ez[4], exz[4];
+        xrow<R, true>(x, zx.w[R - 1], s_pvx + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ex[k] = xfwd<R>(x, k, a.k.cx);
+        xrow<R, false>(x, zz.w[R], s_pvz + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ez[k] = zz.at(0, k, a.k.cz);
+            exz[k] = zx.at(0, k, a.k.cz) + xbwd<R>(x, k, a.k.cx);
+        }
+        update(x4, z4, xz4, ld4s(s_dx + HX - 4 + 4 * q), s_dz[r + R], step4(i0 - R + r, HX - 4 + 4 * q), ex, ez, exz);
+        st4s(s, x4);
+        st4s(s + 4, z4);
+        st4s(s + 8, xz4);
+        sums(ld4s(s + 12), ld4s(s + 16), x4, z4, xz4, c);
+    };
+
+    // The difference set of step t of one row of the block; the set of the step after it is asked into L2.
+    float4 qv[5];
+    auto load_set = [&](int t, int r) {
+        if (!(img >> r & 1)) return;
+        const float *q = p.q + (long long)(t - p.q_t0) * p.state + T.slot * a.fwd_stride + co + r * g.pitch;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) qv[f] = qld4s(q + f * P);
+        if (t > p.t_lo)
+#pragma unroll
+            for (int f = 0; f < 5; ++f) qprefetch4(q + f * P - p.state);
+    };
+
+    // ring items go to the threads without a block first, then to those inside
+    const int rank = tid >= T.nblk ? tid - T.nblk : tid + NT - T.nblk;
+    bool stop = s_stop;
+    for (int t = t_first; t >= p.t_lo && !stop; --t) {
+        // the residual that this step's input lacks in its stresses (the first state of a launch has it)
+        const bool due = res_s && t < t_first && sub_t == 0;
+        if (due) {
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                if (!rs[r]) continue;
+                if (a.res[TXX]) inject(ax[r], t, TXX, rs[r]);
+                if (a.res[TZZ]) inject(az[r], t, TZZ, rs[r]);
+                if (a.res[TXZ]) inject(axz[r], t, TXZ, rs[r]);
+            }
+        }
+        sub_t = sub_t ? sub_t - 1 : p.dt_scale - 1;  // of t - 1
+        const bool epi = nrec && t > 1 && sub_t == 0;
+        if (epi) {  // what this step adds at its end, on its way meanwhile
+            if (rec_d >= 0) stage(row, t - 1);
+            row = row ? row - 1 : p.nt_ext - 1;
+        }
+        // stresses: the blocks inside, then, with the halo, the others
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 1 && t < t_first) {  // the neighbours' products of this step's input
+                if (!fetch_halo<3>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
+                    s_stop = 1;
+                __syncthreads();
+                stop = s_stop;
+                if (stop) break;
+            }
+            if (mine && inside == (pass == 0)) stress();
+        }
+        if (stop) break;
+        for (int e = rank; e < nring; e += NT) ring(e, t, due);
+        load_set(t, 0);
+        cp_wait_all();
+        __syncthreads();
+        if (mine) {
+            uint4 *const xo = strip + ((t - 1) & 1) * xpar;  // what step t - 1 reads
+            const unsigned tag = p.tag0 + (unsigned)(t_first - t + 1);
+            const float4 dx4 = ld4s(s_dx + HX + 4 * bq);
+            {
+                auto row = [&](int r) { return ld4s(s_pxz + ot + r * W); };
+                ZSlide<R, false> zxz(row);
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    const float4 m4 = step4(gi0 + r, HX + 4 * bq);
+                    const float dz = s_dz[br + r + 2 * R];
+                    zxz.next(row(r + R - 1));
+                    float x[12], nx[4];
+                    xrow<R, false>(x, ld4s(s_px + ot + r * W), s_px + ot + r * W);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        nx[k] = f4(vx[r], k) + f4(m4, k) * ((2.f * f4(dx4, k) + dz) * f4(vx[r], k) +
+                                                          (xbwd<R>(x, k, a.k.cx) + zxz.at(k, a.k.cz)));
+                    vx[r] = mk4(nx);
+                }
+            }
+            auto row = [&](int r) { return ld4s(s_pz + ot + r * W); };
+            ZSlide<R, true> zz(row);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const float4 m4 = step4(gi0 + r, HX + 4 * bq);
+                const float dz = s_dz[br + r + 2 * R];
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(gb + r * g.pitch));
+                zz.next(row(r + R));
+                float x[12], nz[4];
+                xrow<R, true>(x, ld4s(s_pxz + ot + r * W), s_pxz + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    nz[k] = f4(vz[r], k) + f4(m4, k) * ((f4(dx4, k) + 2.f * dz) * f4(vz[r], k) +
+                                                      (zz.at(k, a.k.cz) + xfwd<R>(x, k, a.k.cx)));
+                vz[r] = mk4(nz);
+                if (img >> r & 1) {
+                    float *G0 = s_g + og + r * OW, *G1 = G0 + OP, *G2 = G1 + OP;
+                    const float4 g0 = ld4s(G0), g1 = ld4s(G1), g2 = ld4s(G2);
+                    float m0[4], m1[4], m2[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        m0[k] = f4(g0, k);
+                        m1[k] = f4(g1, k);
+                        m2[k] = f4(g2, k);
+                        if (gj0 + k >= glo && gj0 + k <= ghi_x) {
+                            const float atx = f4(ax[r], k), atz = f4(az[r], k), atxz = f4(axz[r], k), bk = f4(b, k);
+                            const float avx = f4(vx[r], k), avz = f4(vz[r], k);
+                            float gmu = m0[k], glam = m1[k], grho = m2[k];
+                            gmu += 2.f * dt * (atx * f4(qv[0], k) + atz * f4(qv[1], k)) + dt * atxz * f4(qv[2], k);
+                            glam += dt * (atx + atz) * (f4(qv[0], k) + f4(qv[1], k));
+                            grho += -(dt * (bk * bk)) * (avx * f4(qv[3], k) + avz * f4(qv[4], k));
+                            m0[k] = gmu;
+                            m1[k] = glam;
+                            m2[k] = grho;
+                        }
+                    }
+                    st4s(G0, mk4(m0));
+                    st4s(G1, mk4(m1));
+                    st4s(G2, mk4(m2));
+                }
+                if (r + 1 < RB) load_set(t, r + 1);
+                if (epi && res_v && rs[r]) {  // what step t - 1 finds in its input
+                    if (a.res[VX]) inject(vx[r], t - 1, VX, rs[r]);
+                    if (a.res[VZ]) inject(vz[r], t - 1, VZ, rs[r]);
+                }
+                const float4 px = times4(vx[r], b), pzz = times4(vz[r], b);
+                st4s(s_pvx + ot + r * W, px);
+                st4s(s_pvz + ot + r * W, pzz);
+                if (!inside) {
+                    const int s = strip_group(br + r);
+                    if (s >= 0) {
+                        st_word(xo + 4 * s, px.x, px.y, px.z, tag);
+                        st_word(xo + 4 * s + 1, px.w, pzz.x, pzz.y, tag);
+                        st_word(xo + 4 * s + 2, pzz.z, pzz.w, 0.f, tag);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (!mine) return;
+    // the state that step t_lo - 1 finds, its residual included
+    const bool last = res_s && p.t_lo > 1 && sub_t == 0;
+    const float nan = __int_as_float(RES_NAN);
+    float *out = a.out + T.slot * a.out_stride;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        if (gi0 + r >= g.tnz) break;
+        if (last && rs[r]) {
+            if (a.res[TXX]) inject(ax[r], p.t_lo - 1, TXX, rs[r]);
+            if (a.res[TZZ]) inject(az[r], p.t_lo - 1, TZZ, rs[r]);
+            if (a.res[TXZ]) inject(axz[r], p.t_lo - 1, TXZ, rs[r]);
+        }
+        if (stop) {
+            vx[r] = vz[r] = ax[r] = az[r] = axz[r] = make_float4(nan, nan, nan, nan);
+            for (int f = 0; f < 3; ++f) st4s(s_g + f * OP + og + r * OW, vx[r]);
+        }
+        float *o = out + co + r * g.pitch;
+        *reinterpret_cast<float4 *>(o + VX * P) = vx[r];
+        *reinterpret_cast<float4 *>(o + VZ * P) = vz[r];
+        *reinterpret_cast<float4 *>(o + TXX * P) = ax[r];
+        *reinterpret_cast<float4 *>(o + TZZ * P) = az[r];
+        *reinterpret_cast<float4 *>(o + TXZ * P) = axz[r];
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            *reinterpret_cast<float4 *>(G + f * P + co + r * g.pitch) = ld4s(s_g + f * OP + og + r * OW);
+    }
+}
+
+}  // namespace pyfwi

@@ -1,0 +1,49 @@
+// Launches of the resident time loops for one half order.
+#pragma once
+
+#include "resident.h"
+
+namespace pyfwi {
+
+template <class Args>
+static cudaError_t launch_resident(const void *kern, const Args &a, size_t floats, cudaStream_t s)
+{
+    const size_t smem = floats * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    void *args[] = {const_cast<Args *>(&a)};
+    return cudaLaunchCooperativeKernel(kern, dim3(a.tl.gz * a.tl.gx * a.tl.nslots), dim3(RES_THREADS), args, smem, s);
+}
+
+// Groups of 4 cells with receivers in a tile and its ring, at most.
+inline int res_slots(int R, const Lines &L, int th, int nq)
+{
+    int n = 0;
+    for (int l = 0; l < L.n; ++l) n += L.drow[l] ? th + 2 * R : nq + 2;
+    return n;
+}
+
+template <int R>
+cudaError_t launch_fwd_resident_r(FwdResArgs &a, cudaStream_t s)
+{
+#define CASE(RB_, Q_) \
+    if (a.tl.rb == RB_ && (a.q != nullptr) == Q_) return launch_resident(reinterpret_cast<const void *>(fwd_resident<R, RB_, Q_>), a, FWD_RES_FLOATS<R, RB_>, s);
+    CASE(1, 0) CASE(1, 1) CASE(2, 0) CASE(2, 1) CASE(3, 0) CASE(3, 1)
+#undef CASE
+    return cudaErrorInvalidValue;
+}
+
+template <int R>
+cudaError_t launch_adj_resident_r(AdjResArgs &a, cudaStream_t s)
+{
+    const int th = a.tl.rb * a.tl.bz;
+    a.slots = res_slots(R, a.a.lines, th, a.tl.nq);
+    const size_t f = ADJ_RES_FLOATS<R> + RES_SLOT_FLOATS * (size_t)a.slots;
+#define CASE(RB_) \
+    if (a.tl.rb == RB_) return launch_resident(reinterpret_cast<const void *>(adj_resident<R, RB_>), a, f, s);
+    CASE(1) CASE(2) CASE(3)
+#undef CASE
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace pyfwi

@@ -94,7 +94,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, int *e
 // The bounded wait on an mbarrier nothing arrives at: one thread waits
 // `limit_ns` and gives up as a streaming kernel does, so the timeout path
 // and the host's handling of the error word can be exercised on purpose.
-__global__ void wait_selftest_kernel(int *err, unsigned long long limit_ns)
+static __global__ void wait_selftest_kernel(int *err, unsigned long long limit_ns)
 {
     __shared__ __align__(8) uint64_t bar;
     if (threadIdx.x == 0) {
@@ -158,7 +158,7 @@ __device__ __forceinline__ void ring_rows(int (&o)[2 * R + 1], int r, int n, int
 // lines are walked in order so two receivers on one cell add in turn.
 // transpose != 0: the exact adjoint of the recording, where a line whose vz
 // trace records vx (crosswell) sends its vz residual to the vx field.
-__global__ void inject_kernel(Grid g, float *adj, long long stride, int shot0, int row, const float *r0,
+static __global__ void inject_kernel(Grid g, float *adj, long long stride, int shot0, int row, const float *r0,
                               const float *r1, const float *r2, const float *r3, const float *r4, Lines L, int ns,
                               int nr, int transpose)
 {

@@ -49,6 +49,8 @@ class Plan:
         size = ctypes.c_size_t()
         N.check(self.lib.pyfwi_workspace_size(h, ctypes.byref(size)))
         self.ws_bytes = size.value
+        if self.resident:
+            opts.graph = 0  # a few launches per call: nothing to replay
         with torch.cuda.device(self.device):
             self._ws = torch.empty(self.ws_bytes + 256, dtype=torch.uint8, device=self.device)
         base = self._ws.data_ptr()
@@ -68,6 +70,11 @@ class Plan:
     @staticmethod
     def workspace_bytes(geom, opts, ns_src):
         """Workspace size a plan with these settings would need."""
+        return Plan.query(geom, opts)[0]
+
+    @staticmethod
+    def query(geom, opts):
+        """(workspace bytes, pyfwi_plan_flags) of a plan with these settings."""
         L = N.lib()
         srcx = np.zeros(geom.ns, np.int32)
         srcz = np.zeros(geom.ns, np.int32)
@@ -77,8 +84,10 @@ class Plan:
                                     ctypes.byref(h)))
         size = ctypes.c_size_t()
         N.check(L.pyfwi_workspace_size(h, ctypes.byref(size)))
+        flags = ctypes.c_int32()
+        N.check(L.pyfwi_plan_flags(h, ctypes.byref(flags)))
         L.pyfwi_plan_destroy(h)
-        return size.value
+        return size.value, flags.value
 
     def launches(self):
         c = ctypes.c_int64()
@@ -94,6 +103,11 @@ class Plan:
     def persist(self):
         """True when the plan runs its time loops as persistent kernels."""
         return bool(self._flags() & 1)
+
+    @property
+    def resident(self):
+        """True when the plan keeps the wavefield on chip for whole runs of steps."""
+        return bool(self._flags() & 8)
 
     @property
     def overlap(self):

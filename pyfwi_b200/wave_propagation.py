@@ -26,8 +26,11 @@ cell-shots, where issuing launches from the host would cost a noticeable
 share, and a call issues at most GRAPH_MAX_LAUNCHES launches; the library
 runs longer calls directly either way), ``persist`` (run the time loops as persistent cooperative kernels,
 many steps per launch with a grid barrier between steps, where the layout
-stores every step in FP32 and the tile kernels run: True, False (the
-default), or 'auto': on where a step carries at most 2 M cell-shots),
+stores every step in FP32 and the tile kernels run: True, False, or 'auto':
+on where a step carries at most 2 M cell-shots; absent, with ``tile`` and
+``adj_tile`` absent and ``graph`` not True: the resident time loops, which keep
+the wavefield on chip for whole runs of steps, where a grid fits and exact
+checkpoints hold difference sets in FP32 -- the same bits as False),
 ``overlap`` (exact checkpoints in FP32 with recompute segments: recompute
 segment m - 1 on a second CUDA stream while the adjoint of segment m runs,
 with two segment buffers), ``store`` ('differences', the default: in exact
@@ -69,6 +72,9 @@ DEFAULT_TILE, SMALL_TILE, SMALL_SURVEY_CELLS = 0, 1, 8_000_000
 # inpa['overlap'] when absent: recompute segment m - 1 on a second stream
 # beside the adjoint of segment m
 OVERLAP_DEFAULT = False
+# options.persist when inpa has no 'persist': the time loops with the
+# wavefield on chip wherever the plan allows it
+RESIDENT = 2
 # inpa['store'] when absent
 STORE_DEFAULT = "differences"
 
@@ -312,7 +318,10 @@ class WavePreparation:
             o.tile, o.adj_tile = variants
             o.adjoint = N.ADJOINT_EXACT if self.adjoint == "exact" else N.ADJOINT_REFERENCE
             o.graph = int(self._graph_on(inpa.get("graph", "auto"), batch, seg))
-            o.persist = int(self._persist_on(inpa.get("persist", False), batch))
+            if "persist" in inpa:
+                o.persist = int(self._persist_on(inpa["persist"], batch))
+            elif self.persist_allowed and not {"tile", "adj_tile"} & set(inpa) and inpa.get("graph") not in (True, 1):
+                o.persist = RESIDENT  # no step kernel and no graph of them was asked for
             o.overlap = int(bool(inpa.get("overlap", OVERLAP_DEFAULT)))
             o.store_diffs = int(store == "differences")
             o.chunk = int(inpa.get("chunk", 0))
@@ -399,6 +408,11 @@ class WavePreparation:
     # to 3 and 64 shots on 593,600 cells: forward 6 us + 7.7 us per shot,
     # adjoint 30 us + 14.4 us per shot).
     COST_ADJ, COST_FWD_STEP, COST_ADJ_STEP = 1.9, 4.6e5, 2.3e6
+    # the same with the wavefield on chip: the cells a launch holds (one
+    # 593,600-cell shot), a step's fixed cost in cells and an adjoint step in
+    # forward steps (forward 1.9 us + 6.6 us per million cells, adjoint 1.2 to 2
+    # times that)
+    RES_CELLS, RES_STEP, RES_ADJ = 6.0e5, 3.0e5, 1.6
 
     def _auto_layout(self, geom, opts, seg, batch):
         """Shot batch and recompute segment of the exact checkpoint mode.
@@ -444,9 +458,14 @@ class WavePreparation:
             # ((M - 1) * s) in a smaller store
             return -(-nt // (-(-nt // lo)))
 
+        resident = Plan.query(geom, opts(nt, 1))[1] & 8
+
         def group_cost(s, b):
             m = -(-nt // s)
             fwd = nt + (m - 1) * s
+            if resident:
+                step = np.ceil(b * cells / self.RES_CELLS) * self.RES_STEP + b * cells
+                return (fwd + nt * self.RES_ADJ) * step
             return fwd * (b * cells + self.COST_FWD_STEP) + nt * (b * cells * self.COST_ADJ + self.COST_ADJ_STEP)
 
         best = None
@@ -514,7 +533,7 @@ class WavePropagator(WavePreparation):
         if torch.cuda.is_current_stream_capturing():
             return
         o = self.plan.opts
-        if synchronous or 3 <= o.tile <= 5 or 4 <= o.adj_tile <= 6 or o.persist:
+        if synchronous or 3 <= o.tile <= 5 or 4 <= o.adj_tile <= 6 or o.persist == 1:
             self.plan.check_device()
 
     def _section(self, traces):
