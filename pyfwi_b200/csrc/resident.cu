@@ -22,7 +22,7 @@ bool fits(int th, int nq, int rb, int ctas, const Lines &lines, bool adjoint)
     const int halo = (th + 4 * R) * (nq + 2 * S::HG) - th * nq, slots = res_slots(R, lines, th, nq);
     return th <= S::TH && nq <= S::NQ && (th / rb) * nq <= RES_THREADS && halo <= RES_HALO &&
            ctas * frame_count(th, nq, 2 * R, S::HG) <= RES_MAX_STRIPS && slots <= RES_MAX_SLOTS &&
-           (!adjoint || ADJ_RES_FLOATS<R> + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
+           (!adjoint || adj_res_floats<R>(rb) + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
 }
 
 static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_FLOATS, "the forward loop fits on an SM");
@@ -34,17 +34,17 @@ static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_
 // launch small; many let one launch hold four times the cells.  The model of a
 // step (us) is a fit to launches of both orders on grids of 140 x 140 to 560 x
 // 1060 cells, each run with 1, 2 and 3 rows and 1 to 8 shots per launch; it is
-// within 10 % of all 36.  Measured, forward / adjoint, per step of all shots:
-// 8 shots of 240 x 440 take 19.2 / 25.8 us with 1 row one after another, 13.8
-// / 19.1 with 2 rows two at a time, 10.7 / 18.9 with 3 rows four at a time; 8
-// of 140 x 140 in one launch 3.10 / 3.88 with 1 row, 4.25 / 7.33 with 3.
+// within 7 % of all that come near their grid's best.  Measured, forward / adjoint, per step of all shots: 8
+// shots of 240 x 440 take 12.6 / 16.0 us with 1 row and two shots at a time,
+// 13.6 / 17.1 with 2 rows and two, 10.8 / 17.0 with 3 rows and four; 8 of 140 x
+// 140 in one launch 3.15 / 3.36 with 1 row, 4.31 / 7.47 with 3.
 bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms, bool adjoint, ResTiles *out)
 {
     struct Cost {
         double step, row, warp_row, ring, row3;  // fixed; per row; per warp of blocks and row; per warp of ring items; with 3 rows
     };
-    constexpr Cost COST[2][2] = {{{1.48, 0.64, 0.072, 0.021, 0.0}, {0.26, 0.35, 0.0, 1.02, 2.54}},
-                                 {{2.62, 0.96, 0.0, 0.15, 0.0}, {4.73, 0.0, 0.139, 0.0, 4.80}}};
+    constexpr Cost COST[2][2] = {{{1.463, 0.368, 0.013, 0.3, 0.737}, {1.335, 0.545, 0.060, 0.3, 2.460}},
+                                 {{1.806, 0.258, 0.090, 0.3, 1.090}, {1.280, 0.721, 0.196, 0.3, 3.239}}};
     const Cost &k = COST[R > 2][adjoint];
     const int ncg = (g.tnx + 3) / 4, hg = R <= 2 ? 1 : 2;
     double best = 0;

@@ -26,9 +26,9 @@
 // bytes per imaged cell, written forward, read backward).
 //
 // Measured, forward / adjoint per step of all shots, against one launch per
-// step: 500 x 1000 cells and 4 shots 50.8 / 59.2 -> 23.0 / 44.4 us; whole
-// gradients of 100 x 100 cells, 4 shots, 500 steps 7.1 -> 2.9 ms, and of 200 x
-// 400 cells, 10 shots, 400 steps 24 -> 13.7 ms.
+// step: 500 x 1000 cells and 4 shots 50.8 / 59.2 -> 22.9 / 37.6 us; whole
+// gradients of 100 x 100 cells, 4 shots, 500 steps 7.1 -> 2.6 ms, and of 200 x
+// 400 cells, 10 shots, 1000 steps 48.4 -> 30.7 ms.
 //
 // The arithmetic is that of fwd_step / adj_step, operation for operation:
 // the results are the step kernels' bits, whatever the tiling.
@@ -164,9 +164,17 @@ struct AdjResArgs {
 template <int R, int RB>
 constexpr int FWD_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 6 * ResShape<R>::RING + 2 * RES_ROWS + 2 * RES_W + 8 +
                                4 * RES_MAX_SAMPLES + 4 * RES_THREADS;
-template <int R>
-constexpr int ADJ_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 5 * ResShape<R>::OPLANE + 22 * ResShape<R>::RING + 2 * RES_ROWS +
-                               3 * RES_W + 3 * RES_THREADS;
+// Adjoint: a thread's places for difference sets on their way, four floats
+// each: three rows share six places, asked for in turns.  Blocks of more than
+// one row keep one of the three gradient accumulators in shared memory: with
+// all of them in registers the loop spills.
+template <int RB>
+constexpr int RES_SETS = RB < 3 ? 0 : 6;
+template <int R, int RB>
+constexpr int RES_OWN = RB < 3 ? 4 * RB * RES_THREADS : ResShape<R>::OPLANE;  // a plane of the blocks alone
+template <int R, int RB>
+constexpr int ADJ_RES_FLOATS = RES_PAD + 5 * RES_PLANE + (RB < 2 ? 2 : 3) * RES_OWN<R, RB> + 22 * ResShape<R>::RING + 2 * RES_ROWS +
+                               3 * RES_W + 3 * RES_THREADS + 4 * RES_SETS<RB> * RES_THREADS;
 constexpr int RES_SLOT_FLOATS = 44;  // and per slot of staged residuals (adjoint)
 
 // 16-byte words that are written and read as one transaction.
@@ -224,27 +232,30 @@ __device__ __forceinline__ void halo_words(unsigned *word, const Grid &g, const 
 // Each of the words read until its tag is `tag`, then handed to put(offset,
 // word of the group, value).  False when the wait gave up (error word set,
 // here or by another CTA).
-template <int W, class Put>
+template <int W, bool LEAN, class Put>
 __device__ __forceinline__ bool fetch_halo(const uint4 *buf, unsigned tag, const unsigned *words, int *err,
                                            unsigned long long limit_ns, Put put)
 {
     unsigned long long t0 = 0;
-    unsigned open = 0, word[W];
+    unsigned open = 0, kept[W];
+    // LEAN: a word's place is read again where it is used, for kernels that are short of registers
+    auto word = [&](int k) { return LEAN ? words[k * RES_THREADS + threadIdx.x] : kept[k]; };
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-        word[k] = words[k * RES_THREADS + threadIdx.x];
-        if (word[k] != ~0u) open |= 1u << k;
+        kept[k] = words[k * RES_THREADS + threadIdx.x];
+        if (kept[k] != ~0u) open |= 1u << k;
     }
     for (unsigned n = 1; open; ++n) {
         uint4 v[W];
 #pragma unroll
         for (int k = 0; k < W; ++k)
-            if (open >> k & 1) v[k] = ld_word(buf + (word[k] >> 14));
+            if (open >> k & 1) v[k] = ld_word(buf + (word(k) >> 14));
 #pragma unroll
         for (int k = 0; k < W; ++k)
             if ((open >> k & 1) && v[k].w == tag) {
+                const unsigned u = word(k);
                 open &= ~(1u << k);
-                put((int)(word[k] & 0x3FFFu), (int)(word[k] >> 14 & 3u), v[k]);
+                put((int)(u & 0x3FFFu), (int)(u >> 14 & 3u), v[k]);
             }
         if (open && (n & 63u) == 0) {
             if (ld_relaxed_gpu(err) != 0) return false;
@@ -349,14 +360,22 @@ struct ZSlide {
 
 // Difference values are written once and read once: streaming accesses.
 __device__ __forceinline__ void qst4s(float *q, float4 v) { __stcs(reinterpret_cast<float4 *>(q), v); }
+// Keeps the compiler from loading early what comes after, where that would cost registers.
+__device__ __forceinline__ void in_order() { asm volatile("" ::: "memory"); }
+
+// Difference values are read once: past L1.
 __device__ __forceinline__ float4 qld4s(const float *q)
 {
     float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(q));
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(q));
     return v;
 }
+
+// Groups of asynchronous copies.
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
 __device__ __forceinline__ void qprefetch4(const float *q) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q)); }
 __device__ __forceinline__ float4 mk4(const float (&v)[4]) { return make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ float4 times4(const float4 &u, const float4 &v)
@@ -780,7 +799,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1) {
                 if (t > p.t0) {  // the neighbours' strips of S_t
-                    if (!fetch_halo<4>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t - p.t0), t_word, p.err, p.limit_ns, put))
+                    if (!fetch_halo<4, false>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t - p.t0), t_word, p.err, p.limit_ns, put))
                         s_stop = 1;
                     __syncthreads();
                     stop = s_stop;
@@ -854,28 +873,45 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
 // ---------------------------------------------------------------------------
 // adjoint steps t_hi - 1 .. t_lo with imaging (adj_step's arithmetic)
 // ---------------------------------------------------------------------------
-// Each thread keeps its block's velocities and stresses in registers.  Shared memory holds what neighbouring blocks difference (b * Av
-// on the tile and its 2R halo; the sums of adj_sums and mu * Atxz on the tile
-// and its ring), the block's lam and mu and its three accumulators, and the
-// ring's stresses and materials.
+// Each thread keeps its block's velocities and stresses in registers, and its
+// gradient accumulators (one of the three only with one row per block).  Shared
+// memory holds what neighbouring blocks difference (b * Av on the tile and its
+// 2R halo; the sums of adj_sums and mu * Atxz on the tile and its ring), the
+// block's lam and mu, and the ring's stresses and materials.
+// What bounds it is latency: the exchange with the neighbours, two barriers and
+// the chains between them.  A register spilled costs more than any arithmetic,
+// since next to this much shared memory there is hardly an L1: 100 bytes of
+// spills a thread cost a third of a 500 x 1000 survey's step.
 template <int R, int RB>
 __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_constant__ AdjResArgs p)
 {
     constexpr int NT = RES_THREADS, HX = ResShape<R>::HX, HG = ResShape<R>::HG;
     extern __shared__ float4 smem4[];
-    __shared__ int s_stop, s_nslot, s_line[4][6];
+    __shared__ int s_stop, s_nslot, s_line[4][6], s_t[6];
     const AdjArgs &a = p.a;
     const Grid &g = a.g;
     const long long P = g.plane;
     const int tid = threadIdx.x;
     const ResTile T = res_tile<R, RB>(p.tl);
+    // With three rows what the loop needs of the tile is read from shared memory, and a thread's places are
+    // worked out again from its block's number in each phase: kept in registers, they would spill the fields.
+    if (tid == 0) {
+        s_t[0] = T.i0;
+        s_t[1] = T.j0;
+        s_t[2] = T.th;
+        s_t[3] = T.nq;
+        s_t[4] = T.slot;
+    }
     const int i0 = T.i0, j0 = T.j0, th = T.th, nq = T.nq;
-    constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING, OW = ResShape<R>::OW, OP = ResShape<R>::OPLANE;
+    constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING;
     float *const sm = reinterpret_cast<float *>(smem4) + RES_PAD;
     // Cell (r, c) of the tile lies at (r + 2R) * W + HX + c of the first five planes, at r * OW + c of the others.
     float *const s_pvx = sm, *const s_pvz = sm + PL, *const s_px = sm + 2 * PL, *const s_pz = sm + 3 * PL, *const s_pxz = sm + 4 * PL;
-    float *const s_lam = sm + 5 * PL, *const s_mu = s_lam + OP, *const s_g = s_mu + OP;  // s_g: three planes
-    float *const s_ring = s_g + 3 * OP;              // [ring item][5][4]: its stresses, lam, mu
+    constexpr int OWN = RES_OWN<R, RB>;
+    float *const s_lam = sm + 5 * PL, *const s_mu = s_lam + OWN;  // row r of a block at om + r * OM
+    float *const s_rho = s_mu + OWN;                              // RB > 1: grho
+    float *const s_set = s_rho + (RB < 2 ? 0 : OWN);              // [place][thread][4]: difference sets on their way
+    float *const s_ring = s_set + 4 * RES_SETS<RB> * NT;          // [ring item][5][4]: its stresses, lam, mu
     float *const s_dx = s_ring + 20 * RING, *const s_mx = s_dx + W, *const s_dz = s_mx + W;  // damping; -dt on the domain's columns
     unsigned *const t_ring = reinterpret_cast<unsigned *>(s_dz + RES_ROWS);
     int *const t_rslot = reinterpret_cast<int *>(t_ring + RING);  // slots of the ring's items
@@ -887,7 +923,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
     const float *in = a.in + T.slot * a.in_stride;
     const int frame = frame_count(RB * p.tl.bz, p.tl.nq, 2 * R, HG);
     const int xpar = 4 * gridDim.x * frame;
-    uint4 *const strip = p.xch + 4 * blockIdx.x * frame;
     const int shot = a.shot0 + T.slot;
     const int glo = a.npml + R, ghi_z = g.tnz - R - a.npml, ghi_x = g.tnx - R - a.npml;
 
@@ -964,17 +999,38 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
     int bz = 0, bq = 0;
     if (mine) res_block<R, RB>(T, tid, bz, bq);
     const int br = bz * RB;
-    const int ot = (br + 2 * R) * W + HX + 4 * bq, og = br * OW + 4 * bq;
+    const int ot = (br + 2 * R) * W + HX + 4 * bq;
+    constexpr int OM = RB < 3 ? 4 * NT : ResShape<R>::OW;
+    const int om = RB < 3 ? 4 * tid : br * OM + 4 * bq;
     const int gi0 = i0 + br, gj0 = j0 + 4 * bq;
     const int co = (gi0 + ZO) * g.pitch + gj0 + XO;
+    const unsigned own = (unsigned)bz << 8 | (unsigned)bq;
+    struct Own {
+        int br, bq, ot, gi0, gj0;
+    };
+    auto place = [&]() {
+        unsigned w = own;
+        if (RB == 3) asm volatile("" : "+r"(w));  // anew each time
+        Own o;
+        o.br = RB * (int)(w >> 8);
+        o.bq = (int)(w & 255u);
+        o.ot = (o.br + 2 * R) * W + HX + 4 * o.bq;
+        o.gi0 = (RB == 3 ? s_t[0] : i0) + o.br;
+        o.gj0 = (RB == 3 ? s_t[1] : j0) + 4 * o.bq;
+        return o;
+    };
+    auto om_of = [&](const Own &o) { return RB < 3 ? 4 * tid : o.br * OM + 4 * o.bq; };
+    auto co_of = [&](const Own &o) { return (o.gi0 + ZO) * g.pitch + o.gj0 + XO; };
     float4 vx[RB], vz[RB], ax[RB], az[RB], axz[RB];
-    const float *const gb = a.mat + 2 * P + co;  // its buoyancy, read where it is used (L1)
+    float4 gmu[RB], glam[RB], grho;  // its gradient accumulators
     int rs[RB];         // its slots of staged residuals
     unsigned img = 0;   // rows with imaged cells
     float *const G = a.gacc + T.slot * a.gacc_stride;
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
         vx[r] = vz[r] = ax[r] = az[r] = axz[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        gmu[r] = glam[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (RB < 2) grho = gmu[r];
         rs[r] = 0;
         if (!mine) continue;
         const int gi = gi0 + r;
@@ -983,12 +1039,17 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
         ax[r] = ld4(in + TXX * P, g, gi, gj0);
         az[r] = ld4(in + TZZ * P, g, gi, gj0);
         axz[r] = ld4(in + TXZ * P, g, gi, gj0);
-        st4s(s_lam + og + r * OW, ld4(a.mat, g, gi, gj0));
-        st4s(s_mu + og + r * OW, ld4(a.mat + P, g, gi, gj0));
-#pragma unroll
-        for (int f = 0; f < 3; ++f)
-            st4s(s_g + f * OP + og + r * OW,
-                 gi < g.tnz ? *reinterpret_cast<const float4 *>(G + f * P + co + r * g.pitch) : make_float4(0.f, 0.f, 0.f, 0.f));
+        st4s(s_lam + om + r * OM, ld4(a.mat, g, gi, gj0));
+        st4s(s_mu + om + r * OM, ld4(a.mat + P, g, gi, gj0));
+        if (gi < g.tnz) {
+            gmu[r] = *reinterpret_cast<const float4 *>(G + co + r * g.pitch);
+            glam[r] = *reinterpret_cast<const float4 *>(G + P + co + r * g.pitch);
+            const float4 gr = *reinterpret_cast<const float4 *>(G + 2 * P + co + r * g.pitch);
+            if (RB < 2)
+                grho = gr;
+            else
+                st4s(s_rho + om + r * OM, gr);
+        }
         rs[r] = slots_of(gi, gj0);
         if (gi >= glo && gi <= ghi_z && gj0 + 3 >= glo && gj0 <= ghi_x) img |= 1u << r;
     }
@@ -1069,26 +1130,96 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
     };
 
     // The strip group of row r of the tile in this thread's column, -1: none.
-    auto strip_group = [&](int r) {
-        return r < 2 * R || r >= th - 2 * R || bq < HG || bq >= nq - HG ? frame_index(r, bq, th, nq, 2 * R, HG) : -1;
+    auto strip_group = [&](int r, int q) {
+        const int h = RB == 3 ? s_t[2] : th, w = RB == 3 ? s_t[3] : nq;
+        return r < 2 * R || r >= h - 2 * R || q < HG || q >= w - HG ? frame_index(r, q, h, w, 2 * R, HG) : -1;
     };
 
+    // Difference sets of step t.  One or two rows read a row's into registers, ahead of their use, and ask for
+    // those of the step after it into L2.
+    auto sets_of = [&](int t) { return p.q + (long long)(t - p.q_t0) * p.state + (RB == 3 ? s_t[4] : T.slot) * a.fwd_stride + co_of(place()); };
+    float4 qv[5];
+    auto load_set = [&](int t, int r) {
+        if (!(img >> r & 1)) return;
+        const float *q = sets_of(t) + r * g.pitch;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) qv[f] = qld4s(q + f * P);
+        if (t > p.t_lo)
+#pragma unroll
+            for (int f = 0; f < 5; ++f) qprefetch4(q + f * P - p.state);
+    };
+    // With three rows asynchronous copies, by each thread for itself: the little L1 that this much shared memory
+    // leaves holds up plain loads, and their registers spill.  500 x 1000 cells, 4 shots: 44.2 us per step
+    // with loads, 37.6 with copies.
+    auto set_at = [&](int place) { return ld4s(s_set + 4 * (place * NT + tid)); };
+    auto ask = [&](const float *q, int f, int r, int place) {
+        if (img >> r & 1)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(s_set + 4 * (place * NT + tid))),
+                         "l"(q + f * P + r * g.pitch)
+                         : "memory");
+    };
+    // What the new stresses of row r add to the gradient (in the step kernels' contractions).
+    auto image_stress = [&](int r, int gj0, const float4 &q0, const float4 &q1, const float4 &q2) {
+        if (img >> r & 1) {
+            float m0[4], m1[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                m0[k] = f4(gmu[r], k);
+                m1[k] = f4(glam[r], k);
+                if (gj0 + k >= glo && gj0 + k <= ghi_x) {
+                    const float atx = f4(ax[r], k), atz = f4(az[r], k), atxz = f4(axz[r], k);
+                    float gm = m0[k], gl = m1[k];
+                    gm += __fmaf_rn(__fmul_rn(dt, atxz), f4(q2, k),
+                                    __fmul_rn(2.f * dt, __fmaf_rn(atx, f4(q0, k), __fmul_rn(atz, f4(q1, k)))));
+                    gl += dt * (atx + atz) * (f4(q0, k) + f4(q1, k));
+                    m0[k] = gm;
+                    m1[k] = gl;
+                }
+            }
+            gmu[r] = mk4(m0);
+            glam[r] = mk4(m1);
+        }
+    };
+    // And its new velocities.
+    auto image_velocity = [&](int r, int gj0, int om, const float4 &b, const float4 &q3, const float4 &q4) {
+        if (img >> r & 1) {
+            const float4 gr4 = RB < 2 ? grho : ld4s(s_rho + om + r * OM);
+            float m2[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                m2[k] = f4(gr4, k);
+                if (gj0 + k >= glo && gj0 + k <= ghi_x) {
+                    const float bk = f4(b, k), avx = f4(vx[r], k), avz = f4(vz[r], k);
+                    float gr = m2[k];
+                    gr += -(dt * (bk * bk)) * (avx * f4(q3, k) + avz * f4(q4, k));
+                    m2[k] = gr;
+                }
+            }
+            if (RB < 2)
+                grho = mk4(m2);
+            else
+                st4s(s_rho + om + r * OM, mk4(m2));
+        }
+    };
     // New stresses of the block.
     auto stress = [&]() {
-        const float4 dx = ld4s(s_dx + HX + 4 * bq);
+        const Own o = place();
+        const int om = om_of(o);
+        const float4 dx = ld4s(s_dx + HX + 4 * o.bq);
         {
-            auto row = [&](int r) { return ld4s(s_pvx + ot + r * W); };
+            auto row = [&](int r) { return ld4s(s_pvx + o.ot + r * W); };
             ZSlide<R, true> zx(row);
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
-                const float4 md = step4(gi0 + r, HX + 4 * bq);
-                const float dz = s_dz[br + r + 2 * R];
+                const float4 md = step4(o.gi0 + r, HX + 4 * o.bq);
+                const float dz = s_dz[o.br + r + 2 * R];
                 float x[12], ox[4], oxz[4];
                 zx.next(row(r + R));
-                xrow<R, true>(x, zx.centre(), s_pvx + ot + r * W);
+                xrow<R, true>(x, zx.centre(), s_pvx + o.ot + r * W);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) ox[k] = f4(ax[r], k) + f4(md, k) * (f4(dx, k) * f4(ax[r], k) + xfwd<R>(x, k, a.k.cx));
-                xrow<R, false>(x, ld4s(s_pvz + ot + r * W), s_pvz + ot + r * W);
+                xrow<R, false>(x, ld4s(s_pvz + o.ot + r * W), s_pvz + o.ot + r * W);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     oxz[k] = f4(axz[r], k) + f4(md, k) * ((f4(dx, k) + dz) * f4(axz[r], k) +
@@ -1097,23 +1228,44 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
                 axz[r] = mk4(oxz);
             }
         }
-        auto row = [&](int r) { return ld4s(s_pvz + ot + r * W); };
+        auto row = [&](int r) { return ld4s(s_pvz + o.ot + r * W); };
         ZSlide<R, false> zz(row);
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
-            const float4 md = step4(gi0 + r, HX + 4 * bq);
-            const float dz = s_dz[br + r + 2 * R];
+            const float4 md = step4(o.gi0 + r, HX + 4 * o.bq);
+            const float dz = s_dz[o.br + r + 2 * R];
             zz.next(row(r + R - 1));
             float oz[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) oz[k] = f4(az[r], k) + f4(md, k) * (dz * f4(az[r], k) + zz.at(k, a.k.cz));
             az[r] = mk4(oz);
-            sums(ld4s(s_lam + og + r * OW), ld4s(s_mu + og + r * OW), ax[r], az[r], axz[r], ot + r * W);
+            sums(ld4s(s_lam + om + r * OM), ld4s(s_mu + om + r * OM), ax[r], az[r], axz[r], o.ot + r * W);
         }
     };
     // New stresses of ring item e, first, where it is due, what the residual of step t adds to them.
     auto ring = [&](int e, int t, bool due) {
         const int r = item_row(t_ring[e]), q = item_col(t_ring[e]), c = (r + R) * W + HX - 4 + 4 * q;
+        float x[12], ex[4], ez[4], exz[4];
+        {
+            const ZWindow<R, 1, true> zx([&](int) { return ld4s(s_pvx + c); }, s_pvx + c);
+            xrow<R, true>(x, zx.w[R - 1], s_pvx + c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                ex[k] = xfwd<R>(x, k, a.k.cx);
+                exz[k] = zx.at(0, k, a.k.cz);
+            }
+        }
+        in_order();
+        {
+            const ZWindow<R, 1, false> zz([&](int) { return ld4s(s_pvz + c); }, s_pvz + c);
+            xrow<R, false>(x, zz.w[R], s_pvz + c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                ez[k] = zz.at(0, k, a.k.cz);
+                exz[k] += xbwd<R>(x, k, a.k.cx);
+            }
+        }
+        in_order();
         float *s = s_ring + 20 * e;
         float4 x4 = ld4s(s), z4 = ld4s(s + 4), xz4 = ld4s(s + 8);
         const int w = t_rslot[e];
@@ -1122,36 +1274,27 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
             if (a.res[TZZ]) inject(z4, t, TZZ, w);
             if (a.res[TXZ]) inject(xz4, t, TXZ, w);
         }
-        const ZWindow<R, 1, true> zx([&](int) { return ld4s(s_pvx + c); }, s_pvx + c);
-        const ZWindow<R, 1, false> zz([&](int) { return ld4s(s_pvz + c); }, s_pvz + c);
-        float x[12], ex[4], ez[4], exz[4];
-        xrow<R, true>(x, zx.w[R - 1], s_pvx + c);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) ex[k] = xfwd<R>(x, k, a.k.cx);
-        xrow<R, false>(x, zz.w[R], s_pvz + c);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            ez[k] = zz.at(0, k, a.k.cz);
-            exz[k] = zx.at(0, k, a.k.cz) + xbwd<R>(x, k, a.k.cx);
-        }
-        update(x4, z4, xz4, ld4s(s_dx + HX - 4 + 4 * q), s_dz[r + R], step4(i0 - R + r, HX - 4 + 4 * q), ex, ez, exz);
+        update(x4, z4, xz4, ld4s(s_dx + HX - 4 + 4 * q), s_dz[r + R], step4(s_t[0] - R + r, HX - 4 + 4 * q), ex, ez, exz);
         st4s(s, x4);
         st4s(s + 4, z4);
         st4s(s + 8, xz4);
         sums(ld4s(s + 12), ld4s(s + 16), x4, z4, xz4, c);
     };
 
-    // The difference set of step t of one row of the block; the set of the step after it is asked into L2.
-    float4 qv[5];
-    auto load_set = [&](int t, int r) {
-        if (!(img >> r & 1)) return;
-        const float *q = p.q + (long long)(t - p.q_t0) * p.state + T.slot * a.fwd_stride + co + r * g.pitch;
+    // The first copies for step t: two rows' for the stresses; the others are asked into L2.
+    auto ask_first = [&](int t) {
+        const float *q = sets_of(t);
 #pragma unroll
-        for (int f = 0; f < 5; ++f) qv[f] = qld4s(q + f * P);
-        if (t > p.t_lo)
+        for (int r = 0; r < RB; ++r)
 #pragma unroll
-            for (int f = 0; f < 5; ++f) qprefetch4(q + f * P - p.state);
+            for (int f = 0; f < 5; ++f)
+                if (r < 2 && f < 3)
+                    ask(q, f, r, 3 * r + f);
+                else if (img >> r & 1)
+                    qprefetch4(q + f * P + r * g.pitch);
+        cp_commit();
     };
+    if (RB == 3) ask_first(t_first);
 
     // ring items go to the threads without a block first, then to those inside
     const int rank = tid >= T.nblk ? tid - T.nblk : tid + NT - T.nblk;
@@ -1174,37 +1317,56 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
             if (rec_d >= 0) stage(row, t - 1);
             row = row ? row - 1 : p.nt_ext - 1;
         }
+        cp_commit();
         // stresses: the blocks inside, then, with the halo, the others
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1 && t < t_first) {  // the neighbours' products of this step's input
-                if (!fetch_halo<3>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
+                if (!fetch_halo<3, (RB == 3)>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
                     s_stop = 1;
                 __syncthreads();
                 stop = s_stop;
                 if (stop) break;
             }
-            if (mine && inside == (pass == 0)) stress();
+            if (mine && inside == (pass == 0)) {
+                if (RB == 3) cp_wait<1>();
+                stress();
+                if (RB == 3) {
+                    const int gj = place().gj0;
+                    image_stress(0, gj, set_at(0), set_at(1), set_at(2));
+                    image_stress(1, gj, set_at(3), set_at(4), set_at(5));
+                    const float *q = sets_of(t);
+                    for (int f = 0; f < 3; ++f) ask(q, f, 2, f);
+                    for (int f = 3; f < 5; ++f) ask(q, f, 0, f);
+                    cp_commit();
+                }
+            }
         }
         if (stop) break;
         for (int e = rank; e < nring; e += NT) ring(e, t, due);
-        load_set(t, 0);
-        cp_wait_all();
+        if (RB < 3) load_set(t, 0);
+        // the staged residuals are there
+        if (RB == 3 && mine)
+            cp_wait<1>();
+        else
+            cp_wait<0>();
         __syncthreads();
         if (mine) {
-            uint4 *const xo = strip + ((t - 1) & 1) * xpar;  // what step t - 1 reads
+            const Own o = place();
+            const float *gb = a.mat + 2 * P + co_of(o);
+            uint4 *const xo = p.xch + 4 * blockIdx.x * frame + ((t - 1) & 1) * xpar;  // what step t - 1 reads
             const unsigned tag = p.tag0 + (unsigned)(t_first - t + 1);
-            const float4 dx4 = ld4s(s_dx + HX + 4 * bq);
+            const float4 dx4 = ld4s(s_dx + HX + 4 * o.bq);
             {
-                auto row = [&](int r) { return ld4s(s_pxz + ot + r * W); };
+                auto row = [&](int r) { return ld4s(s_pxz + o.ot + r * W); };
                 ZSlide<R, false> zxz(row);
 #pragma unroll
                 for (int r = 0; r < RB; ++r) {
-                    const float4 m4 = step4(gi0 + r, HX + 4 * bq);
-                    const float dz = s_dz[br + r + 2 * R];
+                    const float4 m4 = step4(o.gi0 + r, HX + 4 * o.bq);
+                    const float dz = s_dz[o.br + r + 2 * R];
                     zxz.next(row(r + R - 1));
                     float x[12], nx[4];
-                    xrow<R, false>(x, ld4s(s_px + ot + r * W), s_px + ot + r * W);
+                    xrow<R, false>(x, ld4s(s_px + o.ot + r * W), s_px + o.ot + r * W);
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
                         nx[k] = f4(vx[r], k) + f4(m4, k) * ((2.f * f4(dx4, k) + dz) * f4(vx[r], k) +
@@ -1212,56 +1374,51 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
                     vx[r] = mk4(nx);
                 }
             }
-            auto row = [&](int r) { return ld4s(s_pz + ot + r * W); };
+            if (RB == 3) {
+                cp_wait<0>();
+                image_stress(RB - 1, o.gj0, set_at(0), set_at(1), set_at(2));
+                const float *q = sets_of(t);
+                ask(q, 3, 1, 0);
+                ask(q, 4, 1, 1);
+                ask(q, 3, 2, 2);
+                ask(q, 4, 2, 5);
+                cp_commit();
+            }
+            auto row = [&](int r) { return ld4s(s_pz + o.ot + r * W); };
             ZSlide<R, true> zz(row);
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
-                const float4 m4 = step4(gi0 + r, HX + 4 * bq);
-                const float dz = s_dz[br + r + 2 * R];
+                const float4 m4 = step4(o.gi0 + r, HX + 4 * o.bq);
+                const float dz = s_dz[o.br + r + 2 * R];
                 const float4 b = __ldg(reinterpret_cast<const float4 *>(gb + r * g.pitch));
                 zz.next(row(r + R));
                 float x[12], nz[4];
-                xrow<R, true>(x, ld4s(s_pxz + ot + r * W), s_pxz + ot + r * W);
+                xrow<R, true>(x, ld4s(s_pxz + o.ot + r * W), s_pxz + o.ot + r * W);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     nz[k] = f4(vz[r], k) + f4(m4, k) * ((f4(dx4, k) + 2.f * dz) * f4(vz[r], k) +
                                                       (zz.at(k, a.k.cz) + xfwd<R>(x, k, a.k.cx)));
                 vz[r] = mk4(nz);
-                if (img >> r & 1) {
-                    float *G0 = s_g + og + r * OW, *G1 = G0 + OP, *G2 = G1 + OP;
-                    const float4 g0 = ld4s(G0), g1 = ld4s(G1), g2 = ld4s(G2);
-                    float m0[4], m1[4], m2[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        m0[k] = f4(g0, k);
-                        m1[k] = f4(g1, k);
-                        m2[k] = f4(g2, k);
-                        if (gj0 + k >= glo && gj0 + k <= ghi_x) {
-                            const float atx = f4(ax[r], k), atz = f4(az[r], k), atxz = f4(axz[r], k), bk = f4(b, k);
-                            const float avx = f4(vx[r], k), avz = f4(vz[r], k);
-                            float gmu = m0[k], glam = m1[k], grho = m2[k];
-                            gmu += 2.f * dt * (atx * f4(qv[0], k) + atz * f4(qv[1], k)) + dt * atxz * f4(qv[2], k);
-                            glam += dt * (atx + atz) * (f4(qv[0], k) + f4(qv[1], k));
-                            grho += -(dt * (bk * bk)) * (avx * f4(qv[3], k) + avz * f4(qv[4], k));
-                            m0[k] = gmu;
-                            m1[k] = glam;
-                            m2[k] = grho;
-                        }
-                    }
-                    st4s(G0, mk4(m0));
-                    st4s(G1, mk4(m1));
-                    st4s(G2, mk4(m2));
+                if (RB < 3) {
+                    image_stress(r, o.gj0, qv[0], qv[1], qv[2]);
+                    image_velocity(r, o.gj0, om_of(o), b, qv[3], qv[4]);
+                    if (r + 1 < RB) load_set(t, r + 1);
                 }
-                if (r + 1 < RB) load_set(t, r + 1);
-                if (epi && res_v && rs[r]) {  // what step t - 1 finds in its input
-                    if (a.res[VX]) inject(vx[r], t - 1, VX, rs[r]);
-                    if (a.res[VZ]) inject(vz[r], t - 1, VZ, rs[r]);
+                float4 px = vx[r], pzz = vz[r];
+                if (epi && res_v && rs[r]) {  // with what step t - 1 finds in its input
+                    if (a.res[VX]) inject(px, t - 1, VX, rs[r]);
+                    if (a.res[VZ]) inject(pzz, t - 1, VZ, rs[r]);
                 }
-                const float4 px = times4(vx[r], b), pzz = times4(vz[r], b);
-                st4s(s_pvx + ot + r * W, px);
-                st4s(s_pvz + ot + r * W, pzz);
+                if (RB < 3) {
+                    vx[r] = px;
+                    vz[r] = pzz;
+                }
+                px = times4(px, b);
+                pzz = times4(pzz, b);
+                st4s(s_pvx + o.ot + r * W, px);
+                st4s(s_pvz + o.ot + r * W, pzz);
                 if (!inside) {
-                    const int s = strip_group(br + r);
+                    const int s = strip_group(o.br + r, o.bq);
                     if (s >= 0) {
                         st_word(xo + 4 * s, px.x, px.y, px.z, tag);
                         st_word(xo + 4 * s + 1, px.w, pzz.x, pzz.y, tag);
@@ -1271,6 +1428,26 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
             }
         }
         __syncthreads();
+        if (RB == 3 && mine) {  // with the strips on their way
+            cp_wait<0>();
+            {
+                const Own o = place();
+                const float *gb = a.mat + 2 * P + co_of(o);
+#pragma unroll
+                for (int r = 0; r < RB; ++r)
+                    image_velocity(r, o.gj0, om_of(o), __ldg(reinterpret_cast<const float4 *>(gb + r * g.pitch)),
+                                   set_at(r == 0 ? 3 : r == 1 ? 0 : 2), set_at(r == 0 ? 4 : r == 1 ? 1 : 5));
+            }
+            if (epi && res_v) {
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    if (!rs[r]) continue;
+                    if (a.res[VX]) inject(vx[r], t - 1, VX, rs[r]);
+                    if (a.res[VZ]) inject(vz[r], t - 1, VZ, rs[r]);
+                }
+            }
+            if (t > p.t_lo) ask_first(t - 1);
+        }
     }
     if (!mine) return;
     // the state that step t_lo - 1 finds, its residual included
@@ -1287,7 +1464,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
         }
         if (stop) {
             vx[r] = vz[r] = ax[r] = az[r] = axz[r] = make_float4(nan, nan, nan, nan);
-            for (int f = 0; f < 3; ++f) st4s(s_g + f * OP + og + r * OW, vx[r]);
+            gmu[r] = glam[r] = vx[r];
+            if (RB < 2)
+                grho = vx[r];
+            else
+                st4s(s_rho + om + r * OM, vx[r]);
         }
         float *o = out + co + r * g.pitch;
         *reinterpret_cast<float4 *>(o + VX * P) = vx[r];
@@ -1295,9 +1476,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
         *reinterpret_cast<float4 *>(o + TXX * P) = ax[r];
         *reinterpret_cast<float4 *>(o + TZZ * P) = az[r];
         *reinterpret_cast<float4 *>(o + TXZ * P) = axz[r];
-#pragma unroll
-        for (int f = 0; f < 3; ++f)
-            *reinterpret_cast<float4 *>(G + f * P + co + r * g.pitch) = ld4s(s_g + f * OP + og + r * OW);
+        *reinterpret_cast<float4 *>(G + co + r * g.pitch) = gmu[r];
+        *reinterpret_cast<float4 *>(G + P + co + r * g.pitch) = glam[r];
+        *reinterpret_cast<float4 *>(G + 2 * P + co + r * g.pitch) = RB < 2 ? grho : ld4s(s_rho + om + r * OM);
     }
 }
 

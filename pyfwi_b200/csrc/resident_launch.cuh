@@ -23,6 +23,13 @@ inline int res_slots(int R, const Lines &L, int th, int nq)
     return n;
 }
 
+// Shared memory of the adjoint loop without its staged residuals, in floats.
+template <int R>
+constexpr size_t adj_res_floats(int rb)
+{
+    return rb == 1 ? ADJ_RES_FLOATS<R, 1> : rb == 2 ? ADJ_RES_FLOATS<R, 2> : ADJ_RES_FLOATS<R, 3>;
+}
+
 template <int R>
 cudaError_t launch_fwd_resident_r(FwdResArgs &a, cudaStream_t s)
 {
@@ -38,7 +45,7 @@ cudaError_t launch_adj_resident_r(AdjResArgs &a, cudaStream_t s)
 {
     const int th = a.tl.rb * a.tl.bz;
     a.slots = res_slots(R, a.a.lines, th, a.tl.nq);
-    const size_t f = ADJ_RES_FLOATS<R> + RES_SLOT_FLOATS * (size_t)a.slots;
+    const size_t f = adj_res_floats<R>(a.tl.rb) + RES_SLOT_FLOATS * (size_t)a.slots;
 #define CASE(RB_) \
     if (a.tl.rb == RB_) return launch_resident(reinterpret_cast<const void *>(adj_resident<R, RB_>), a, f, s);
     CASE(1) CASE(2) CASE(3)
