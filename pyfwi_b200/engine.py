@@ -76,8 +76,9 @@ class Plan:
     def query(geom, opts):
         """(workspace bytes, pyfwi_plan_flags) of a plan with these settings."""
         L = N.lib()
-        srcx = np.zeros(geom.ns, np.int32)
-        srcz = np.zeros(geom.ns, np.int32)
+        # sources in the middle of the model: some options apply only to sources in the update domain
+        srcx = np.full(geom.ns, geom.npml + geom.nx // 2, np.int32)
+        srcz = np.full(geom.ns, geom.npml + geom.nz // 2, np.int32)
         h = ctypes.c_void_p()
         N.check(L.pyfwi_plan_create(ctypes.byref(geom), srcx.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
                                     srcz.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), ctypes.byref(opts),
