@@ -84,3 +84,24 @@ def test_device_lowpass_shapes_match_oracle(planes, nt, ncols, hc):
     assert rel_l2(y.cpu().numpy(), ref) < 1e-5, rel_l2(y.cpu().numpy(), ref)
     for p in range(planes):  # each plane on its own too
         assert rel_l2(y[p].cpu().numpy(), ref[p]) < 1e-5
+
+
+@pytest.mark.parametrize("logn", range(1, 15))
+def test_device_lowpass_every_transform_length(logn):
+    """Every split of the transform into passes, at the longest record and at
+    the shortest one of its length, with trace counts around a CTA's pairs
+    (odd ones, and pairs that are no aligned float2).  White noise through a
+    transform of n points and back keeps a relative error of the order of
+    2^-24 per level and direction: 2^-23 log2 n."""
+    import torch
+    from pyfwi_b200 import fwi_tools
+    n = 1 << logn
+    for nt in sorted({max(1, n // 4 + 1), n // 2}):
+        assert fwi_tools.lowpass_spectrum(nt, 20.0, FN, 3)[0] == n
+        for ncols in (1, 2, 7, 8, 10):
+            rng = np.random.default_rng(nt * 16 + ncols)
+            x = rng.standard_normal((2, nt, ncols)).astype(np.float32)
+            y = fwi_tools.lowpass(torch.from_numpy(x).cuda(), 20.0, FN, order=3, axis=1).cpu().numpy()
+            spec = np.float64(fwi_tools.lowpass_spectrum(nt, 20.0, FN, 3)[1][:n]) * n
+            ref = np.fft.ifft(np.fft.fft(x.astype(np.float64), n, axis=1) * spec[None, :, None], axis=1).real[:, :nt]
+            assert rel_l2(y, ref) < 2.0 ** -23 * logn, (nt, ncols, rel_l2(y, ref))
