@@ -141,9 +141,12 @@ typedef struct pyfwi_options {
                                otherwise (and inside a caller's stream capture) one launch per step.
                                2: resident time loops, one cooperative launch per run of steps
                                and few shots with the wavefield kept on chip, where checkpoint
-                               segments hold difference sets in FP32 (store_diffs), no overlap is
-                               on, every source lies in the update domain and the grid fits on
-                               the SMs (up to about 600,000 cells); the step kernels otherwise */
+                               segments hold difference sets in FP32 (store_diffs), or the sets
+                               can be formed from FP32 states (energy terms, reverse checkpoints;
+                               a chunk of sets more in the workspace), for the reference adjoint,
+                               no overlap is on, every source lies in the update domain and the
+                               grid fits on the SMs (up to about 600,000 cells); the step kernels
+                               otherwise */
     int32_t overlap;        /* 1: exact checkpoints in FP32 with recompute segments: recompute
                                segment m-1 on a second stream of the plan while the adjoint of
                                segment m runs (two segment buffers in the workspace) */

@@ -187,6 +187,50 @@ __device__ __forceinline__ void adj_sums(float lam, float mu, float atx, float a
     pz = __fmaf_rn(lam, atx, __fmul_rn(l2m, atz));
 }
 
+// Grad (elastic.cl:470-560): what a step adds to the accumulators of mu and lam
+// (new adjoint stresses, the differences Dx+ vx, Dz- vz and Dz+ vx + Dx- vz of
+// the forward state) and of rho (new adjoint velocities, the sums of the stress
+// differences), and the energy terms: e0 += p0, e1 += p1 * q1, e2 += dt^2 s2.
+// Every rounding is spelled out, so that whichever kernels run a survey, its
+// gradient has the same bits.
+__device__ __forceinline__ void image_stress_terms(float dt, float atx, float atz, float atxz, float q0, float q1, float q2,
+                                                   float &gmu, float &glam)
+{
+    gmu = __fadd_rn(gmu, __fmaf_rn(__fmul_rn(dt, atxz), q2,
+                                   __fmul_rn(2.f * dt, __fmaf_rn(atx, q0, __fmul_rn(atz, q1)))));
+    glam = __fmaf_rn(__fmul_rn(dt, __fadd_rn(atx, atz)), __fadd_rn(q0, q1), glam);
+}
+
+__device__ __forceinline__ void image_velocity_terms(float dt, float b, float avx, float avz, float q3, float q4, float &grho)
+{
+    grho = __fmaf_rn(-__fmul_rn(dt, __fmul_rn(b, b)), __fmaf_rn(avx, q3, __fmul_rn(avz, q4)), grho);
+}
+
+struct EnergyTerms {
+    float p0, p1, q1, s2;
+};
+__device__ __forceinline__ EnergyTerms energy_terms(float dt, float vx, float vz, float tx, float tz, float txz, float dxp_vx,
+                                                    float dzm_vz, float dzp_vx, float dxm_vz, float dxm_tx, float dzm_txz,
+                                                    float dzp_tz, float dxp_txz)
+{
+    const float dt2 = __fmul_rn(dt, dt);
+    auto sq2 = [](float a, float b) { return __fmaf_rn(a, a, __fmul_rn(b, b)); };
+    const float fx = __fmul_rn(tx, dxp_vx), fz = __fmul_rn(tz, dzm_vz);
+    EnergyTerms e;
+    e.p0 = __fmaf_rn(__fmul_rn(dt2, __fmul_rn(txz, txz)), sq2(dzp_vx, dxm_vz), __fmul_rn(4.f * dt2, sq2(fx, fz)));
+    e.p1 = __fmul_rn(dt2, sq2(tx, tz));
+    e.q1 = sq2(dxp_vx, dzm_vz);
+    e.s2 = __fmaf_rn(__fmul_rn(vx, vx), sq2(dxm_tx, dzm_txz), __fmul_rn(__fmul_rn(vz, vz), sq2(dzp_tz, dxp_txz)));
+    return e;
+}
+
+__device__ __forceinline__ void add_energy(const EnergyTerms &e, float dt, float &e0, float &e1, float &e2)
+{
+    e0 = __fadd_rn(e0, e.p0);
+    e1 = __fmaf_rn(e.p1, e.q1, e1);
+    e2 = __fmaf_rn(__fmul_rn(dt, dt), e.s2, e2);
+}
+
 // Differences of (lam + 2 mu) * A.
 template <int R>
 __device__ __forceinline__ float dfwd_l2m(const float *lam, const float *mu, const float *A, int i, int s,
@@ -1467,17 +1511,12 @@ __device__ __forceinline__ void adj_tile(const AdjArgs &a, const V &av, int bx, 
 #pragma unroll
                     for (int f = 0; f < NACC; ++f) img[f] = s_acc[(f * TZ + r) * TX + c];
                 }
-                img[0] += 2.f * dt * (atx * dxp_vx + atz * dzm_vz) + dt * atxz * (dzp_vx + dxm_vz);
-                img[1] += dt * (atx + atz) * (dxp_vx + dzm_vz);
-                img[2] += -(dt * (b * b)) * (avx * (dxm_tx + dzm_txz) + avz * (dzp_tz + dxp_txz));
-                if (ENERGY) {
-                    float dt2 = dt * dt;
-                    img[3 % NACC] += 4.f * dt2 * (tx * tx * dxp_vx * dxp_vx + tz * tz * dzm_vz * dzm_vz) +
-                                     dt2 * txz * txz * (dzp_vx * dzp_vx + dxm_vz * dxm_vz);
-                    img[4 % NACC] += dt2 * (tx * tx + tz * tz) * (dxp_vx * dxp_vx + dzm_vz * dzm_vz);
-                    img[5 % NACC] += dt2 * (vx * vx * (dxm_tx * dxm_tx + dzm_txz * dzm_txz) +
-                                            vz * vz * (dzp_tz * dzp_tz + dxp_txz * dxp_txz));
-                }
+                image_stress_terms(dt, atx, atz, atxz, dxp_vx, dzm_vz, dzp_vx + dxm_vz, img[0], img[1]);
+                image_velocity_terms(dt, b, avx, avz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, img[2]);
+                if (ENERGY)
+                    add_energy(energy_terms(dt, vx, vz, tx, tz, txz, dxp_vx, dzm_vz, dzp_vx, dxm_vz, dxm_tx, dzm_txz, dzp_tz,
+                                            dxp_txz),
+                               dt, img[3 % NACC], img[4 % NACC], img[5 % NACC]);
                 if (NS == 1) {
 #pragma unroll
                     for (int f = 0; f < NACC; ++f) G[f * P + co] = img[f];
@@ -1735,9 +1774,8 @@ __global__ void __launch_bounds__(NTHREADS, (R == 2 && !ENERGY) ? (PF ? 5 : 6) :
                         q2 = qld<QD>(F, F16, F8, Q_VZS * P + co), q3 = qld<QD>(F, F16, F8, Q_TXS * P + co),
                         q4 = qld<QD>(F, F16, F8, Q_TZS * P + co);
             float gmu = G[0 * P + co], glam = G[1 * P + co], grho = G[2 * P + co];
-            gmu += 2.f * dt * (atx * q0 + atz * q1) + dt * atxz * q2;
-            glam += dt * (atx + atz) * (q0 + q1);
-            grho += -(dt * (b * b)) * (avx * q3 + avz * q4);
+            image_stress_terms(dt, atx, atz, atxz, q0, q1, q2, gmu, glam);
+            image_velocity_terms(dt, b, avx, avz, q3, q4, grho);
             G[0 * P + co] = gmu;
             G[1 * P + co] = glam;
             G[2 * P + co] = grho;
@@ -1745,20 +1783,14 @@ __global__ void __launch_bounds__(NTHREADS, (R == 2 && !ENERGY) ? (PF ? 5 : 6) :
         float gmu = PF ? s_g[(0 * TZ + r) * TX + c] : G[0 * P + co];
         float glam = PF ? s_g[(1 * TZ + r) * TX + c] : G[1 * P + co];
         float grho = PF ? s_g[(2 * TZ + r) * TX + c] : G[2 * P + co];
-        gmu += 2.f * dt * (atx * dxp_vx + atz * dzm_vz) + dt * atxz * (dzp_vx + dxm_vz);
-        glam += dt * (atx + atz) * (dxp_vx + dzm_vz);
-        grho += -(dt * (b * b)) * (avx * (dxm_tx + dzm_txz) + avz * (dzp_tz + dxp_txz));
+        image_stress_terms(dt, atx, atz, atxz, dxp_vx, dzm_vz, dzp_vx + dxm_vz, gmu, glam);
+        image_velocity_terms(dt, b, avx, avz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, grho);
         G[0 * P + co] = gmu;
         G[1 * P + co] = glam;
         G[2 * P + co] = grho;
-        if (ENERGY) {
-            float dt2 = dt * dt;
-            G[3 * P + co] += 4.f * dt2 * (tx * tx * dxp_vx * dxp_vx + tz * tz * dzm_vz * dzm_vz) +
-                             dt2 * txz * txz * (dzp_vx * dzp_vx + dxm_vz * dxm_vz);
-            G[4 * P + co] += dt2 * (tx * tx + tz * tz) * (dxp_vx * dxp_vx + dzm_vz * dzm_vz);
-            G[5 * P + co] += dt2 * (vx * vx * (dxm_tx * dxm_tx + dzm_txz * dzm_txz) +
-                                    vz * vz * (dzp_tz * dzp_tz + dxp_txz * dxp_txz));
-        }
+        if (ENERGY)
+            add_energy(energy_terms(dt, vx, vz, tx, tz, txz, dxp_vx, dzm_vz, dzp_vx, dxm_vz, dxm_tx, dzm_txz, dzp_tz, dxp_txz), dt,
+                       G[3 * P + co], G[4 * P + co], G[5 * P + co]);
         }
         }
         // the residual the next step injects (Adj_injSrc, elastic_surface.cl:48-71),
@@ -1784,6 +1816,80 @@ __global__ void __launch_bounds__(256) qstress_kernel(Grid g, Coef k, const floa
     const float *S = in + blockIdx.z * in_stride;
     qst1<QD>(q, q8, qo + Q_TXS * P, gbwd<R>(S + TXX * P, co, 1, k.cx) + gbwd<R>(S + TXZ * P, co, g.pitch, k.cz));
     qst1<QD>(q, q8, qo + Q_TZS * P, gfwd<R>(S + TZZ * P, co, g.pitch, k.cz) + gfwd<R>(S + TXZ * P, co, 1, k.cx));
+}
+
+// Difference sets of stored states, for an adjoint that reads sets: step s of
+// the nsteps given (in backward order, the sets in the same order) has its state
+// at S[s].  The imaging domain only.  Without ENERGY a block takes one step
+// (blockIdx.z = slot * nsteps + step).  With it the energy terms are added to
+// accumulators 3 to 5, which depend on the forward states alone: four threads
+// work out the terms of four steps of a cell and one adds them up in adj_step's
+// order (one thread per cell: too few in flight, 141 us a launch of 64 steps of 4 shots of 100 x 150
+// cells, eighth order, against 80).  It reads 20 bytes of state per cell and step and writes 20.
+constexpr int SETS_STEPS = 64;  // steps of a launch, at most
+struct SetsArgs {
+    Grid g;
+    Coef k;
+    int npml, nsteps;
+    const float *S[SETS_STEPS];
+    long long s_stride[SETS_STEPS];
+    float *q;                // set of step s, slot 0, at q + s * q_step
+    long long q_step, q_stride;
+    float *gacc;
+    long long gacc_stride;
+};
+
+template <int R, bool ENERGY>
+__global__ void __launch_bounds__(256) sets_kernel(const __grid_constant__ SetsArgs a)
+{
+    const Grid &g = a.g;
+    const int glo = a.npml + R;
+    constexpr int TG = ENERGY ? 4 : 1, ROWS = 8 / TG;  // threads per cell, rows per block
+    __shared__ EnergyTerms part[TG][ROWS * 32];
+    const int cell = threadIdx.x % (ROWS * 32), tg = threadIdx.x / (ROWS * 32);
+    const int j = glo + blockIdx.x * 32 + cell % 32, i = glo + blockIdx.y * ROWS + cell / 32;
+    const bool in = i <= g.tnz - R - a.npml && j <= g.tnx - R - a.npml;
+    const int slot = ENERGY ? blockIdx.z : blockIdx.z / a.nsteps;
+    const long long P = g.plane, co = cell_off(g, i, j);
+    float e0 = 0.f, e1 = 0.f, e2 = 0.f;  // (in the cell's first thread)
+    float *const G = ENERGY ? a.gacc + slot * a.gacc_stride + co + 3 * P : nullptr;
+    if (ENERGY && in && tg == 0) {
+        e0 = G[0];
+        e1 = G[P];
+        e2 = G[2 * P];
+    }
+    const int first = ENERGY ? 0 : blockIdx.z % a.nsteps, end = ENERGY ? a.nsteps : first + 1;
+    for (int s0 = first; s0 < end; s0 += TG) {
+        const int s = s0 + tg;
+        if (in && s < end) {
+            const float *F = a.S[s] + slot * a.s_stride[s];
+            // DzpVx is formed from vz, as the reference does (elastic.cl:485)
+            const float dzp_vx = gfwd<R>(F + VZ * P, co, g.pitch, a.k.cz), dxm_vz = gbwd<R>(F + VZ * P, co, 1, a.k.cx);
+            const float dxp_vx = gfwd<R>(F + VX * P, co, 1, a.k.cx), dzm_vz = gbwd<R>(F + VZ * P, co, g.pitch, a.k.cz);
+            const float dzp_tz = gfwd<R>(F + TZZ * P, co, g.pitch, a.k.cz), dxm_tx = gbwd<R>(F + TXX * P, co, 1, a.k.cx);
+            const float dxp_txz = gfwd<R>(F + TXZ * P, co, 1, a.k.cx), dzm_txz = gbwd<R>(F + TXZ * P, co, g.pitch, a.k.cz);
+            float *q = a.q + s * a.q_step + slot * a.q_stride + co;
+            q[Q_DXP_VX * P] = dxp_vx;
+            q[Q_DZM_VZ * P] = dzm_vz;
+            q[Q_VZS * P] = dzp_vx + dxm_vz;
+            q[Q_TXS * P] = dxm_tx + dzm_txz;
+            q[Q_TZS * P] = dzp_tz + dxp_txz;
+            if (ENERGY)
+                part[tg][cell] = energy_terms(a.k.dt, F[VX * P + co], F[VZ * P + co], F[TXX * P + co], F[TZZ * P + co],
+                                              F[TXZ * P + co], dxp_vx, dzm_vz, dzp_vx, dxm_vz, dxm_tx, dzm_txz, dzp_tz, dxp_txz);
+        }
+        if constexpr (ENERGY) {
+            __syncthreads();
+            if (in && tg == 0)  // in adj_step's order
+                for (int k = 0; k < TG && s0 + k < end; ++k) add_energy(part[k][cell], a.k.dt, e0, e1, e2);
+            __syncthreads();
+        }
+    }
+    if (ENERGY && in && tg == 0) {
+        G[0] = e0;
+        G[P] = e1;
+        G[2 * P] = e2;
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -105,6 +105,7 @@ struct pyfwi_plan {
     bool exact_adj = false;  // PYFWI_ADJOINT_EXACT
     bool persist = false;    // time loops as persistent kernels (options.persist, where the layout allows)
     bool resident = false;   // time loops with the wavefield on chip (options.persist 2, where it fits)
+    int rchunk = 0;          // resident without sets in the store: steps whose sets are formed from their states at a time
     int sms = 0;             // SMs of the device the resident launches run on (0: not asked yet)
     unsigned tag = 1;        // next unused tag of the exchange buffer in this call
     bool overlap = false;    // recompute of segment m-1 on a second stream beside the adjoint of segment m
@@ -115,7 +116,7 @@ struct pyfwi_plan {
     int fwd_cap = 0, adj_cap = 0;  // co-resident CTAs of the persistent kernels on this device
     long long state;  // floats per state (5 planes)
     // workspace offsets in bytes
-    size_t o_hdr, o_src, o_red, o_mat, o_dampx, o_dampz, o_work, o_adj, o_gacc, o_store, o_store16, o_store8, o_xch, total;
+    size_t o_hdr, o_src, o_red, o_mat, o_dampx, o_dampz, o_work, o_adj, o_gacc, o_store, o_store16, o_store8, o_xch, o_sets, o_states, total;
     long long launches = 0;
     bool model_set = false, fwd_valid = false;
     // per-kernel event timing (pyfwi_profile_enable)
@@ -858,7 +859,7 @@ Buf slot_of(const Buf &b, int slot) { return {b.base + slot * b.stride, b.stride
 
 // Forward steps [t0, t1) of slots c0 .. c0 + n - 1 of the group starting at
 // shot s0, from state `in` (slot 0's) to `out`; sets: their difference sets
-// (null: none), the first of which is that of step q_t0.  Several launches
+// or states (null: neither is stored), the first of which is that of step q_t0.  Several launches
 // when more source samples than travel with one are not zero.
 int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl, int t0, int t1, const Buf &in,
                      const Buf &out, float *traces, const Buf *sets, int q_t0, cudaStream_t st)
@@ -877,6 +878,7 @@ int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl
     fa.record = traces != nullptr;
     fa.q_t0 = q_t0;
     if (sets) {
+        fa.store = p->qd ? 1 : 2;
         fa.q = slot_of(*sets, c0).base;
         fa.a.q_stride = sets->stride;
     }
@@ -910,10 +912,10 @@ int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl
     return PYFWI_OK;
 }
 
-// Adjoint steps t_hi - 1 .. t_lo of a whole group with the sets of segment m,
-// from adjoint state `ping` to the other one.
-int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, int m, int t_hi, int t_lo, int &ping,
-                     float *adj, cudaStream_t st)
+// Adjoint steps t_hi - 1 .. t_lo of a whole group, from adjoint state `ping`
+// to the other one; sets: the difference sets, from that of step q_t0 on.
+int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, const Buf &sets, int q_t0, int t_hi, int t_lo,
+                     int &ping, float *adj, cudaStream_t st)
 {
     const pyfwi_geometry &G = p->geom;
     if (t_hi - 1 < t_lo) return PYFWI_OK;
@@ -925,7 +927,6 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, int m,
         int rc = launch_inject(p, a, n, st);
         if (rc) return rc;
     }
-    const Buf sets = seg_state(p, ws, m, 0);
     AdjResArgs r;
     memset(&r, 0, sizeof r);
     r.state = p->state;
@@ -934,7 +935,7 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, int m,
     r.nt = G.nt;
     r.nt_ext = G.nt_ext;
     r.dt_scale = G.dt_scale;
-    r.q_t0 = m * p->seg;
+    r.q_t0 = q_t0;
     r.err = at<int>(ws, ERR_OFF);
     r.limit_ns = BARRIER_WAIT_NS;
     ResTiles tl;
@@ -963,8 +964,54 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, int m,
     return PYFWI_OK;
 }
 
+// The same with the sets formed from the states, a chunk of steps at a time;
+// state(t): where S_{t+1} is, called for each step of a chunk in backward
+// order before any of the chunk's sets are formed.
+template <class State>
+int resident_chunks(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, State state, int t_hi, int t_lo, int &ping,
+                    float *adj, cudaStream_t st)
+{
+    SetsArgs a;
+    memset(&a, 0, sizeof a);
+    a.g = p->g;
+    a.k = p->k;
+    a.npml = p->geom.npml;
+    a.q_step = -p->state;
+    a.q_stride = p->rchunk * p->state;
+    a.gacc = base.gacc;
+    a.gacc_stride = base.gacc_stride;
+    const bool energy = p->nacc == 6;
+    const Buf sets = {at<float>(ws, p->o_sets), a.q_stride};
+    for (int hi = t_hi; hi > t_lo;) {
+        const int lo = std::max(t_lo, hi - p->rchunk);
+        a.nsteps = hi - lo;
+        for (int t = hi - 1; t >= lo; --t) {
+            const Buf s = state(t);
+            if (!s.base) return fail(PYFWI_E_STATE, "no state to image at step %d", t);
+            a.S[hi - 1 - t] = s.base;
+            a.s_stride[hi - 1 - t] = s.stride;
+        }
+        a.q = sets.base + (long long)(a.nsteps - 1) * p->state;  // set of step lo first
+        const int iz = p->g.tnz - 2 * (p->R + a.npml) + 1, ix = p->g.tnx - 2 * (p->R + a.npml) + 1;
+        if (iz > 0 && ix > 0) {
+            const int rows = energy ? 2 : 8;  // of a block
+            dim3 grid((ix + 31) / 32, (iz + rows - 1) / rows, energy ? n : n * a.nsteps);
+            if (p->R == 4)
+                energy ? sets_kernel<4, true><<<grid, 256, 0, st>>>(a) : sets_kernel<4, false><<<grid, 256, 0, st>>>(a);
+            else
+                energy ? sets_kernel<2, true><<<grid, 256, 0, st>>>(a) : sets_kernel<2, false><<<grid, 256, 0, st>>>(a);
+            p->launches++;
+            CKL();
+        }
+        int rc = resident_adjoint(p, ws, base, n, sets, lo, hi, lo, ping, adj, st);
+        if (rc) return rc;
+        hi = lo;
+    }
+    return PYFWI_OK;
+}
+
 // The forward pass of a group on chip: restart states, and the difference
-// sets of the last segment.
+// sets or states of the last segment.
 int resident_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
 {
     const int nt = p->geom.nt;
@@ -986,10 +1033,10 @@ int resident_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStr
             if (rc) return rc;
         }
     }
-    return last_diffs(p, ws, p->M - 1, nt, n, st);
+    return p->qd ? last_diffs(p, ws, p->M - 1, nt, n, st) : PYFWI_OK;
 }
 
-// Recompute of segment m on chip: its difference sets.
+// Recompute of segment m on chip: its difference sets or states.
 int resident_recompute(pyfwi_plan *p, void *ws, int s0, int n, int m, cudaStream_t st)
 {
     const int t0 = m * p->seg, t1 = std::min(t0 + p->seg, p->geom.nt);
@@ -1005,7 +1052,7 @@ int resident_recompute(pyfwi_plan *p, void *ws, int s0, int n, int m, cudaStream
                                   slot_of(work_state(p, ws, t1 & 1), c0), nullptr, &sets, t0, st);
         if (rc) return rc;
     }
-    return last_diffs(p, ws, m, t1, n, st);
+    return p->qd ? last_diffs(p, ws, m, t1, n, st) : PYFWI_OK;
 }
 
 int exact_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
@@ -1048,11 +1095,39 @@ Buf chp_state(pyfwi_plan *p, void *ws, int s0, int k)
     return {store + (long long)s0 * stride + (long long)k * p->state, stride};
 }
 
+// The forward pass of a group on chip, from checkpoint to checkpoint.
+int resident_reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
+{
+    ResTiles tl;
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, false, &tl))
+        return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
+    int rc = clear_exchange(p, ws, st);
+    if (rc) return rc;
+    const int conc = tl.nslots;
+    for (int c0 = 0; c0 < n; c0 += conc) {
+        tl.nslots = std::min(conc, n - c0);
+        Buf cur = slot_of(work_state(p, ws, 0), c0);
+        int t = 0;
+        for (size_t kc = 0; t < p->geom.nt; ++kc) {
+            const bool keep = kc < p->chp.size();
+            const int t1 = keep ? p->chp[kc] + 1 : p->geom.nt;
+            const Buf out = slot_of(keep ? chp_state(p, ws, s0, (int)kc) : work_state(p, ws, 1), c0);
+            if (t1 <= t) continue;  // listed again
+            rc = resident_forward(p, ws, s0, c0, tl, t, t1, cur, out, traces, nullptr, 0, st);
+            if (rc) return rc;
+            cur = out;
+            t = t1;
+        }
+    }
+    return PYFWI_OK;
+}
+
 int reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
 {
     // states stored after the steps listed in chp (wave_propagation.py:710-727)
     Buf cur = work_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(cur.base + q * cur.stride, 0, p->state * sizeof(float), st));
+    if (use_resident(p, st)) return resident_reverse_pass(p, ws, s0, n, traces, st);
     int wcur = 0;  // work buffer holding the current state (-1: a checkpoint slot)
     size_t kc = 0;
     StepArgs a = base_step(p, ws);
@@ -1412,7 +1487,11 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
                     if (rc) return rc;
                 }
                 Range range("pyfwi adjoint segment");
-                rc = resident_adjoint(p, ws, a, n, m, t_hi, std::max(t_lo, 1), ping, adj, st);
+                if (p->qd)
+                    rc = resident_adjoint(p, ws, a, n, seg_state(p, ws, m, 0), t_lo, t_hi, std::max(t_lo, 1), ping, adj, st);
+                else
+                    rc = resident_chunks(p, ws, a, n, [&](int t) { return seg_state(p, ws, m, t - t_lo); }, t_hi,
+                                         std::max(t_lo, 1), ping, adj, st);
                 if (rc) return rc;
             }
         } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT) {
@@ -1471,28 +1550,46 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
             Buf cur = {nullptr, 0};
             StepArgs f = base_step(p, ws);
             f.shot0 = s0;
-            for (int t = G.nt - 1; t > 0; --t) {
+            rc = PYFWI_OK;
+            // S_{t+1}: a checkpoint, or reconstructed from S_{t+2} into `to`
+            auto state = [&](int t, const Buf &to) {
                 int kk = chpc >= 0 ? chpc : chpc + nchp;
                 if (t == p->chp[kk]) {
                     cur = chp_state(p, ws, s0, kk);
                     chpc -= 1;
-                } else {
-                    if (!cur.base) return fail(PYFWI_E_STATE, "reverse schedule has no starting checkpoint");
-                    int w = 1 - wlast;
-                    Buf out = work_state(p, ws, w);
-                    f.in = cur.base;
-                    f.in_stride = cur.stride;
-                    f.out = out.base;
-                    f.out_stride = out.stride;
-                    rc = step_fwd(p, f, n, st, true, at<float>(ws, 0));
-                    if (rc) return rc;
-                    cur = out;
-                    wlast = w;
+                    return cur;
                 }
-                a.fwd = cur.base;
-                a.fwd_stride = cur.stride;
-                rc = adjoint_iter(p, ws, a, t, t_src, ping, adj, n, st);
+                if (!cur.base) {
+                    rc = fail(PYFWI_E_STATE, "reverse schedule has no starting checkpoint");
+                    return cur;
+                }
+                f.in = cur.base;
+                f.in_stride = cur.stride;
+                f.out = to.base;
+                f.out_stride = to.stride;
+                rc = step_fwd(p, f, n, st, true, at<float>(ws, 0));
+                cur = rc ? Buf{nullptr, 0} : to;
+                return cur;
+            };
+            if (use_resident(p, st)) {
+                rc = clear_exchange(p, ws, st);
                 if (rc) return rc;
+                const int ring = p->rchunk + 1;  // the newest state of a chunk is still read by the next one's first step
+                auto in_ring = [&](int t) {
+                    return state(t, {at<float>(ws, p->o_states) + (long long)(t % ring) * p->state, ring * p->state});
+                };
+                rc = resident_chunks(p, ws, a, n, in_ring, G.nt, 1, ping, adj, st);
+                if (rc) return rc;
+            } else {
+                for (int t = G.nt - 1; t > 0; --t) {
+                    const Buf s = state(t, work_state(p, ws, 1 - wlast));
+                    if (rc) return rc;
+                    if (s.base == work_state(p, ws, 1 - wlast).base) wlast = 1 - wlast;
+                    a.fwd = s.base;
+                    a.fwd_stride = s.stride;
+                    rc = adjoint_iter(p, ws, a, t, t_src, ping, adj, n, st);
+                    if (rc) return rc;
+                }
             }
         }
     }
@@ -1741,10 +1838,21 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     bool src_in = true;  // every source inside the update domain
     for (int s = 0; s < G.ns; ++s)
         src_in = src_in && srcz[s] >= p->R && srcz[s] <= tnz - p->R && srcx[s] >= p->R && srcx[s] <= tnx - p->R;
-    p->resident = opt->persist == 2 && p->qd == 1 && !p->overlap && src_in &&
+    // (FP32, the reference adjoint, the plain tile kernels), or states that the
+    // sets can be formed from: energy terms, reconstructed states
+    const bool from_states = !p->qd && (p->nacc == 6 || opt->checkpoint != PYFWI_CKPT_EXACT) &&
+                             opt->snapshot == PYFWI_SNAP_FP32 && !p->exact_adj && !p->persist && !p->st_w && !p->ftma &&
+                             !p->ast_w && p->ans == 1 && !p->apf && G.npml + p->R >= 4;
+    p->resident = opt->persist == 2 && (p->qd == 1 || from_states) && !p->overlap && src_in &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, false, &tl) &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, true, &tl);
     if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
+    if (p->resident && !p->qd) {
+        // long enough that the launches' own cost is a small part, in at most 256 MB or half of the states kept
+        const size_t kept = opt->checkpoint == PYFWI_CKPT_EXACT ? (size_t)p->seg : p->chp.size() * G.ns / p->G;
+        const size_t room = (256ull << 20) / ((size_t)p->state * sizeof(float) * p->G);
+        p->rchunk = (int)std::max<size_t>(4, std::min<size_t>({(size_t)SETS_STEPS, room, kept / 2}));
+    }
 
     const size_t pf = (size_t)p->g.plane * sizeof(float), sb = (size_t)p->state * sizeof(float);
     // regions holding planes start on a row of the workspace (a multiple of
@@ -1788,6 +1896,12 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     if (fp24_snaps(p)) o += up((size_t)p->seg * p->state * p->G);
     p->o_xch = o;
     if (p->resident) o += up(RES_XCH_BYTES);
+    o = upr(o);
+    p->o_sets = o;
+    o += up(p->rchunk * sb * p->G);
+    o = upr(o);
+    p->o_states = o;
+    if (opt->checkpoint != PYFWI_CKPT_EXACT && p->rchunk) o += up((p->rchunk + 1) * sb * p->G);
     p->total = o;
     *out = p;
     return PYFWI_OK;

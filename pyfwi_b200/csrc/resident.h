@@ -11,7 +11,6 @@ namespace pyfwi {
 __attribute__((visibility("hidden"))) bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms,
                                                           bool adjoint, ResTiles *out);
 
-// With difference sets (a.q set) or without.
 __attribute__((visibility("hidden"))) cudaError_t launch_fwd_resident(FwdResArgs &a, int R, cudaStream_t s);
 __attribute__((visibility("hidden"))) cudaError_t launch_adj_resident(AdjResArgs &a, int R, cudaStream_t s);
 

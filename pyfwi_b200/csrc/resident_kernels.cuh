@@ -137,8 +137,9 @@ struct FwdResArgs {
     long long state;   // floats per state
     int t0, t1;
     int dt_scale, nt_ext, record;
-    float *q;          // difference sets of slot 0 (a.q_stride apart): the set of S_{t+1} at q + (t - q_t0) * state
-    int q_t0;
+    float *q;          // difference sets (store 1) or states (2) of slot 0 (a.q_stride apart): S_{t+1}'s at
+                       // q + (t - q_t0) * state
+    int q_t0, store;
     int *err;
     unsigned long long limit_ns;
     int k0, nk;        // samples k0 .. k0 + nk - 1 are in wav, the others are zero
@@ -443,6 +444,7 @@ __device__ __forceinline__ void res_block(const ResTile &t, int e, int &bz, int 
 // ---------------------------------------------------------------------------
 // forward steps t0 .. t1 - 1 (fwd_step's arithmetic)
 // ---------------------------------------------------------------------------
+// QD: 1 stores the difference sets of the states, 2 the states, 0 neither.
 template <int R, int RB, int QD>
 __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_constant__ FwdResArgs p)
 {
@@ -560,7 +562,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         lam[r] = masked(a.mat, gi, gj0);
         mu[r] = masked(a.mat + P, gi, gj0);
         damp = damp || damped(gi, gj0);
-        if (QD && gi >= a.qlo && gi <= a.qhi_z && gj0 + 3 >= a.qlo && gj0 <= a.qhi_x) img |= 1u << r;
+        if (QD == 1 && gi >= a.qlo && gi <= a.qhi_z && gj0 + 3 >= a.qlo && gj0 <= a.qhi_x) img |= 1u << r;
     }
 
     // The strip group of row r of the tile in this thread's column, -1: none.
@@ -613,7 +615,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     s[k] = xbwd<R>(x, k, a.k.cx) + z.at(r, k, a.k.cz);
                     n[k] = f4(vx[r], k) + dt * (f4(b[r], k) * s[k]);
                 }
-                if (QD && qi && (img >> r & 1)) qst4s(qi + Q_TXS * P + co + r * g.pitch, mk4(s));
+                if (QD == 1 && qi && (img >> r & 1)) qst4s(qi + Q_TXS * P + co + r * g.pitch, mk4(s));
                 vx[r] = mk4(n);
             }
         }
@@ -628,7 +630,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     s[k] = z.at(r, k, a.k.cz) + xfwd<R>(x, k, a.k.cx);
                     n[k] = f4(vz[r], k) + dt * (f4(b[r], k) * s[k]);
                 }
-                if (QD && qi && (img >> r & 1)) qst4s(qi + Q_TZS * P + co + r * g.pitch, mk4(s));
+                if (QD == 1 && qi && (img >> r & 1)) qst4s(qi + Q_TZS * P + co + r * g.pitch, mk4(s));
                 vz[r] = mk4(n);
             }
         }
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     ez[k] = zz.at(r, k, a.k.cz);
                 }
                 hx[r] = mk4(h);
-                if (QD && (img >> r & 1)) {
+                if (QD == 1 && (img >> r & 1)) {
                     float *q = qo + co + r * g.pitch, s[4];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) s[k] = zi.at(r, k, a.k.cz) + h[k];
@@ -769,7 +771,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         float *qi = nullptr, *qo = nullptr;
         if constexpr (QD) {
             qo = p.q + (long long)(t - p.q_t0) * p.state + T.slot * a.q_stride;
-            if (t > p.q_t0) qi = qo - p.state;
+            if (QD == 1 && t > p.q_t0) qi = qo - p.state;
         }
         if (add) {
             __syncthreads();
@@ -820,7 +822,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         }
         if (stop) break;
         for (int e = rank; e < nring; e += NT) ring(e);
-        if constexpr (QD) {
+        if constexpr (QD == 1) {
             // the stress differences near the source cell again, without this
             // step's source (see fwd_step)
             if (qi && add) {
@@ -843,6 +845,19 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         }
         __syncthreads();
         if (mine) stress(strip + ((t + 1) & 1) * xpar, p.tag0 + (unsigned)(t + 1 - p.t0), qo);
+        if constexpr (QD == 2) {
+            if (mine)
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    if (gi0 + r >= g.tnz) break;
+                    float *o = qo + co + r * g.pitch;
+                    qst4s(o + VX * P, vx[r]);
+                    qst4s(o + VZ * P, vz[r]);
+                    qst4s(o + TXX * P, sxx[r]);
+                    qst4s(o + TZZ * P, szz[r]);
+                    qst4s(o + TXZ * P, sxz[r]);
+                }
+        }
         if (rec_o >= 0 && t + 1 < p.t1 && sub + 1 == p.dt_scale && k + 1 < p.nt_ext) record_v(k + 1);
         if (++sub == p.dt_scale) {
             sub = 0;
@@ -1169,12 +1184,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
                 m1[k] = f4(glam[r], k);
                 if (gj0 + k >= glo && gj0 + k <= ghi_x) {
                     const float atx = f4(ax[r], k), atz = f4(az[r], k), atxz = f4(axz[r], k);
-                    float gm = m0[k], gl = m1[k];
-                    gm += __fmaf_rn(__fmul_rn(dt, atxz), f4(q2, k),
-                                    __fmul_rn(2.f * dt, __fmaf_rn(atx, f4(q0, k), __fmul_rn(atz, f4(q1, k)))));
-                    gl += dt * (atx + atz) * (f4(q0, k) + f4(q1, k));
-                    m0[k] = gm;
-                    m1[k] = gl;
+                    image_stress_terms(dt, atx, atz, atxz, f4(q0, k), f4(q1, k), f4(q2, k), m0[k], m1[k]);
                 }
             }
             gmu[r] = mk4(m0);
@@ -1191,9 +1201,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
                 m2[k] = f4(gr4, k);
                 if (gj0 + k >= glo && gj0 + k <= ghi_x) {
                     const float bk = f4(b, k), avx = f4(vx[r], k), avz = f4(vz[r], k);
-                    float gr = m2[k];
-                    gr += -(dt * (bk * bk)) * (avx * f4(q3, k) + avz * f4(q4, k));
-                    m2[k] = gr;
+                    image_velocity_terms(dt, bk, avx, avz, f4(q3, k), f4(q4, k), m2[k]);
                 }
             }
             if (RB < 2)

@@ -589,23 +589,19 @@ __global__ void __launch_bounds__(W - 2 * R) adj_stream(const __grid_constant__ 
                 const float b = b_r[ai + rc];
                 float gmu = s_g[0 * NQ * W + gi + rc], glam = s_g[1 * NQ * W + gi + rc],
                       grho = s_g[2 * NQ * W + gi + rc];
-                gmu += 2.f * dt * (atx0 * dxp_vx + atz0 * dzm_vz) + dt * atxz0 * (dzp_vx + dxm_vz);
-                glam += dt * (atx0 + atz0) * (dxp_vx + dzm_vz);
-                grho += -(dt * (b * b)) * (avx * (dxm_tx + dzm_txz) + avz * (dzp_tz + dxp_txz));
+                image_stress_terms(dt, atx0, atz0, atxz0, dxp_vx, dzm_vz, dzp_vx + dxm_vz, gmu, glam);
+                image_velocity_terms(dt, b, avx, avz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, grho);
                 G[0 * P + co] = gmu;
                 G[1 * P + co] = glam;
                 G[2 * P + co] = grho;
                 if constexpr (ENERGY) {
-                    const float dt2 = dt * dt, vx = fvx[fi + rc], vz = fvz[fi + rc], tx = ftx[fi + rc],
-                                tz = ftz[fi + rc], txz = ftxz[fi + rc];
-                    G[3 * P + co] = s_g[3 * NQ * W + gi + rc] +
-                                    (4.f * dt2 * (tx * tx * dxp_vx * dxp_vx + tz * tz * dzm_vz * dzm_vz) +
-                                     dt2 * txz * txz * (dzp_vx * dzp_vx + dxm_vz * dxm_vz));
-                    G[4 * P + co] = s_g[4 * NQ * W + gi + rc] +
-                                    dt2 * (tx * tx + tz * tz) * (dxp_vx * dxp_vx + dzm_vz * dzm_vz);
-                    G[5 * P + co] = s_g[5 * NQ * W + gi + rc] +
-                                    dt2 * (vx * vx * (dxm_tx * dxm_tx + dzm_txz * dzm_txz) +
-                                           vz * vz * (dzp_tz * dzp_tz + dxp_txz * dxp_txz));
+                    const float vx = fvx[fi + rc], vz = fvz[fi + rc], tx = ftx[fi + rc], tz = ftz[fi + rc], txz = ftxz[fi + rc];
+                    float e0 = s_g[3 * NQ * W + gi + rc], e1 = s_g[4 * NQ * W + gi + rc], e2 = s_g[5 * NQ * W + gi + rc];
+                    add_energy(energy_terms(dt, vx, vz, tx, tz, txz, dxp_vx, dzm_vz, dzp_vx, dxm_vz, dxm_tx, dzm_txz, dzp_tz, dxp_txz),
+                               dt, e0, e1, e2);
+                    G[3 * P + co] = e0;
+                    G[4 * P + co] = e1;
+                    G[5 * P + co] = e2;
                 }
             }
         }

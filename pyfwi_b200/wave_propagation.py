@@ -30,7 +30,8 @@ stores every step in FP32 and the tile kernels run: True, False, or 'auto':
 on where a step carries at most 2 M cell-shots; absent, with ``tile`` and
 ``adj_tile`` absent and ``graph`` not True: the resident time loops, which keep
 the wavefield on chip for whole runs of steps, where a grid fits and exact
-checkpoints hold difference sets in FP32 -- the same bits as False),
+checkpoints hold difference sets in FP32, energy terms are asked for or states
+are reconstructed -- the same bits as False),
 ``overlap`` (exact checkpoints in FP32 with recompute segments: recompute
 segment m - 1 on a second CUDA stream while the adjoint of segment m runs,
 with two segment buffers), ``store`` ('differences', the default: in exact
@@ -307,6 +308,9 @@ class WavePreparation:
         srcz = np.asarray(self.srcz, np.int32).reshape(-1)
         chp = np.asarray(self.chp, np.int32) if mode == "reverse" else None
 
+        # unless step kernels or a graph of them were asked for
+        resident = self.persist_allowed and not {"tile", "adj_tile"} & set(inpa) and inpa.get("graph") not in (True, 1)
+
         def opts(seg, batch):
             o = N.Options()
             o.checkpoint = N.CKPT_EXACT if mode == "exact" else N.CKPT_REVERSE
@@ -320,8 +324,8 @@ class WavePreparation:
             o.graph = int(self._graph_on(inpa.get("graph", "auto"), batch, seg))
             if "persist" in inpa:
                 o.persist = int(self._persist_on(inpa["persist"], batch))
-            elif self.persist_allowed and not {"tile", "adj_tile"} & set(inpa) and inpa.get("graph") not in (True, 1):
-                o.persist = RESIDENT  # no step kernel and no graph of them was asked for
+            elif resident:
+                o.persist = RESIDENT
             o.overlap = int(bool(inpa.get("overlap", OVERLAP_DEFAULT)))
             o.store_diffs = int(store == "differences")
             o.chunk = int(inpa.get("chunk", 0))
@@ -350,8 +354,18 @@ class WavePreparation:
         variants = (0 if tile == "auto" else int(tile), 0 if adj_tile is None else int(adj_tile) + 1)
         seg = int(inpa.get("segment", 0))
         batch = int(inpa.get("shot_batch", 0))
-        if mode == "exact" and ("segment" not in inpa or "shot_batch" not in inpa):
-            seg, batch = self._auto_layout(geom, opts, seg, batch)
+        asked = seg, batch
+        while True:
+            try:
+                if mode == "exact" and ("segment" not in inpa or "shot_batch" not in inpa):
+                    seg, batch = self._auto_layout(geom, opts, *asked)
+                elif resident and Plan.workspace_bytes(geom, opts(seg, batch), int(self.ns)) > self._memory():
+                    raise MemoryError
+                break
+            except MemoryError:
+                if not resident:
+                    raise
+                resident = False  # the step kernels need less
         if tile == "auto":
             from .autotune import tune
             fwd, adj, _ = tune(geom, srcx, srcz, self.energy_balancing, batch or int(self.ns), self.device)
@@ -414,6 +428,18 @@ class WavePreparation:
     # times that)
     RES_CELLS, RES_STEP, RES_ADJ = 6.0e5, 3.0e5, 1.6
 
+    def _memory(self):
+        """Bytes a workspace may take: of the free device memory (or the
+        survey's budget), what the traces and the calls leave."""
+        free, _ = torch.cuda.mem_get_info(self.device)
+        # blocks torch's caching allocator holds but does not use count as
+        # free: it releases them when an allocation would otherwise fail
+        free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        if self.memory_budget is not None:
+            free = min(free, int(self.memory_budget / 0.9))
+        traces = 5 * self.nt_ext * int(self.ns) * int(self.nr) * 4
+        return int(0.9 * free) - 4 * traces - (256 << 20)
+
     def _auto_layout(self, geom, opts, seg, batch):
         """Shot batch and recompute segment of the exact checkpoint mode.
 
@@ -424,14 +450,7 @@ class WavePreparation:
         its cells x shots plus a fixed cost per step.  Storing every step of a
         few shots beats recomputing a large batch only where the grid is large
         enough to fill the GPU with a few shots."""
-        free, _ = torch.cuda.mem_get_info(self.device)
-        # blocks torch's caching allocator holds but does not use count as
-        # free: it releases them when an allocation would otherwise fail
-        free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
-        if self.memory_budget is not None:
-            free = min(free, int(self.memory_budget / 0.9))
-        traces = 5 * self.nt_ext * int(self.ns) * int(self.nr) * 4
-        budget = int(0.9 * free) - 4 * traces - (256 << 20)
+        budget = self._memory()
         nt, ns = int(self.nt), int(self.ns)
         cells = float(int(self.tnz) * int(self.tnx))
         memo = {}
@@ -477,7 +496,7 @@ class WavePreparation:
             if best is None or cost < best[0]:
                 best = (cost, s, b)
         if best is None:
-            raise MemoryError("the survey does not fit in device memory (%.1f GB free)" % (free / 2 ** 30))
+            raise MemoryError("the survey does not fit in device memory (%.1f GB for its workspace)" % (budget / 2 ** 30))
         return best[1], best[2]
 
     # ---- helpers ---------------------------------------------------------

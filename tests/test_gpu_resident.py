@@ -66,6 +66,26 @@ def test_resident_loops_give_the_step_kernels_bits(what, extra):
     assert Wr.plan.launches() * 4 < Ws.plan.launches()
 
 
+def _reverse(percent, *size):
+    return dict(_survey(*size), chpr=percent)
+
+
+@pytest.mark.parametrize("what,extra", [("tiny_s8", {}), ("tiny_s8", {"segment": 11}), ("c1", {"energy_balancing": True}),
+                                        ("tiny_chpr", {}), ("tiny_crosswell", {}), ((10, 190, 291, 5, 200), {}),
+                                        ((5, 100, 121, 3, 150), {"shot_batch": 2}), ((60, 61, 70, 2, 90), {}),
+                                        ((20, 75, 90, 2, 120, 8), {})], ids=lambda v: str(v))
+def test_sets_formed_from_states(what, extra):
+    """Energy terms (states stored) and reconstructed states: the difference
+    sets are formed a chunk of steps at a time.  The step kernels' bits."""
+    case = cases.by_name(what) if isinstance(what, str) else _reverse(*what)
+    Wr, r = _run(case, **extra)
+    Ws, s = _run(case, persist=False, **extra)
+    assert Wr.plan.resident and not Ws.plan.resident
+    for k in s:
+        assert bool((r[k] == s[k]).all()), k
+    assert Wr.plan.frame_check() == 0
+
+
 def test_steps_kernels_where_they_are_asked_for():
     case = cases.by_name("tiny_dxr")
     for asked in ({"tile": 1}, {"adj_tile": 1}, {"graph": True}, {"persist": False}, {"store": "states"}, {"overlap": True, "segment": 20}):
