@@ -143,8 +143,8 @@ typedef struct pyfwi_options {
                                and few shots with the wavefield kept on chip, where checkpoint
                                segments hold difference sets in FP32 (store_diffs), or the sets
                                can be formed from FP32 states (energy terms, reverse checkpoints;
-                               a chunk of sets more in the workspace), for the reference adjoint,
-                               no overlap is on, every source lies in the update domain and the
+                               a chunk of sets more in the workspace), or for the exact adjoint
+                               with FP32 states; no overlap is on, every source lies in the update domain and the
                                grid fits on the SMs (up to about 600,000 cells); the step kernels
                                otherwise */
     int32_t overlap;        /* 1: exact checkpoints in FP32 with recompute segments: recompute

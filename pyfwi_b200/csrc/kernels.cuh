@@ -1822,10 +1822,10 @@ __global__ void __launch_bounds__(256) qstress_kernel(Grid g, Coef k, const floa
 // the nsteps given (in backward order, the sets in the same order) has its state
 // at S[s].  The imaging domain only.  Without ENERGY a block takes one step
 // (blockIdx.z = slot * nsteps + step).  With it the energy terms are added to
-// accumulators 3 to 5, which depend on the forward states alone: four threads
-// work out the terms of four steps of a cell and one adds them up in adj_step's
+// accumulators 3 to 5, which depend on the forward states alone: eight threads
+// work out the terms of eight steps of a cell and one adds them up in adj_step's
 // order (one thread per cell: too few in flight, 141 us a launch of 64 steps of 4 shots of 100 x 150
-// cells, eighth order, against 80).  It reads 20 bytes of state per cell and step and writes 20.
+// cells, eighth order, against 100).  It reads 20 bytes of state per cell and step and writes 20.
 constexpr int SETS_STEPS = 64;  // steps of a launch, at most
 struct SetsArgs {
     Grid g;
@@ -1844,7 +1844,7 @@ __global__ void __launch_bounds__(256) sets_kernel(const __grid_constant__ SetsA
 {
     const Grid &g = a.g;
     const int glo = a.npml + R;
-    constexpr int TG = ENERGY ? 4 : 1, ROWS = 8 / TG;  // threads per cell, rows per block
+    constexpr int TG = ENERGY ? 8 : 1, ROWS = 8 / TG;  // threads per cell, rows per block
     __shared__ EnergyTerms part[TG][ROWS * 32];
     const int cell = threadIdx.x % (ROWS * 32), tg = threadIdx.x / (ROWS * 32);
     const int j = glo + blockIdx.x * 32 + cell % 32, i = glo + blockIdx.y * ROWS + cell / 32;

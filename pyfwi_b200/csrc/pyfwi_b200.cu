@@ -119,6 +119,7 @@ struct pyfwi_plan {
     size_t o_hdr, o_src, o_red, o_mat, o_dampx, o_dampz, o_work, o_adj, o_gacc, o_store, o_store16, o_store8, o_xch, o_sets, o_states, total;
     long long launches = 0;
     bool model_set = false, fwd_valid = false;
+    bool sets_kept = false;  // exact adjoint: the last forward pass ran on chip and kept sets where others keep states
     // per-kernel event timing (pyfwi_profile_enable)
     bool profiling = false;
     struct Ev {
@@ -843,8 +844,8 @@ bool use_resident(pyfwi_plan *p, cudaStream_t st)
         p->sms = coop ? std::min(sms, RES_MAX_CTAS) : 1;
     }
     ResTiles tl;
-    return resident_tiles(p->g, p->R, p->lines, p->G, p->sms, false, &tl) &&
-           resident_tiles(p->g, p->R, p->lines, p->G, p->sms, true, &tl);
+    return resident_tiles(p->g, p->R, p->lines, p->G, p->sms, RES_FORWARD, &tl) &&
+           resident_tiles(p->g, p->R, p->lines, p->G, p->sms, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
 }
 
 // A call's first use of the exchange buffer: no word holds a tag of this call.
@@ -878,7 +879,12 @@ int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl
     fa.record = traces != nullptr;
     fa.q_t0 = q_t0;
     if (sets) {
-        fa.store = p->qd ? 1 : 2;
+        fa.store = p->exact_adj ? 3 : p->qd ? 1 : 2;
+        if (p->exact_adj) {  // whose gradient takes the whole update domain
+            fa.a.qlo = p->R;
+            fa.a.qhi_z = p->g.tnz - p->R;
+            fa.a.qhi_x = p->g.tnx - p->R;
+        }
         fa.q = slot_of(*sets, c0).base;
         fa.a.q_stride = sets->stride;
     }
@@ -922,7 +928,7 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, const 
     AdjArgs a = base;
     a.in = adj + (long long)ping * p->state;
     a.in_stride = a.out_stride = 2 * p->state;
-    if (t_hi == G.nt) {  // later steps' residuals are added by the step before
+    if (t_hi == G.nt && !p->exact_adj) {  // later steps' residuals are added by the step before
         a.inj_row = inj_row_of(p, G.nt - 1);
         int rc = launch_inject(p, a, n, st);
         if (rc) return rc;
@@ -939,7 +945,7 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, const 
     r.err = at<int>(ws, ERR_OFF);
     r.limit_ns = BARRIER_WAIT_NS;
     ResTiles tl;
-    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, true, &tl))
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl))
         return fail(PYFWI_E_INVALID, "the adjoint does not fit on chip");
     const int conc = tl.nslots;
     for (int c0 = 0; c0 < n; c0 += conc) {
@@ -956,7 +962,7 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, const 
         r.tag0 = p->tag;
         p->tag += (unsigned)(t_hi - t_lo) + 1;
         ProfileScope prof(p, st, 1, tl.nslots * (t_hi - t_lo));
-        cudaError_t e = launch_adj_resident(r, p->R, st);
+        cudaError_t e = p->exact_adj ? launch_exact_resident(r, p->R, st) : launch_adj_resident(r, p->R, st);
         if (e != cudaSuccess) return fail(PYFWI_E_CUDA, "resident adjoint launch: %s", cudaGetErrorString(e));
         p->launches++;
     }
@@ -994,7 +1000,7 @@ int resident_chunks(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, State s
         a.q = sets.base + (long long)(a.nsteps - 1) * p->state;  // set of step lo first
         const int iz = p->g.tnz - 2 * (p->R + a.npml) + 1, ix = p->g.tnx - 2 * (p->R + a.npml) + 1;
         if (iz > 0 && ix > 0) {
-            const int rows = energy ? 2 : 8;  // of a block
+            const int rows = energy ? 1 : 8;  // of a block
             dim3 grid((ix + 31) / 32, (iz + rows - 1) / rows, energy ? n : n * a.nsteps);
             if (p->R == 4)
                 energy ? sets_kernel<4, true><<<grid, 256, 0, st>>>(a) : sets_kernel<4, false><<<grid, 256, 0, st>>>(a);
@@ -1016,7 +1022,7 @@ int resident_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStr
 {
     const int nt = p->geom.nt;
     ResTiles tl;
-    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, false, &tl))
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, RES_FORWARD, &tl))
         return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
     int rc = clear_exchange(p, ws, st);
     if (rc) return rc;
@@ -1041,7 +1047,7 @@ int resident_recompute(pyfwi_plan *p, void *ws, int s0, int n, int m, cudaStream
 {
     const int t0 = m * p->seg, t1 = std::min(t0 + p->seg, p->geom.nt);
     ResTiles tl;
-    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, false, &tl))
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, RES_FORWARD, &tl))
         return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
     const int conc = tl.nslots;
     const Buf sets = seg_state(p, ws, m, 0);
@@ -1060,7 +1066,8 @@ int exact_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream
     Buf z = exact_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(z.base + q * z.stride, 0, p->state * sizeof(float), st));
     if (use_persist(p, st)) return persist_pass(p, ws, s0, n, traces, st);
-    if (use_resident(p, st)) return resident_pass(p, ws, s0, n, traces, st);
+    p->sets_kept = use_resident(p, st);
+    if (p->sets_kept) return resident_pass(p, ws, s0, n, traces, st);
     StepArgs a = base_step(p, ws);
     a.shot0 = s0;
     a.traces = traces;
@@ -1099,7 +1106,7 @@ Buf chp_state(pyfwi_plan *p, void *ws, int s0, int k)
 int resident_reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
 {
     ResTiles tl;
-    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, false, &tl))
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, RES_FORWARD, &tl))
         return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
     int rc = clear_exchange(p, ws, st);
     if (rc) return rc;
@@ -1461,13 +1468,23 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
             if (rc) return rc;
             rc = misfit_group(p, *mf, s0, n, st);
             if (rc) return rc;
-        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && (p->ngroups > 1 || !p->fwd_valid)) {
+        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT &&
+                   (p->ngroups > 1 || !p->fwd_valid || (p->exact_adj && p->sets_kept != use_resident(p, st)))) {
             rc = exact_pass(p, ws, s0, n, nullptr, st);  // the states of this group are gone
             if (rc) return rc;
         }
         for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(adj + 2 * q * p->state, 0, p->state * sizeof(float), st));
         int ping = 0, t_src = G.nt_ext;
-        if (p->exact_adj) {
+        if (p->exact_adj && use_resident(p, st)) {
+            rc = clear_exchange(p, ws, st);
+            if (rc) return rc;
+            for (int m = p->M - 1; m >= 0; --m) {
+                const int t_lo = m * p->seg, t_hi = std::min((m + 1) * p->seg, G.nt);
+                rc = m < p->M - 1 ? resident_recompute(p, ws, s0, n, m, st) : PYFWI_OK;
+                if (!rc) rc = resident_adjoint(p, ws, a, n, seg_state(p, ws, m, 0), t_lo, t_hi, t_lo, ping, adj, st);
+                if (rc) return rc;
+            }
+        } else if (p->exact_adj) {
             const float *zero[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
             rc = exact_backward(p, ws, residual ? residual : zero, s0, n, st);
             if (rc) return rc;
@@ -1840,14 +1857,15 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
         src_in = src_in && srcz[s] >= p->R && srcz[s] <= tnz - p->R && srcx[s] >= p->R && srcx[s] <= tnx - p->R;
     // (FP32, the reference adjoint, the plain tile kernels), or states that the
     // sets can be formed from: energy terms, reconstructed states
-    const bool from_states = !p->qd && (p->nacc == 6 || opt->checkpoint != PYFWI_CKPT_EXACT) &&
-                             opt->snapshot == PYFWI_SNAP_FP32 && !p->exact_adj && !p->persist && !p->st_w && !p->ftma &&
+    // (or the exact adjoint, whose resident form keeps sets where its step kernels keep states)
+    const bool from_states = !p->qd && (p->nacc == 6 || opt->checkpoint != PYFWI_CKPT_EXACT || p->exact_adj) &&
+                             opt->snapshot == PYFWI_SNAP_FP32 && !p->persist && !p->st_w && !p->ftma &&
                              !p->ast_w && p->ans == 1 && !p->apf && G.npml + p->R >= 4;
     p->resident = opt->persist == 2 && (p->qd == 1 || from_states) && !p->overlap && src_in &&
-                  resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, false, &tl) &&
-                  resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, true, &tl);
+                  resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, RES_FORWARD, &tl) &&
+                  resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
     if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
-    if (p->resident && !p->qd) {
+    if (p->resident && !p->qd && !p->exact_adj) {
         // long enough that the launches' own cost is a small part, in at most 256 MB or half of the states kept
         const size_t kept = opt->checkpoint == PYFWI_CKPT_EXACT ? (size_t)p->seg : p->chp.size() * G.ns / p->G;
         const size_t room = (256ull << 20) / ((size_t)p->state * sizeof(float) * p->G);

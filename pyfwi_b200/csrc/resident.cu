@@ -8,21 +8,24 @@ namespace pyfwi {
 
 template cudaError_t launch_fwd_resident_r<2>(FwdResArgs &a, cudaStream_t s);
 template cudaError_t launch_adj_resident_r<2>(AdjResArgs &a, cudaStream_t s);
+template cudaError_t launch_exact_resident_r<2>(AdjResArgs &a, cudaStream_t s);
 extern template cudaError_t launch_fwd_resident_r<4>(FwdResArgs &a, cudaStream_t s);
 extern template cudaError_t launch_adj_resident_r<4>(AdjResArgs &a, cudaStream_t s);
+extern template cudaError_t launch_exact_resident_r<4>(AdjResArgs &a, cudaStream_t s);
 
 namespace {
 
 constexpr size_t MAX_FLOATS = (232448 - 1024) / sizeof(float);  // 227 KB per CTA less the static words
 
 template <int R>
-bool fits(int th, int nq, int rb, int ctas, const Lines &lines, bool adjoint)
+bool fits(int th, int nq, int rb, int ctas, const Lines &lines, ResLoop loop)
 {
     using S = ResShape<R>;
     const int halo = (th + 4 * R) * (nq + 2 * S::HG) - th * nq, slots = res_slots(R, lines, th, nq);
     return th <= S::TH && nq <= S::NQ && (th / rb) * nq <= RES_THREADS && halo <= RES_HALO &&
            ctas * frame_count(th, nq, 2 * R, S::HG) <= RES_MAX_STRIPS && slots <= RES_MAX_SLOTS &&
-           (!adjoint || adj_res_floats<R>(rb) + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
+           (loop == RES_FORWARD ||
+            (loop == RES_EXACT ? exact_res_floats<R>(rb) : adj_res_floats<R>(rb)) + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
 }
 
 static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_FLOATS, "the forward loop fits on an SM");
@@ -38,18 +41,18 @@ static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_
 // shots of 240 x 440 take 12.6 / 16.0 us with 1 row and two shots at a time,
 // 13.6 / 17.1 with 2 rows and two, 10.8 / 17.0 with 3 rows and four; 8 of 140 x
 // 140 in one launch 3.15 / 3.36 with 1 row, 4.31 / 7.47 with 3.
-bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms, bool adjoint, ResTiles *out)
+bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms, ResLoop loop, ResTiles *out)
 {
     struct Cost {
         double step, row, warp_row, ring, row3;  // fixed; per row; per warp of blocks and row; per warp of ring items; with 3 rows
     };
     constexpr Cost COST[2][2] = {{{1.463, 0.368, 0.013, 0.3, 0.737}, {1.335, 0.545, 0.060, 0.3, 2.460}},
                                  {{1.806, 0.258, 0.090, 0.3, 1.090}, {1.280, 0.721, 0.196, 0.3, 3.239}}};
-    const Cost &k = COST[R > 2][adjoint];
+    const Cost &k = COST[R > 2][loop != RES_FORWARD];
     const int ncg = (g.tnx + 3) / 4, hg = R <= 2 ? 1 : 2;
     double best = 0;
     if (g.tnz < 4 * R || g.tnx < 4 * R) return false;
-    for (int rb = 1; rb <= 3; ++rb) {
+    for (int rb = 1; rb <= (loop == RES_EXACT ? RES_EXACT_ROWS : 3); ++rb) {
         const int nbz = (g.tnz + rb - 1) / rb;
         for (int c = 1; c <= std::min(shots, sms); ++c) {
             const int most = sms / c, waves = (shots + c - 1) / c;
@@ -57,7 +60,7 @@ bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms
             for (int gz = 1; gz <= most && (gz == 1 || nbz / gz * rb >= 2 * R); ++gz) {
                 const int gx = std::min(most / gz, std::max(1, ncg / hg));
                 const int bz = (nbz + gz - 1) / gz, nq = (ncg + gx - 1) / gx, th = rb * bz;
-                if (!(R == 2 ? fits<2>(th, nq, rb, c * gz * gx, lines, adjoint) : fits<4>(th, nq, rb, c * gz * gx, lines, adjoint)))
+                if (!(R == 2 ? fits<2>(th, nq, rb, c * gz * gx, lines, loop) : fits<4>(th, nq, rb, c * gz * gx, lines, loop)))
                     continue;
                 const double ring = (double)(th + 2 * R) * (nq + 2) - (double)th * nq;
                 const double cost = waves * (k.step + rb * (k.row + k.warp_row * bz * nq / 32.0) + k.ring * ring / 32.0 +
@@ -75,6 +78,11 @@ bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms
 cudaError_t launch_fwd_resident(FwdResArgs &a, int R, cudaStream_t s)
 {
     return R == 2 ? launch_fwd_resident_r<2>(a, s) : launch_fwd_resident_r<4>(a, s);
+}
+
+cudaError_t launch_exact_resident(AdjResArgs &a, int R, cudaStream_t s)
+{
+    return R == 2 ? launch_exact_resident_r<2>(a, s) : launch_exact_resident_r<4>(a, s);
 }
 
 cudaError_t launch_adj_resident(AdjResArgs &a, int R, cudaStream_t s)

@@ -138,7 +138,7 @@ struct FwdResArgs {
     int t0, t1;
     int dt_scale, nt_ext, record;
     float *q;          // difference sets (store 1) or states (2) of slot 0 (a.q_stride apart): S_{t+1}'s at
-                       // q + (t - q_t0) * state
+                       // q + (t - q_t0) * state; 3: the exact adjoint's sets of step t
     int q_t0, store;
     int *err;
     unsigned long long limit_ns;
@@ -176,6 +176,9 @@ constexpr int RES_OWN = RB < 3 ? 4 * RB * RES_THREADS : ResShape<R>::OPLANE;  //
 template <int R, int RB>
 constexpr int ADJ_RES_FLOATS = RES_PAD + 5 * RES_PLANE + (RB < 2 ? 2 : 3) * RES_OWN<R, RB> + 22 * ResShape<R>::RING + 2 * RES_ROWS +
                                3 * RES_W + 3 * RES_THREADS + 4 * RES_SETS<RB> * RES_THREADS;
+template <int R, int RB>
+constexpr int EXA_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 2 * RES_OWN<R, RB> + 14 * ResShape<R>::RING + RES_ROWS + RES_W +
+                               4 * RES_THREADS;
 constexpr int RES_SLOT_FLOATS = 44;  // and per slot of staged residuals (adjoint)
 
 // 16-byte words that are written and read as one transaction.
@@ -444,7 +447,9 @@ __device__ __forceinline__ void res_block(const ResTile &t, int e, int &bz, int 
 // ---------------------------------------------------------------------------
 // forward steps t0 .. t1 - 1 (fwd_step's arithmetic)
 // ---------------------------------------------------------------------------
-// QD: 1 stores the difference sets of the states, 2 the states, 0 neither.
+// QD: 1 stores the difference sets of the states, 2 the states, 3 the exact
+// adjoint's sets (stress differences of S_t with step t's source, velocity
+// differences of S_{t+1}; zero outside the update domain), 0 neither.
 template <int R, int RB, int QD>
 __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_constant__ FwdResArgs p)
 {
@@ -545,6 +550,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
     const int co = (gi0 + ZO) * g.pitch + gj0 + XO;        // its first cell in a plane
     float4 vx[RB], vz[RB], sxx[RB], szz[RB], sxz[RB];
     float4 b[RB], lam[RB], mu[RB];
+    constexpr bool SETS = QD == 1 || QD == 3;
     bool damp = false;
     unsigned img = 0;                                      // rows with imaged cells
 #pragma unroll
@@ -562,7 +568,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         lam[r] = masked(a.mat, gi, gj0);
         mu[r] = masked(a.mat + P, gi, gj0);
         damp = damp || damped(gi, gj0);
-        if (QD == 1 && gi >= a.qlo && gi <= a.qhi_z && gj0 + 3 >= a.qlo && gj0 <= a.qhi_x) img |= 1u << r;
+        if (SETS && gi >= a.qlo && gi <= a.qhi_z && gj0 + 3 >= a.qlo && gj0 <= a.qhi_x) img |= 1u << r;
     }
 
     // The strip group of row r of the tile in this thread's column, -1: none.
@@ -602,6 +608,14 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         tr[4 * a.trace_plane] = s_txz[rec_o];
     };
 
+    // Four values of a set: (QD 3) zero on columns outside the update domain.
+    auto within = [&](float (&s)[4]) {
+        if (QD == 3)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (gj0 + k < a.qlo || gj0 + k > a.qhi_x) s[k] = 0.f;
+        return mk4(s);
+    };
     // New velocities of the block; qi: the difference set of the input state (null: none).
     auto velocity = [&](float *qi) {
         {
@@ -615,7 +629,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     s[k] = xbwd<R>(x, k, a.k.cx) + z.at(r, k, a.k.cz);
                     n[k] = f4(vx[r], k) + dt * (f4(b[r], k) * s[k]);
                 }
-                if (QD == 1 && qi && (img >> r & 1)) qst4s(qi + Q_TXS * P + co + r * g.pitch, mk4(s));
+                if (SETS && qi && (img >> r & 1)) qst4s(qi + Q_TXS * P + co + r * g.pitch, within(s));
                 vx[r] = mk4(n);
             }
         }
@@ -630,7 +644,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     s[k] = z.at(r, k, a.k.cz) + xfwd<R>(x, k, a.k.cx);
                     n[k] = f4(vz[r], k) + dt * (f4(b[r], k) * s[k]);
                 }
-                if (QD == 1 && qi && (img >> r & 1)) qst4s(qi + Q_TZS * P + co + r * g.pitch, mk4(s));
+                if (SETS && qi && (img >> r & 1)) qst4s(qi + Q_TZS * P + co + r * g.pitch, within(s));
                 vz[r] = mk4(n);
             }
         }
@@ -704,6 +718,10 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     ez[k] = zz.at(r, k, a.k.cz);
                 }
                 hx[r] = mk4(h);
+                if (QD == 3 && (img >> r & 1)) {
+                    qst4s(qo + Q_DXP_VX * P + co + r * g.pitch, within(ex));
+                    qst4s(qo + Q_DZM_VZ * P + co + r * g.pitch, within(ez));
+                }
                 if (QD == 1 && (img >> r & 1)) {
                     float *q = qo + co + r * g.pitch, s[4];
 #pragma unroll
@@ -728,6 +746,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
             float oxz[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) oxz[k] = f4(sxz[r], k) + dt * (f4(mu[r], k) * (f4(hx[r], k) + zx.at(r, k, a.k.cz)));
+            if (QD == 3 && (img >> r & 1)) {
+                float s[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) s[k] = f4(hx[r], k) + zx.at(r, k, a.k.cz);
+                qst4s(qo + Q_VZS * P + co + r * g.pitch, within(s));
+            }
             if (damp) {
                 const float4 dx = ld4s(s_dx + HX + 4 * bq);
                 const float dr = s_dz[br + r + 2 * R];
@@ -772,6 +796,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         if constexpr (QD) {
             qo = p.q + (long long)(t - p.q_t0) * p.state + T.slot * a.q_stride;
             if (QD == 1 && t > p.q_t0) qi = qo - p.state;
+            if (QD == 3) qi = qo;
         }
         if (add) {
             __syncthreads();
@@ -1487,6 +1512,430 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
         *reinterpret_cast<float4 *>(G + co + r * g.pitch) = gmu[r];
         *reinterpret_cast<float4 *>(G + P + co + r * g.pitch) = glam[r];
         *reinterpret_cast<float4 *>(G + 2 * P + co + r * g.pitch) = RB < 2 ? grho : ld4s(s_rho + om + r * OM);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// exact adjoint steps t_hi - 1 .. t_lo (exact_adj_step's formulas)
+// ---------------------------------------------------------------------------
+// The transpose runs as the forward loop does, velocities from differences of
+// three stress planes (P1 .. P3), then stresses from differences of two
+// velocity planes (Q1, Q2), so it exchanges and recomputes what that does: the
+// P planes' outermost 2R rows and columns, the Q planes of the ring.  The
+// residuals are staged as in adj_resident, and added to the new state at the
+// end of a step (to the ring's velocities at the start of the next one).  The
+// materials are zero outside the update domain, which is all that keeps P and Q
+// zero there.  Latency bounds it, as the other loops: for 101 x 203 cells and 4
+// shots a step took 15.6 us in exact_adj_step and 3.5 in the injection after it,
+// and takes 4.0 us here.
+template <int R, int RB>
+__global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_constant__ AdjResArgs p)
+{
+    constexpr int NT = RES_THREADS, HX = ResShape<R>::HX, HG = ResShape<R>::HG;
+    extern __shared__ float4 smem4[];
+    __shared__ int s_stop, s_nslot, s_line[4][6];
+    const AdjArgs &a = p.a;
+    const Grid &g = a.g;
+    const long long P = g.plane;
+    const int tid = threadIdx.x;
+    const ResTile T = res_tile<R, RB>(p.tl);
+    const int i0 = T.i0, j0 = T.j0, th = T.th, nq = T.nq;
+    constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING, OWN = RES_OWN<R, RB>;
+    float *const sm = reinterpret_cast<float *>(smem4) + RES_PAD;
+    // Cell (r, c) of the tile lies at (r + 2R) * W + HX + c of every plane.
+    float *const s_p1 = sm, *const s_p2 = sm + PL, *const s_p3 = sm + 2 * PL, *const s_q1 = sm + 3 * PL, *const s_q2 = sm + 4 * PL;
+    float *const s_lam = sm + 5 * PL, *const s_mu = s_lam + OWN;  // [row][thread][4] of the blocks
+    float *const s_ring = s_mu + OWN;                             // [ring item][3][4]: its velocities, buoyancy
+    float *const s_dx = s_ring + 12 * RING, *const s_dz = s_dx + W;  // damping
+    unsigned *const t_ring = reinterpret_cast<unsigned *>(s_dz + RES_ROWS);
+    int *const t_rslot = reinterpret_cast<int *>(t_ring + RING);
+    unsigned *const t_word = reinterpret_cast<unsigned *>(t_rslot + RING);
+    float *const s_res = reinterpret_cast<float *>(t_word + 4 * RES_THREADS);  // [2][5][slots][4] staged residuals
+    int *const t_dst = reinterpret_cast<int *>(s_res + 40 * p.slots);
+    const int nring = (th + 2 * R) * (nq + 2) - th * nq;
+    const float dt = a.k.dt;
+    const float *in = a.in + T.slot * a.in_stride;
+    const int frame = frame_count(RB * p.tl.bz, p.tl.nq, 2 * R, HG);
+    const int xpar = 4 * gridDim.x * frame;
+    uint4 *const strip = p.xch + 4 * blockIdx.x * frame;
+    const int shot = a.shot0 + T.slot;
+
+    // receivers of the tile and its ring, as in adj_resident
+    if (tid < 32) {
+        int k0 = 0, n = 0;
+        const Lines &L = a.lines;
+        if (tid < L.n) line_range(L, tid, i0 - R, i0 + th + R, j0 - 4, j0 + 4 * nq + 4, k0, n);
+        const int n0 = __shfl_sync(0xffffffffu, n, 0), n1 = __shfl_sync(0xffffffffu, n, 1), n2 = __shfl_sync(0xffffffffu, n, 2);
+        if (tid < L.n) {
+            s_line[tid][0] = n;
+            s_line[tid][1] = k0;
+            s_line[tid][2] = shot * a.nr + L.slot0[tid] + k0;
+            s_line[tid][3] = tid == 0 ? 0 : tid == 1 ? n0 : n0 + n1;
+        }
+        if (tid == 0) {
+            s_line[3][0] = n0 + n1 + n2;
+            s_nslot = 0;
+            s_stop = ld_relaxed_gpu(p.err) != 0;
+        }
+    }
+    for (int e = tid; e < 40 * p.slots; e += NT) s_res[e] = 0.f;
+    for (int e = tid; e < 4 * nq + 2 * HX; e += NT) {
+        const int c = j0 - HX + e + XO;
+        s_dx[e] = c >= 0 && c < g.pitch ? __ldg(a.dampx + c) : 0.f;
+    }
+    for (int e = tid; e < th + 4 * R; e += NT) {
+        const int i = i0 - 2 * R + e + ZO;
+        s_dz[e] = i >= 0 && i < g.rows ? __ldg(a.dampz + i) : 0.f;
+    }
+    __syncthreads();
+    const int nrec = s_line[3][0];
+    auto slots_of = [&](int gi, int gj) {
+        int w = 0;
+        for (int l = 0; nrec && l < a.lines.n; ++l) {
+            int slot = 0;
+            for (int c = 0; c < 4; ++c) {
+                const int ks = line_slot(a.lines, l, gi, gj + c);
+                if (ks < 0) continue;
+                if (!slot) slot = atomicAdd(&s_nslot, 1) + 1;
+                t_dst[s_line[l][3] + ks - s_line[l][1]] = 4 * (slot - 1) + c;
+            }
+            w |= slot << 10 * l;
+        }
+        return w;
+    };
+    auto masked = [&](const float *plane, int gi, int gj) {
+        float4 v = ld4(plane, g, gi, gj);
+        if (!in_domain(g, R, gi, gj)) v.x = 0.f;
+        if (!in_domain(g, R, gi, gj + 1)) v.y = 0.f;
+        if (!in_domain(g, R, gi, gj + 2)) v.z = 0.f;
+        if (!in_domain(g, R, gi, gj + 3)) v.w = 0.f;
+        return v;
+    };
+    // 1 - dt d of four cells: column place c of s_dx, row place r of s_dz
+    auto damp4_of = [&](int r, int c) {
+        const float4 dx = ld4s(s_dx + c);
+        const float dz = s_dz[r];
+        return make_float4(1.f - dt * (dx.x + dz), 1.f - dt * (dx.y + dz), 1.f - dt * (dx.z + dz), 1.f - dt * (dx.w + dz));
+    };
+    // P1 .. P3 of four cells
+    auto products = [&](const float4 &l, const float4 &m, const float4 &d, const float4 &xx, const float4 &zz, const float4 &xz,
+                        float4 &p1, float4 &p2, float4 &p3) {
+        float v1[4], v2[4], v3[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float axx = f4(d, k) * f4(xx, k), azz = f4(d, k) * f4(zz, k), axz = f4(d, k) * f4(xz, k);
+            const float lam = f4(l, k), l2m = lam + 2.f * f4(m, k);
+            v1[k] = dt * (l2m * axx + lam * azz);
+            v2[k] = dt * (f4(m, k) * axz);
+            v3[k] = dt * (lam * axx + l2m * azz);
+        }
+        p1 = mk4(v1);
+        p2 = mk4(v2);
+        p3 = mk4(v3);
+    };
+    for (int e = tid; e < (th + 4 * R) * (nq + 2 * HG); e += NT) {
+        const int r = e / (nq + 2 * HG), q = e - r * (nq + 2 * HG), o = r * W + 4 * q;
+        const int gi = i0 - 2 * R + r, gj = j0 - HX + 4 * q;
+        float4 p1, p2, p3;
+        products(masked(a.mat, gi, gj), masked(a.mat + P, gi, gj), damp4_of(r, 4 * q), ld4(in + TXX * P, g, gi, gj),
+                 ld4(in + TZZ * P, g, gi, gj), ld4(in + TXZ * P, g, gi, gj), p1, p2, p3);
+        st4s(s_p1 + o, p1);
+        st4s(s_p2 + o, p2);
+        st4s(s_p3 + o, p3);
+    }
+    for (int e = tid; e < nring; e += NT) {
+        int r, q;
+        frame_item(e, th + 2 * R, nq + 2, R, 1, r, q);
+        t_ring[e] = pack_item(r, q);
+        const int gi = i0 - R + r, gj = j0 - 4 + 4 * q;
+        t_rslot[e] = slots_of(gi, gj);
+        float *s = s_ring + 12 * e;
+        st4s(s, ld4(in + VX * P, g, gi, gj));
+        st4s(s + 4, ld4(in + VZ * P, g, gi, gj));
+        st4s(s + 8, masked(a.mat + 2 * P, gi, gj));
+    }
+
+    // this thread's block
+    const bool mine = tid < T.nblk, inside = tid < T.nin;
+    int bz = 0, bq = 0;
+    if (mine) res_block<R, RB>(T, tid, bz, bq);
+    const int br = bz * RB;
+    const int ot = (br + 2 * R) * W + HX + 4 * bq;
+    const int gi0 = i0 + br, gj0 = j0 + 4 * bq;
+    const int co = (gi0 + ZO) * g.pitch + gj0 + XO;
+    float4 vx[RB], vz[RB], xx[RB], zz[RB], xz[RB], b[RB];
+    float4 glam[RB], gmu[RB], gb[RB];  // its gradient accumulators
+    int rs[RB];
+    unsigned img = 0;                  // rows of the update domain
+    float *const G = a.gacc + T.slot * a.gacc_stride;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        vx[r] = vz[r] = xx[r] = zz[r] = xz[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        glam[r] = gmu[r] = gb[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        rs[r] = 0;
+        if (!mine) continue;
+        const int gi = gi0 + r;
+        vx[r] = ld4(in + VX * P, g, gi, gj0);
+        vz[r] = ld4(in + VZ * P, g, gi, gj0);
+        xx[r] = ld4(in + TXX * P, g, gi, gj0);
+        zz[r] = ld4(in + TZZ * P, g, gi, gj0);
+        xz[r] = ld4(in + TXZ * P, g, gi, gj0);
+        b[r] = masked(a.mat + 2 * P, gi, gj0);
+        st4s(s_lam + 4 * (r * NT + tid), masked(a.mat, gi, gj0));
+        st4s(s_mu + 4 * (r * NT + tid), masked(a.mat + P, gi, gj0));
+        if (gi < g.tnz) {
+            glam[r] = *reinterpret_cast<const float4 *>(G + co + r * g.pitch);
+            gmu[r] = *reinterpret_cast<const float4 *>(G + P + co + r * g.pitch);
+            gb[r] = *reinterpret_cast<const float4 *>(G + 2 * P + co + r * g.pitch);
+        }
+        rs[r] = slots_of(gi, gj0);
+        if (gi >= R && gi <= g.tnz - R && gj0 + 3 >= R && gj0 <= g.tnx - R) img |= 1u << r;
+    }
+    __syncthreads();
+
+    int rec_d = -1, rec_c = 0;
+    for (int l = 0, e = tid; l < a.lines.n; e -= s_line[l++][0])
+        if (e >= 0 && e < s_line[l][0]) {
+            rec_d = t_dst[s_line[l][3] + e];
+            rec_c = s_line[l][2] + e;
+        }
+    auto stage = [&](int row, int t) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(s_res + (t & 1) * 20 * p.slots + rec_d);
+        const long long o = (long long)row * a.ns * a.nr + rec_c;
+#pragma unroll
+        for (int f = 0; f < 5; ++f)
+            if (a.res[f])
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + f * 16 * p.slots), "l"(a.res[f] + o) : "memory");
+    };
+    // Adds the staged residuals of step t to field f of a group: line after line, and the residual of a line's vz
+    // trace to the field it was recorded from.
+    auto add4 = [&](float4 &v, int t, int f, int slot) {
+        if (!a.res[f]) return;
+        const float4 x = ld4s(s_res + (((t & 1) * 5 + f) * p.slots + slot) * 4);
+        v.x += x.x;
+        v.y += x.y;
+        v.z += x.z;
+        v.w += x.w;
+    };
+    auto inject = [&](float4 &v, int t, int f, int w) {
+        for (int l = 0; w; w = (int)((unsigned)w >> 10), ++l) {
+            const int s = w & 1023;
+            if (!s) continue;
+            if (f != VZ || !a.lines.vzx[l]) add4(v, t, f, s - 1);
+            if (f == VX && a.lines.vzx[l]) add4(v, t, VZ, s - 1);
+        }
+    };
+    const int t_first = p.t_hi - 1;
+    halo_words<R, 4>(t_word, g, p.tl, frame, T.slot, T.tz, T.tx, i0, th, T.q0, nq);
+    auto put = [&](int o, int c, const uint4 &w) {
+        s_p1[o + c] = __uint_as_float(w.x);
+        s_p2[o + c] = __uint_as_float(w.y);
+        s_p3[o + c] = __uint_as_float(w.z);
+    };
+    const float *const q0 = p.q + T.slot * a.fwd_stride + co;
+    auto set_of = [&](int t, int f, int r) { return q0 + (long long)(t - p.q_t0) * p.state + f * P + r * g.pitch; };
+
+    // New velocities of the block, and Q1, Q2.
+    auto velocity = [&](int t) {
+        float4 qx[RB], qz[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            qx[r] = qz[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!(img >> r & 1)) continue;
+            qx[r] = qld4s(set_of(t, Q_TXS, r));
+            qz[r] = qld4s(set_of(t, Q_TZS, r));
+        }
+        {
+            auto row = [&](int r) { return ld4s(s_p2 + ot + r * W); };
+            ZSlide<R, false> z(row);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                z.next(row(r + R - 1));
+                float x[12], n[4];
+                xrow<R, false>(x, ld4s(s_p1 + ot + r * W), s_p1 + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) n[k] = f4(vx[r], k) - xbwd<R>(x, k, a.k.cx) - z.at(k, a.k.cz);
+                vx[r] = mk4(n);
+            }
+        }
+        auto row = [&](int r) { return ld4s(s_p3 + ot + r * W); };
+        ZSlide<R, true> z(row);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            z.next(row(r + R));
+            float x[12], n[4], m[4], w[4], u[4], gg[4];
+            const float4 d = damp4_of(br + r + 2 * R, HX + 4 * bq);
+            xrow<R, true>(x, ld4s(s_p2 + ot + r * W), s_p2 + ot + r * W);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                n[k] = f4(d, k) * (f4(vz[r], k) - z.at(k, a.k.cz) - xfwd<R>(x, k, a.k.cx));
+                m[k] = f4(d, k) * f4(vx[r], k);
+                u[k] = dt * (f4(b[r], k) * m[k]);
+                w[k] = dt * (f4(b[r], k) * n[k]);
+                gg[k] = f4(gb[r], k) + dt * (m[k] * f4(qx[r], k) + n[k] * f4(qz[r], k));
+            }
+            vx[r] = mk4(m);
+            vz[r] = mk4(n);
+            gb[r] = mk4(gg);
+            st4s(s_q1 + ot + r * W, mk4(u));
+            st4s(s_q2 + ot + r * W, mk4(w));
+        }
+    };
+    // The same for ring item e, first, where it is due, what the residual of step t + 1 added to its velocities.
+    auto ring = [&](int e, int t, bool due) {
+        const int r = item_row(t_ring[e]), q = item_col(t_ring[e]), c = (r + R) * W + HX - 4 + 4 * q;
+        float *s = s_ring + 12 * e;
+        float4 ovx = ld4s(s), ovz = ld4s(s + 4);
+        const float4 bb = ld4s(s + 8), d = damp4_of(r + R, HX - 4 + 4 * q);
+        const int w = t_rslot[e];
+        if (due && w) {
+            inject(ovx, t + 1, VX, w);
+            inject(ovz, t + 1, VZ, w);
+        }
+        float x[12], nx[4], nz[4], u[4], v[4];
+        const ZWindow<R, 1, false> z2([&](int) { return ld4s(s_p2 + c); }, s_p2 + c);
+        xrow<R, false>(x, ld4s(s_p1 + c), s_p1 + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) nx[k] = f4(d, k) * (f4(ovx, k) - xbwd<R>(x, k, a.k.cx) - z2.at(0, k, a.k.cz));
+        const ZWindow<R, 1, true> z3([&](int) { return ld4s(s_p3 + c); }, s_p3 + c);
+        xrow<R, true>(x, ld4s(s_p2 + c), s_p2 + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            nz[k] = f4(d, k) * (f4(ovz, k) - z3.at(0, k, a.k.cz) - xfwd<R>(x, k, a.k.cx));
+            u[k] = dt * (f4(bb, k) * nx[k]);
+            v[k] = dt * (f4(bb, k) * nz[k]);
+        }
+        st4s(s, mk4(nx));
+        st4s(s + 4, mk4(nz));
+        st4s(s_q1 + c, mk4(u));
+        st4s(s_q2 + c, mk4(v));
+    };
+    auto strip_group = [&](int r) {
+        return r < 2 * R || r >= th - 2 * R || bq < HG || bq >= nq - HG ? frame_index(r, bq, th, nq, 2 * R, HG) : -1;
+    };
+    // New stresses of the block with the residual of step t, their products, and the strips to xo.
+    auto stress = [&](int t, bool epi, uint4 *xo, unsigned tag) {
+        float4 q0v[RB], q1v[RB], q2v[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            q0v[r] = q1v[r] = q2v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!(img >> r & 1)) continue;
+            q0v[r] = qld4s(set_of(t, Q_DXP_VX, r));
+            q1v[r] = qld4s(set_of(t, Q_DZM_VZ, r));
+            q2v[r] = qld4s(set_of(t, Q_VZS, r));
+        }
+        {
+            auto row = [&](int r) { return ld4s(s_q2 + ot + r * W); };
+            ZSlide<R, false> z(row);  // Dz- Q2
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                z.next(row(r + R - 1));
+                const float4 d = damp4_of(br + r + 2 * R, HX + 4 * bq);
+                float x[12], oz[4], oxz[4], gl[4], gm[4], ax[4];
+                xrow<R, false>(x, z.centre(), s_q2 + ot + r * W);  // Dx- Q2
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    ax[k] = f4(d, k) * f4(xx[r], k);
+                    const float az = f4(d, k) * f4(zz[r], k), axz = f4(d, k) * f4(xz[r], k);
+                    gl[k] = f4(glam[r], k) + dt * (ax[k] + az) * (f4(q0v[r], k) + f4(q1v[r], k));
+                    gm[k] = f4(gmu[r], k) + dt * (2.f * ax[k] * f4(q0v[r], k) + 2.f * az * f4(q1v[r], k) + axz * f4(q2v[r], k));
+                    oz[k] = az - z.at(k, a.k.cz);
+                    oxz[k] = xbwd<R>(x, k, a.k.cx);  // taken off after Dz+ Q1
+                }
+                xx[r] = mk4(ax);
+                zz[r] = mk4(oz);
+                glam[r] = mk4(gl);
+                gmu[r] = mk4(gm);
+                xz[r] = make_float4(d.x * xz[r].x, d.y * xz[r].y, d.z * xz[r].z, d.w * xz[r].w);
+                q2v[r] = mk4(oxz);
+            }
+        }
+        auto row = [&](int r) { return ld4s(s_q1 + ot + r * W); };
+        ZSlide<R, true> z(row);  // Dz+ Q1
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            z.next(row(r + R));
+            float x[12], ox[4], oxz[4];
+            xrow<R, true>(x, z.centre(), s_q1 + ot + r * W);  // Dx+ Q1
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                ox[k] = f4(xx[r], k) - xfwd<R>(x, k, a.k.cx);
+                oxz[k] = f4(xz[r], k) - z.at(k, a.k.cz) - f4(q2v[r], k);
+            }
+            xx[r] = mk4(ox);
+            xz[r] = mk4(oxz);
+            if (epi && rs[r]) {
+                inject(vx[r], t, VX, rs[r]);
+                inject(vz[r], t, VZ, rs[r]);
+                inject(xx[r], t, TXX, rs[r]);
+                inject(zz[r], t, TZZ, rs[r]);
+                inject(xz[r], t, TXZ, rs[r]);
+            }
+            float4 p1, p2, p3;
+            products(ld4s(s_lam + 4 * (r * NT + tid)), ld4s(s_mu + 4 * (r * NT + tid)), damp4_of(br + r + 2 * R, HX + 4 * bq),
+                     xx[r], zz[r], xz[r], p1, p2, p3);
+            st4s(s_p1 + ot + r * W, p1);
+            st4s(s_p2 + ot + r * W, p2);
+            st4s(s_p3 + ot + r * W, p3);
+            if (!inside) {
+                const int s = strip_group(br + r);
+                if (s >= 0) {
+                    st_word(xo + 4 * s, p1.x, p2.x, p3.x, tag);
+                    st_word(xo + 4 * s + 1, p1.y, p2.y, p3.y, tag);
+                    st_word(xo + 4 * s + 2, p1.z, p2.z, p3.z, tag);
+                    st_word(xo + 4 * s + 3, p1.w, p2.w, p3.w, tag);
+                }
+            }
+        }
+    };
+
+    const int rank = tid >= T.nblk ? tid - T.nblk : tid + NT - T.nblk;
+    bool stop = s_stop, due = false;
+    for (int t = t_first; t >= p.t_lo && !stop; --t) {
+        const bool epi = nrec && t % p.dt_scale == 0 && t / p.dt_scale < p.nt_ext;
+        if (epi && rec_d >= 0) stage(t / p.dt_scale, t);
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 1 && t < t_first) {
+                if (!fetch_halo<4, false>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
+                    s_stop = 1;
+                __syncthreads();
+                stop = s_stop;
+                if (stop) break;
+            }
+            if (mine && inside == (pass == 0)) velocity(t);
+        }
+        if (stop) break;
+        for (int e = rank; e < nring; e += NT) ring(e, t, due);
+        cp_wait<0>();
+        __syncthreads();
+        if (mine) stress(t, epi, strip + ((t - 1) & 1) * xpar, p.tag0 + (unsigned)(t_first - t + 1));
+        due = epi;
+        __syncthreads();
+    }
+    if (!mine) return;
+    const float nan = __int_as_float(RES_NAN);
+    float *out = a.out + T.slot * a.out_stride;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        if (gi0 + r >= g.tnz) break;
+        if (stop) {
+            vx[r] = vz[r] = xx[r] = zz[r] = xz[r] = make_float4(nan, nan, nan, nan);
+            glam[r] = gmu[r] = gb[r] = vx[r];
+        }
+        // nothing is kept beyond the grid's last column
+        auto kept = [&](const float4 &v) {
+            return make_float4(v.x, gj0 + 1 < g.tnx ? v.y : 0.f, gj0 + 2 < g.tnx ? v.z : 0.f, gj0 + 3 < g.tnx ? v.w : 0.f);
+        };
+        float *o = out + co + r * g.pitch;
+        *reinterpret_cast<float4 *>(o + VX * P) = kept(vx[r]);
+        *reinterpret_cast<float4 *>(o + VZ * P) = kept(vz[r]);
+        *reinterpret_cast<float4 *>(o + TXX * P) = kept(xx[r]);
+        *reinterpret_cast<float4 *>(o + TZZ * P) = kept(zz[r]);
+        *reinterpret_cast<float4 *>(o + TXZ * P) = kept(xz[r]);
+        *reinterpret_cast<float4 *>(G + co + r * g.pitch) = glam[r];
+        *reinterpret_cast<float4 *>(G + P + co + r * g.pitch) = gmu[r];
+        *reinterpret_cast<float4 *>(G + 2 * P + co + r * g.pitch) = gb[r];
     }
 }
 

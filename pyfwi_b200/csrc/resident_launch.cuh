@@ -30,12 +30,32 @@ constexpr size_t adj_res_floats(int rb)
     return rb == 1 ? ADJ_RES_FLOATS<R, 1> : rb == 2 ? ADJ_RES_FLOATS<R, 2> : ADJ_RES_FLOATS<R, 3>;
 }
 
+// And of the exact adjoint, whose blocks have one or two rows (three would
+// spill: 32 floats a cell are live).
+constexpr int RES_EXACT_ROWS = 2;
+template <int R>
+constexpr size_t exact_res_floats(int rb)
+{
+    return rb == 1 ? EXA_RES_FLOATS<R, 1> : EXA_RES_FLOATS<R, 2>;
+}
+
+template <int R>
+cudaError_t launch_exact_resident_r(AdjResArgs &a, cudaStream_t s)
+{
+    a.slots = res_slots(R, a.a.lines, a.tl.rb * a.tl.bz, a.tl.nq);
+    const size_t f = exact_res_floats<R>(a.tl.rb) + RES_SLOT_FLOATS * (size_t)a.slots;
+    const void *kern = a.tl.rb == 1 ? reinterpret_cast<const void *>(exact_resident<R, 1>)
+                                    : reinterpret_cast<const void *>(exact_resident<R, 2>);
+    return launch_resident(kern, a, f, s);
+}
+
 template <int R>
 cudaError_t launch_fwd_resident_r(FwdResArgs &a, cudaStream_t s)
 {
 #define CASE(RB_, Q_) \
     if (a.tl.rb == RB_ && a.store == Q_) return launch_resident(reinterpret_cast<const void *>(fwd_resident<R, RB_, Q_>), a, FWD_RES_FLOATS<R, RB_>, s);
-    CASE(1, 0) CASE(1, 1) CASE(1, 2) CASE(2, 0) CASE(2, 1) CASE(2, 2) CASE(3, 0) CASE(3, 1) CASE(3, 2)
+    CASE(1, 0) CASE(1, 1) CASE(1, 2) CASE(1, 3) CASE(2, 0) CASE(2, 1) CASE(2, 2) CASE(2, 3) CASE(3, 0) CASE(3, 1) CASE(3, 2)
+    CASE(3, 3)
 #undef CASE
     return cudaErrorInvalidValue;
 }

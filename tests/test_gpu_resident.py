@@ -86,6 +86,26 @@ def test_sets_formed_from_states(what, extra):
     assert Wr.plan.frame_check() == 0
 
 
+@pytest.mark.parametrize("what,extra", [("tiny_dxr", {}), ("tiny_dtscale", {}), ("tiny_both", {"segment": 40, "shot_batch": 1}),
+                                        ("c1", {}), ((37, 61, 1, 90), {}), ((101, 203, 4, 100), {"segment": 30}),
+                                        ((150, 301, 2, 70, 8), {}), ((33, 900, 2, 60), {})], ids=lambda v: str(v))
+def test_exact_adjoint_on_chip(what, extra):
+    """The exact adjoint's resident loop against its step kernels: the traces'
+    bits; the gradient sums the same terms with roundings of their own (the
+    source's part of a stress difference is added to the stress, not to the
+    difference), so it agrees to float32 rounding."""
+    case = cases.by_name(what) if isinstance(what, str) else _survey(*what)
+    Wr, r = _run(case, adjoint="exact", **extra)
+    Ws, s = _run(case, adjoint="exact", persist=False, **extra)
+    assert Wr.plan.resident and not Ws.plan.resident
+    for k in s:
+        if k.startswith("d_") or k == "rms":
+            assert bool((r[k] == s[k]).all()), k
+        else:
+            assert float((r[k] - s[k]).norm()) <= 1e-6 * float(s[k].norm()), k
+    assert Wr.plan.frame_check() == 0
+
+
 def test_steps_kernels_where_they_are_asked_for():
     case = cases.by_name("tiny_dxr")
     for asked in ({"tile": 1}, {"adj_tile": 1}, {"graph": True}, {"persist": False}, {"store": "states"}, {"overlap": True, "segment": 20}):
