@@ -162,9 +162,13 @@ struct AdjResArgs {
 };
 
 // Shared memory in floats.
+// Forward: materials of the blocks that lie in shared memory: with three rows
+// in registers the fields alone fill them.
+template <int RB>
+constexpr int FWD_SHARED_MATS = RB < 3 ? 0 : 3;
 template <int R, int RB>
 constexpr int FWD_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 6 * ResShape<R>::RING + 2 * RES_ROWS + 2 * RES_W + 8 +
-                               4 * RES_MAX_SAMPLES + 4 * RES_THREADS;
+                               4 * RES_MAX_SAMPLES + 4 * RES_THREADS + 4 * FWD_SHARED_MATS<RB> * RB * RES_THREADS;
 // Adjoint: a thread's places for difference sets on their way, four floats
 // each: three rows share six places, asked for in turns.  Blocks of more than
 // one row keep one of the three gradient accumulators in shared memory: with
@@ -472,6 +476,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
     float4 *const s_wav = reinterpret_cast<float4 *>(s_org + 4);
     unsigned *const t_ring = reinterpret_cast<unsigned *>(s_wav + RES_MAX_SAMPLES);
     unsigned *const t_word = t_ring + RING;                       // the threads' halo words
+    float *const s_mat = reinterpret_cast<float *>(t_word + 4 * NT);  // [lam, mu, b][row][thread][4], RB 3
+    constexpr int SM = FWD_SHARED_MATS<RB>;
     const int frame = frame_count(RB * p.tl.bz, p.tl.nq, 2 * R, HG);  // strip groups of the largest tile
     const int nring = (th + 2 * R) * (nq + 2) - th * nq;
     const int shot = a.shot0 + T.slot;
@@ -567,6 +573,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         b[r] = masked(a.mat + 2 * P, gi, gj0);
         lam[r] = masked(a.mat, gi, gj0);
         mu[r] = masked(a.mat + P, gi, gj0);
+        if (SM > 0) st4s(s_mat + 4 * (r * NT + tid), lam[r]);
+        if (SM > 1) st4s(s_mat + 4 * ((RB + r) * NT + tid), mu[r]);
+        if (SM > 2) st4s(s_mat + 4 * ((2 * RB + r) * NT + tid), b[r]);
         damp = damp || damped(gi, gj0);
         if (SETS && gi >= a.qlo && gi <= a.qhi_z && gj0 + 3 >= a.qlo && gj0 <= a.qhi_x) img |= 1u << r;
     }
@@ -608,6 +617,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         tr[4 * a.trace_plane] = s_txz[rec_o];
     };
 
+    auto lam_of = [&](int r) { return SM > 0 ? ld4s(s_mat + 4 * (r * NT + tid)) : lam[r]; };
+    auto mu_of = [&](int r) { return SM > 1 ? ld4s(s_mat + 4 * ((RB + r) * NT + tid)) : mu[r]; };
+    auto b_of = [&](int r) { return SM > 2 ? ld4s(s_mat + 4 * ((2 * RB + r) * NT + tid)) : b[r]; };
     // Four values of a set: (QD 3) zero on columns outside the update domain.
     auto within = [&](float (&s)[4]) {
         if (QD == 3)
@@ -623,11 +635,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
                 float x[12], s[4], n[4];
+                const float4 br4 = b_of(r);
                 xrow<R, false>(x, sxx[r], s_txx + ot + r * W);  // Dx- txx
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     s[k] = xbwd<R>(x, k, a.k.cx) + z.at(r, k, a.k.cz);
-                    n[k] = f4(vx[r], k) + dt * (f4(b[r], k) * s[k]);
+                    n[k] = f4(vx[r], k) + dt * (f4(br4, k) * s[k]);
                 }
                 if (SETS && qi && (img >> r & 1)) qst4s(qi + Q_TXS * P + co + r * g.pitch, within(s));
                 vx[r] = mk4(n);
@@ -638,11 +651,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
                 float x[12], s[4], n[4];
+                const float4 br4 = b_of(r);
                 xrow<R, true>(x, sxz[r], s_txz + ot + r * W);  // Dx+ txz
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     s[k] = z.at(r, k, a.k.cz) + xfwd<R>(x, k, a.k.cx);
-                    n[k] = f4(vz[r], k) + dt * (f4(b[r], k) * s[k]);
+                    n[k] = f4(vz[r], k) + dt * (f4(br4, k) * s[k]);
                 }
                 if (SETS && qi && (img >> r & 1)) qst4s(qi + Q_TZS * P + co + r * g.pitch, within(s));
                 vz[r] = mk4(n);
@@ -730,9 +744,10 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                     qst4s(q + Q_DZM_VZ * P, mk4(ez));
                     qst4s(q + Q_VZS * P, mk4(s));
                 }
+                const float4 l4 = lam_of(r), m4 = mu_of(r);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {  // normal_pair_fwd, the damping apart
-                    const float l = f4(lam[r], k), m = f4(mu[r], k), l2m = l + 2.f * m;
+                    const float l = f4(l4, k), m = f4(m4, k), l2m = l + 2.f * m;
                     oxx[k] = __fmaf_rn(dt, __fmaf_rn(l2m, ex[k], __fmul_rn(l, ez[k])), f4(sxx[r], k));
                     ozz[k] = __fmaf_rn(dt, __fmaf_rn(l, ex[k], __fmul_rn(l2m, ez[k])), f4(szz[r], k));
                 }
@@ -744,8 +759,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
             float oxz[4];
+            const float4 m4 = mu_of(r);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) oxz[k] = f4(sxz[r], k) + dt * (f4(mu[r], k) * (f4(hx[r], k) + zx.at(r, k, a.k.cz)));
+            for (int k = 0; k < 4; ++k) oxz[k] = f4(sxz[r], k) + dt * (f4(m4, k) * (f4(hx[r], k) + zx.at(r, k, a.k.cz)));
             if (QD == 3 && (img >> r & 1)) {
                 float s[4];
 #pragma unroll
