@@ -179,7 +179,7 @@ template <int R, int RB>
 constexpr int RES_OWN = RB < 3 ? 4 * RB * RES_THREADS : ResShape<R>::OPLANE;  // a plane of the blocks alone
 template <int R, int RB>
 constexpr int ADJ_RES_FLOATS = RES_PAD + 5 * RES_PLANE + (RB < 2 ? 2 : 3) * RES_OWN<R, RB> + 22 * ResShape<R>::RING + 2 * RES_ROWS +
-                               3 * RES_W + 3 * RES_THREADS + 4 * RES_SETS<RB> * RES_THREADS;
+                               3 * RES_W + 4 * RES_SETS<RB> * RES_THREADS;
 template <int R, int RB>
 constexpr int EXA_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 2 * RES_OWN<R, RB> + 14 * ResShape<R>::RING + RES_ROWS + RES_W +
                                4 * RES_THREADS;
@@ -240,28 +240,26 @@ __device__ __forceinline__ void halo_words(unsigned *word, const Grid &g, const 
 // Each of the words read until its tag is `tag`, then handed to put(offset,
 // word of the group, value).  False when the wait gave up (error word set,
 // here or by another CTA).
-template <int W, bool LEAN, class Put>
+template <int W, class Put>
 __device__ __forceinline__ bool fetch_halo(const uint4 *buf, unsigned tag, const unsigned *words, int *err,
                                            unsigned long long limit_ns, Put put)
 {
     unsigned long long t0 = 0;
-    unsigned open = 0, kept[W];
-    // LEAN: a word's place is read again where it is used, for kernels that are short of registers
-    auto word = [&](int k) { return LEAN ? words[k * RES_THREADS + threadIdx.x] : kept[k]; };
+    unsigned open = 0, word[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-        kept[k] = words[k * RES_THREADS + threadIdx.x];
-        if (kept[k] != ~0u) open |= 1u << k;
+        word[k] = words[k * RES_THREADS + threadIdx.x];
+        if (word[k] != ~0u) open |= 1u << k;
     }
     for (unsigned n = 1; open; ++n) {
         uint4 v[W];
 #pragma unroll
         for (int k = 0; k < W; ++k)
-            if (open >> k & 1) v[k] = ld_word(buf + (word(k) >> 14));
+            if (open >> k & 1) v[k] = ld_word(buf + (word[k] >> 14));
 #pragma unroll
         for (int k = 0; k < W; ++k)
             if ((open >> k & 1) && v[k].w == tag) {
-                const unsigned u = word(k);
+                const unsigned u = word[k];
                 open &= ~(1u << k);
                 put((int)(u & 0x3FFFu), (int)(u >> 14 & 3u), v[k]);
             }
@@ -275,6 +273,56 @@ __device__ __forceinline__ bool fetch_halo(const uint4 *buf, unsigned tag, const
             }
         }
     }
+    return true;
+}
+
+// This thread's halo group: where it lies in the exchange buffer (its strip
+// group, 16 bits) and where its values go (14 bits); ~0u: none.
+template <int R>
+__device__ __forceinline__ unsigned halo_group(const Grid &g, const ResTiles &tl, int frame, int slot, int tz, int tx, int i0,
+                                               int th, int q0, int nq)
+{
+    constexpr int HG = ResShape<R>::HG;
+    if ((int)threadIdx.x >= (th + 4 * R) * (nq + 2 * HG) - th * nq) return ~0u;
+    int r, q;
+    frame_item(threadIdx.x, th + 4 * R, nq + 2 * HG, 2 * R, HG, r, q);
+    const unsigned src = halo_source<R>(g, tl, frame, slot, tz, tx, i0, th, q0, nq, i0 - 2 * R + r, q0 - HG + q);
+    return src == ~0u ? src : src << 14 | (unsigned)(r * RES_W + 4 * q);
+}
+
+// The W words of a halo group, each read until its tag is `tag`, then handed to
+// put(offset, words); as fetch_halo.  A thread that takes a whole group needs one
+// address and stores four values at a time, where words dealt out evenly are
+// fewer per thread.  Measured, us per step: backward (three words, the two
+// velocity products) 240 x 440 cells, 1 shot 2.96 with dealt words, 2.65 with
+// groups; forward (four, three stresses) 2.39 and 2.50.
+template <int W, class Put>
+__device__ __forceinline__ bool fetch_group(const uint4 *buf, unsigned tag, unsigned group, int *err,
+                                           unsigned long long limit_ns, Put put)
+{
+    if (group == ~0u) return true;
+    buf += 4 * (group >> 14);
+    unsigned long long t0 = 0;
+    unsigned open = (1u << W) - 1;
+    uint4 v[W];
+    for (unsigned n = 1; open; ++n) {
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if (open >> k & 1) v[k] = ld_word(buf + k);
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            if (v[k].w == tag) open &= ~(1u << k);
+        if (open && (n & 63u) == 0) {
+            if (ld_relaxed_gpu(err) != 0) return false;
+            if (!t0) {
+                t0 = global_ns();
+            } else if (global_ns() - t0 > limit_ns) {
+                atomicCAS(err, 0, 3);
+                return false;
+            }
+        }
+    }
+    put((int)(group & 0x3FFFu), v);
     return true;
 }
 
@@ -842,7 +890,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1) {
                 if (t > p.t0) {  // the neighbours' strips of S_t
-                    if (!fetch_halo<4, false>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t - p.t0), t_word, p.err, p.limit_ns, put))
+                    if (!fetch_halo<4>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t - p.t0), t_word, p.err, p.limit_ns, put))
                         s_stop = 1;
                     __syncthreads();
                     stop = s_stop;
@@ -971,8 +1019,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
     float *const s_dx = s_ring + 20 * RING, *const s_mx = s_dx + W, *const s_dz = s_mx + W;  // damping; -dt on the domain's columns
     unsigned *const t_ring = reinterpret_cast<unsigned *>(s_dz + RES_ROWS);
     int *const t_rslot = reinterpret_cast<int *>(t_ring + RING);  // slots of the ring's items
-    unsigned *const t_word = reinterpret_cast<unsigned *>(t_rslot + RING);  // the threads' halo words
-    float *const s_res = reinterpret_cast<float *>(t_word + 3 * RES_THREADS);  // [2][5][slots][4] staged residuals
+    float *const s_res = reinterpret_cast<float *>(t_rslot + RING);  // [2][5][slots][4] staged residuals
     int *const t_dst = reinterpret_cast<int *>(s_res + 40 * p.slots);  // [4 slots] where a receiver's residual goes
     const int nring = (th + 2 * R) * (nq + 2) - th * nq;
     const float dt = a.k.dt;
@@ -1144,13 +1191,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
         }
     };
     const int t_first = p.t_hi - 1;
+    const unsigned halo = halo_group<R>(g, p.tl, frame, T.slot, T.tz, T.tx, i0, th, T.q0, nq);
     // word w of a group holds values 3 w .. of its 4 vx and 4 vz products
-    halo_words<R, 3>(t_word, g, p.tl, frame, T.slot, T.tz, T.tx, i0, th, T.q0, nq);
-    auto put = [&](int o, int w, const uint4 &v) {
-        const int f = 3 * w;
-        (f < 4 ? s_pvx + o + f : s_pvz + o + f - 4)[0] = __uint_as_float(v.x);
-        (f + 1 < 4 ? s_pvx + o + f + 1 : s_pvz + o + f - 3)[0] = __uint_as_float(v.y);
-        if (w < 2) (w == 0 ? s_pvx + o + 2 : s_pvz + o + 1)[0] = __uint_as_float(v.z);
+    auto put = [&](int o, const uint4 (&w)[3]) {
+        auto f = [](unsigned u) { return __uint_as_float(u); };
+        st4s(s_pvx + o, make_float4(f(w[0].x), f(w[0].y), f(w[0].z), f(w[1].x)));
+        st4s(s_pvz + o, make_float4(f(w[1].y), f(w[1].z), f(w[2].x), f(w[2].y)));
     };
     // A step injects where its t mod dt_scale is 0 (step 0 never runs); kept by counting down: that of t, and
     // the residual row of the next injecting step below t.
@@ -1371,7 +1417,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1 && t < t_first) {  // the neighbours' products of this step's input
-                if (!fetch_halo<3, (RB == 3)>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
+                if (!fetch_group<3>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), halo, p.err, p.limit_ns, put))
                     s_stop = 1;
                 __syncthreads();
                 stop = s_stop;
@@ -1913,7 +1959,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1 && t < t_first) {
-                if (!fetch_halo<4, false>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
+                if (!fetch_halo<4>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), t_word, p.err, p.limit_ns, put))
                     s_stop = 1;
                 __syncthreads();
                 stop = s_stop;
