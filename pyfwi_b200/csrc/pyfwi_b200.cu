@@ -860,10 +860,11 @@ Buf slot_of(const Buf &b, int slot) { return {b.base + slot * b.stride, b.stride
 
 // Forward steps [t0, t1) of slots c0 .. c0 + n - 1 of the group starting at
 // shot s0, from state `in` (slot 0's) to `out`; sets: their difference sets
-// or states (null: neither is stored), the first of which is that of step q_t0.  Several launches
+// or states (null: neither is stored), the first of which is that of step q_t0,
+// or (checkpoints) the states of the steps in p->chp.  Several launches
 // when more source samples than travel with one are not zero.
 int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl, int t0, int t1, const Buf &in,
-                     const Buf &out, float *traces, const Buf *sets, int q_t0, cudaStream_t st)
+                     const Buf &out, float *traces, const Buf *sets, int q_t0, cudaStream_t st, bool checkpoints = false)
 {
     const pyfwi_geometry &G = p->geom;
     FwdResArgs fa;
@@ -879,7 +880,8 @@ int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl
     fa.record = traces != nullptr;
     fa.q_t0 = q_t0;
     if (sets) {
-        fa.store = p->exact_adj ? 3 : p->qd ? 1 : 2;
+        fa.store = checkpoints ? 2 : p->exact_adj ? 3 : p->qd ? 1 : 2;
+        fa.some = checkpoints;
         if (p->exact_adj) {  // whose gradient takes the whole update domain
             fa.a.qlo = p->R;
             fa.a.qhi_z = p->g.tnz - p->R;
@@ -897,7 +899,15 @@ int resident_forward(pyfwi_plan *p, void *ws, int s0, int c0, const ResTiles &tl
         fa.k0 = t / G.dt_scale;
         const int left = std::min(last, (t1 - 1) / G.dt_scale) - fa.k0 + 1;
         fa.nk = std::max(0, std::min(left, RES_MAX_SAMPLES));
-        const int te = left > RES_MAX_SAMPLES ? (fa.k0 + RES_MAX_SAMPLES) * G.dt_scale : t1;
+        int te = left > RES_MAX_SAMPLES ? (fa.k0 + RES_MAX_SAMPLES) * G.dt_scale : t1;
+        if (checkpoints) {
+            te = std::min(te, t + RES_KEEP_STEPS);
+            memset(fa.keep, 0, sizeof fa.keep);
+            size_t k = 0;
+            for (; k < p->chp.size() && p->chp[k] < t; ++k) {}
+            fa.q = slot_of(*sets, c0).base + (long long)k * p->state;
+            for (; k < p->chp.size() && p->chp[k] < te; ++k) fa.keep[(p->chp[k] - t) >> 5] |= 1u << ((p->chp[k] - t) & 31);
+        }
         for (int q = 0; q < fa.nk; ++q) fa.wav[q] = src_at(p, fa.k0 + q);
         const Buf to = te == t1 ? out : slot_of(work_state(p, ws, te & 1), c0);
         fa.t0 = t;
@@ -970,9 +980,45 @@ int resident_adjoint(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, const 
     return PYFWI_OK;
 }
 
+// The states of steps t_hi - 1 .. t_lo of a whole group from that of step t_hi
+// (at `in`), into the ring of reconstructed states.
+int resident_reverse(pyfwi_plan *p, void *ws, int n, int t_hi, int t_lo, const Buf &in, int ring, cudaStream_t st)
+{
+    RevResArgs r;
+    memset(&r, 0, sizeof r);
+    r.a = base_step(p, ws);
+    r.a.in_stride = in.stride;
+    r.xch = at<uint4>(ws, p->o_xch);
+    r.state = p->state;
+    r.t_hi = t_hi;
+    r.t_lo = t_lo;
+    r.ring = ring;
+    r.q_stride = ring * p->state;
+    r.err = at<int>(ws, ERR_OFF);
+    r.limit_ns = BARRIER_WAIT_NS;
+    ResTiles tl;
+    if (!resident_tiles(p->g, p->R, p->lines, n, p->sms, RES_FORWARD, &tl))
+        return fail(PYFWI_E_INVALID, "the reverse-time loop does not fit on chip");
+    const int conc = tl.nslots;
+    const Buf out = {at<float>(ws, p->o_states), r.q_stride};
+    for (int c0 = 0; c0 < n; c0 += conc) {
+        tl.nslots = std::min(conc, n - c0);
+        r.tl = tl;
+        r.a.in = slot_of(in, c0).base;
+        r.q = slot_of(out, c0).base;
+        r.tag0 = p->tag;
+        p->tag += (unsigned)(t_hi - t_lo) + 1;
+        ProfileScope prof(p, st, 0, tl.nslots * (t_hi - t_lo));
+        cudaError_t e = launch_rev_resident(r, p->R, st);
+        if (e != cudaSuccess) return fail(PYFWI_E_CUDA, "resident reverse-time launch: %s", cudaGetErrorString(e));
+        p->launches++;
+    }
+    return PYFWI_OK;
+}
+
 // The same with the sets formed from the states, a chunk of steps at a time;
-// state(t): where S_{t+1} is, called for each step of a chunk in backward
-// order before any of the chunk's sets are formed.
+// state(t, lo): where S_{t+1} is, called for each step of a chunk (whose last
+// is lo) in backward order before any of the chunk's sets are formed.
 template <class State>
 int resident_chunks(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, State state, int t_hi, int t_lo, int &ping,
                     float *adj, cudaStream_t st)
@@ -992,7 +1038,7 @@ int resident_chunks(pyfwi_plan *p, void *ws, const AdjArgs &base, int n, State s
         const int lo = std::max(t_lo, hi - p->rchunk);
         a.nsteps = hi - lo;
         for (int t = hi - 1; t >= lo; --t) {
-            const Buf s = state(t);
+            const Buf s = state(t, lo);
             if (!s.base) return fail(PYFWI_E_STATE, "no state to image at step %d", t);
             a.S[hi - 1 - t] = s.base;
             a.s_stride[hi - 1 - t] = s.stride;
@@ -1102,7 +1148,7 @@ Buf chp_state(pyfwi_plan *p, void *ws, int s0, int k)
     return {store + (long long)s0 * stride + (long long)k * p->state, stride};
 }
 
-// The forward pass of a group on chip, from checkpoint to checkpoint.
+// The forward pass of a group on chip, its checkpoints kept on the way.
 int resident_reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream_t st)
 {
     ResTiles tl;
@@ -1110,21 +1156,13 @@ int resident_reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces,
         return fail(PYFWI_E_INVALID, "the forward pass does not fit on chip");
     int rc = clear_exchange(p, ws, st);
     if (rc) return rc;
-    const int conc = tl.nslots;
+    const int conc = tl.nslots, nt = p->geom.nt;
+    const Buf kept = chp_state(p, ws, s0, 0);
     for (int c0 = 0; c0 < n; c0 += conc) {
         tl.nslots = std::min(conc, n - c0);
-        Buf cur = slot_of(work_state(p, ws, 0), c0);
-        int t = 0;
-        for (size_t kc = 0; t < p->geom.nt; ++kc) {
-            const bool keep = kc < p->chp.size();
-            const int t1 = keep ? p->chp[kc] + 1 : p->geom.nt;
-            const Buf out = slot_of(keep ? chp_state(p, ws, s0, (int)kc) : work_state(p, ws, 1), c0);
-            if (t1 <= t) continue;  // listed again
-            rc = resident_forward(p, ws, s0, c0, tl, t, t1, cur, out, traces, nullptr, 0, st);
-            if (rc) return rc;
-            cur = out;
-            t = t1;
-        }
+        rc = resident_forward(p, ws, s0, c0, tl, 0, nt, slot_of(work_state(p, ws, 0), c0), slot_of(work_state(p, ws, 1), c0),
+                              traces, &kept, 0, st, true);
+        if (rc) return rc;
     }
     return PYFWI_OK;
 }
@@ -1507,7 +1545,7 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
                 if (p->qd)
                     rc = resident_adjoint(p, ws, a, n, seg_state(p, ws, m, 0), t_lo, t_hi, std::max(t_lo, 1), ping, adj, st);
                 else
-                    rc = resident_chunks(p, ws, a, n, [&](int t) { return seg_state(p, ws, m, t - t_lo); }, t_hi,
+                    rc = resident_chunks(p, ws, a, n, [&](int t, int) { return seg_state(p, ws, m, t - t_lo); }, t_hi,
                                          std::max(t_lo, 1), ping, adj, st);
                 if (rc) return rc;
             }
@@ -1592,8 +1630,19 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
                 rc = clear_exchange(p, ws, st);
                 if (rc) return rc;
                 const int ring = p->rchunk + 1;  // the newest state of a chunk is still read by the next one's first step
-                auto in_ring = [&](int t) {
-                    return state(t, {at<float>(ws, p->o_states) + (long long)(t % ring) * p->state, ring * p->state});
+                int done = G.nt;                 // states of steps from here on are there
+                auto in_ring = [&](int t, int lo) {
+                    const Buf slot = {at<float>(ws, p->o_states) + (long long)(t % ring) * p->state, ring * p->state};
+                    if (t >= done) return slot;
+                    const int kk = chpc >= 0 ? chpc : chpc + nchp;
+                    if (t != p->chp[kk] && cur.base) {  // down to the chunk's end or the next checkpoint
+                        const int to = std::max(lo, p->chp[kk] < t ? p->chp[kk] + 1 : 0);
+                        rc = resident_reverse(p, ws, n, t + 1, to, cur, ring, st);
+                        done = to;
+                        cur = {at<float>(ws, p->o_states) + (long long)(to % ring) * p->state, ring * p->state};
+                        return rc ? Buf{nullptr, 0} : slot;
+                    }
+                    return state(t, slot);
                 };
                 rc = resident_chunks(p, ws, a, n, in_ring, G.nt, 1, ping, adj, st);
                 if (rc) return rc;
@@ -1866,10 +1915,11 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
     if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
     if (p->resident && !p->qd && !p->exact_adj) {
-        // long enough that the launches' own cost is a small part, in at most 256 MB or half of the states kept
+        // long enough that the launches' own cost is a small part, in a quarter of the memory of the states kept
+        // or, up to half of it, 256 MB
         const size_t kept = opt->checkpoint == PYFWI_CKPT_EXACT ? (size_t)p->seg : p->chp.size() * G.ns / p->G;
         const size_t room = (256ull << 20) / ((size_t)p->state * sizeof(float) * p->G);
-        p->rchunk = (int)std::max<size_t>(4, std::min<size_t>({(size_t)SETS_STEPS, room, kept / 2}));
+        p->rchunk = (int)std::min<size_t>(SETS_STEPS, std::max<size_t>({4, kept / 4, std::min(kept / 2, room)}));
     }
 
     const size_t pf = (size_t)p->g.plane * sizeof(float), sb = (size_t)p->state * sizeof(float);

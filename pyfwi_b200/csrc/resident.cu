@@ -9,6 +9,8 @@ namespace pyfwi {
 template cudaError_t launch_fwd_resident_r<2>(FwdResArgs &a, cudaStream_t s);
 template cudaError_t launch_adj_resident_r<2>(AdjResArgs &a, cudaStream_t s);
 template cudaError_t launch_exact_resident_r<2>(AdjResArgs &a, cudaStream_t s);
+template cudaError_t launch_rev_resident_r<2>(RevResArgs &a, cudaStream_t s);
+extern template cudaError_t launch_rev_resident_r<4>(RevResArgs &a, cudaStream_t s);
 extern template cudaError_t launch_fwd_resident_r<4>(FwdResArgs &a, cudaStream_t s);
 extern template cudaError_t launch_adj_resident_r<4>(AdjResArgs &a, cudaStream_t s);
 extern template cudaError_t launch_exact_resident_r<4>(AdjResArgs &a, cudaStream_t s);
@@ -28,7 +30,9 @@ bool fits(int th, int nq, int rb, int ctas, const Lines &lines, ResLoop loop)
             (loop == RES_EXACT ? exact_res_floats<R>(rb) : adj_res_floats<R>(rb)) + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
 }
 
-static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_FLOATS, "the forward loop fits on an SM");
+static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_FLOATS && REV_RES_FLOATS<2, 3> <= MAX_FLOATS &&
+                  REV_RES_FLOATS<4, 3> <= MAX_FLOATS,
+              "the forward and reverse-time loops fit on an SM");
 
 }  // namespace
 
@@ -78,6 +82,11 @@ bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms
 cudaError_t launch_fwd_resident(FwdResArgs &a, int R, cudaStream_t s)
 {
     return R == 2 ? launch_fwd_resident_r<2>(a, s) : launch_fwd_resident_r<4>(a, s);
+}
+
+cudaError_t launch_rev_resident(RevResArgs &a, int R, cudaStream_t s)
+{
+    return R == 2 ? launch_rev_resident_r<2>(a, s) : launch_rev_resident_r<4>(a, s);
 }
 
 cudaError_t launch_exact_resident(AdjResArgs &a, int R, cudaStream_t s)

@@ -58,6 +58,7 @@ constexpr int RES_NAN = 0x7fc00000;    // what a loop that gave up leaves
 constexpr int RES_MAX_SLOTS = 1000;   // 4-cell groups with receivers of a CTA (10 bits)
 constexpr size_t RES_XCH_BYTES = 2ull * RES_MAX_STRIPS * 64;  // exchange buffer of a workspace
 constexpr int RES_MAX_SAMPLES = 1024; // source samples that travel as launch parameters
+constexpr int RES_KEEP_STEPS = 2048;  // steps of a launch that keeps some states
 
 // Tiles of a resident launch.  Rows are dealt out in blocks of rb; the last
 // block may reach past the grid, where nothing moves.
@@ -140,8 +141,10 @@ struct FwdResArgs {
     float *q;          // difference sets (store 1) or states (2) of slot 0 (a.q_stride apart): S_{t+1}'s at
                        // q + (t - q_t0) * state; 3: the exact adjoint's sets of step t
     int q_t0, store;
+    int some;          // store 2: only the states of the steps in `keep`, one after another from q on
     int *err;
     unsigned long long limit_ns;
+    unsigned keep[RES_KEEP_STEPS / 32];  // bit t - t0: step t's state
     int k0, nk;        // samples k0 .. k0 + nk - 1 are in wav, the others are zero
     float4 wav[RES_MAX_SAMPLES];
 };
@@ -157,6 +160,20 @@ struct AdjResArgs {
     const float *q;    // the set of S_{t+1} at q + (t - q_t0) * state, slots a.fwd_stride apart
     int q_t0;
     int slots;         // 4-cell groups with receivers whose residuals a CTA stages
+    int *err;
+    unsigned long long limit_ns;
+};
+
+struct RevResArgs {
+    StepArgs a;        // constant fields; in: the state of step t_hi
+    ResTiles tl;
+    uint4 *xch;
+    unsigned tag0;     // tag of the strips that step t reads: tag0 + t_hi - 1 - t
+    long long state;
+    int t_hi, t_lo;    // the states of steps t_hi - 1 .. t_lo
+    float *q;          // that of step t, slot 0, at q + (t % ring) * state, slots q_stride apart
+    long long q_stride;
+    int ring;
     int *err;
     unsigned long long limit_ns;
 };
@@ -180,6 +197,9 @@ constexpr int RES_OWN = RB < 3 ? 4 * RB * RES_THREADS : ResShape<R>::OPLANE;  //
 template <int R, int RB>
 constexpr int ADJ_RES_FLOATS = RES_PAD + 5 * RES_PLANE + (RB < 2 ? 2 : 3) * RES_OWN<R, RB> + 22 * ResShape<R>::RING + 2 * RES_ROWS +
                                3 * RES_W + 4 * RES_SETS<RB> * RES_THREADS;
+template <int R, int RB>
+constexpr int REV_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 21 * ResShape<R>::RING + RES_ROWS + RES_W +
+                               4 * FWD_SHARED_MATS<RB> * RB * RES_THREADS;
 template <int R, int RB>
 constexpr int EXA_RES_FLOATS = RES_PAD + 5 * RES_PLANE + 2 * RES_OWN<R, RB> + 14 * ResShape<R>::RING + RES_ROWS + RES_W +
                                4 * RES_THREADS;
@@ -850,6 +870,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
     // ring items go to the threads without a block first, then to those inside
     const int rank = tid >= T.nblk ? tid - T.nblk : tid + NT - T.nblk;
     bool stop = s_stop;
+    int nkept = 0;
     for (int t = p.t0; t < p.t1 && !stop; ++t) {
         if (rec_o >= 0 && sub == 0 && k < p.nt_ext) record_t(k);
         // this step's source sample, where it reaches the tile (uniform over the CTA)
@@ -935,7 +956,10 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         __syncthreads();
         if (mine) stress(strip + ((t + 1) & 1) * xpar, p.tag0 + (unsigned)(t + 1 - p.t0), qo);
         if constexpr (QD == 2) {
-            if (mine)
+            const bool keep = !p.some || (p.keep[(t - p.t0) >> 5] >> ((t - p.t0) & 31) & 1u);
+            if (p.some) qo = p.q + (long long)nkept * p.state + T.slot * a.q_stride;
+            nkept += keep;
+            if (mine && keep)
 #pragma unroll
                 for (int r = 0; r < RB; ++r) {
                     if (gi0 + r >= g.tnz) break;
@@ -1999,6 +2023,281 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
         *reinterpret_cast<float4 *>(G + P + co + r * g.pitch) = gmu[r];
         *reinterpret_cast<float4 *>(G + 2 * P + co + r * g.pitch) = gb[r];
     }
+}
+
+// ---------------------------------------------------------------------------
+// reverse-time steps (rev_step's arithmetic)
+// ---------------------------------------------------------------------------
+// The state of step t from that of step t + 1: stresses first, then velocities,
+// so it exchanges velocities and recomputes the ring's stresses, as
+// adj_resident does with its products.  Every state goes to memory, 20 bytes a
+// cell.  190 x 290 cells, 5 shots: 5.1 us a step in runs of nine, 8.2 in rev_step.
+template <int R, int RB>
+__global__ void __launch_bounds__(RES_THREADS, 1) rev_resident(const __grid_constant__ RevResArgs p)
+{
+    constexpr int NT = RES_THREADS, HX = ResShape<R>::HX, HG = ResShape<R>::HG;
+    extern __shared__ float4 smem4[];
+    __shared__ int s_stop;
+    const StepArgs &a = p.a;
+    const Grid &g = a.g;
+    const long long P = g.plane;
+    const int tid = threadIdx.x;
+    const ResTile T = res_tile<R, RB>(p.tl);
+    const int i0 = T.i0, j0 = T.j0, th = T.th, nq = T.nq;
+    constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING, SM = FWD_SHARED_MATS<RB>;
+    float *const sm = reinterpret_cast<float *>(smem4) + RES_PAD;
+    // Cell (r, c) of the tile lies at (r + 2R) * W + HX + c of every plane.
+    float *const s_vx = sm, *const s_vz = sm + PL, *const s_txx = sm + 2 * PL, *const s_tzz = sm + 3 * PL, *const s_txz = sm + 4 * PL;
+    float *const s_ring = sm + 5 * PL;                               // [ring item][5][4]: its stresses, lam, mu
+    float *const s_dx = s_ring + 20 * RING, *const s_dz = s_dx + W;  // damping
+    unsigned *const t_ring = reinterpret_cast<unsigned *>(s_dz + RES_ROWS);
+    float *const s_mat = reinterpret_cast<float *>(t_ring + RING);   // [lam, mu, b][row][thread][4], RB 3
+    const int nring = (th + 2 * R) * (nq + 2) - th * nq;
+    const float dt = a.k.dt;
+    const float *in = a.in + T.slot * a.in_stride;
+    const int frame = frame_count(RB * p.tl.bz, p.tl.nq, 2 * R, HG);
+    const int xpar = 4 * gridDim.x * frame;
+    uint4 *const strip = p.xch + 4 * blockIdx.x * frame;
+
+    if (tid == 0) s_stop = ld_relaxed_gpu(p.err) != 0;
+    for (int e = tid; e < (th + 4 * R) * (nq + 2 * HG); e += NT) {
+        const int r = e / (nq + 2 * HG), q = e - r * (nq + 2 * HG), o = r * W + 4 * q;
+        const int gi = i0 - 2 * R + r, gj = j0 - HX + 4 * q;
+        st4s(s_vx + o, ld4(in + VX * P, g, gi, gj));
+        st4s(s_vz + o, ld4(in + VZ * P, g, gi, gj));
+    }
+    // Zero materials outside the update domain, where every field is zero, keep it so.
+    auto masked = [&](const float *plane, int gi, int gj) {
+        float4 v = ld4(plane, g, gi, gj);
+        if (!in_domain(g, R, gi, gj)) v.x = 0.f;
+        if (!in_domain(g, R, gi, gj + 1)) v.y = 0.f;
+        if (!in_domain(g, R, gi, gj + 2)) v.z = 0.f;
+        if (!in_domain(g, R, gi, gj + 3)) v.w = 0.f;
+        return v;
+    };
+    for (int e = tid; e < nring; e += NT) {
+        int r, q;
+        frame_item(e, th + 2 * R, nq + 2, R, 1, r, q);
+        t_ring[e] = pack_item(r, q);
+        const int gi = i0 - R + r, gj = j0 - 4 + 4 * q;
+        float *s = s_ring + 20 * e;
+        st4s(s, ld4(in + TXX * P, g, gi, gj));
+        st4s(s + 4, ld4(in + TZZ * P, g, gi, gj));
+        st4s(s + 8, ld4(in + TXZ * P, g, gi, gj));
+        st4s(s + 12, masked(a.mat, gi, gj));
+        st4s(s + 16, masked(a.mat + P, gi, gj));
+    }
+    for (int e = tid; e < 4 * nq + 2 * HX; e += NT) {
+        const int c = j0 - HX + e + XO;
+        s_dx[e] = c >= 0 && c < g.pitch ? __ldg(a.dampx + c) : 0.f;
+    }
+    for (int e = tid; e < th + 4 * R; e += NT) {
+        const int i = i0 - 2 * R + e + ZO;
+        s_dz[e] = i >= 0 && i < g.rows ? __ldg(a.dampz + i) : 0.f;
+    }
+
+    const bool mine = tid < T.nblk, inside = tid < T.nin;
+    int bz = 0, bq = 0;
+    if (mine) res_block<R, RB>(T, tid, bz, bq);
+    const int br = bz * RB;
+    const int ot = (br + 2 * R) * W + HX + 4 * bq;
+    const int gi0 = i0 + br, gj0 = j0 + 4 * bq;
+    const int co = (gi0 + ZO) * g.pitch + gj0 + XO;
+    float4 vx[RB], vz[RB], sxx[RB], szz[RB], sxz[RB], b[RB], lam[RB], mu[RB];
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        vx[r] = vz[r] = sxx[r] = szz[r] = sxz[r] = b[r] = lam[r] = mu[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!mine) continue;
+        const int gi = gi0 + r;
+        vx[r] = ld4(in + VX * P, g, gi, gj0);
+        vz[r] = ld4(in + VZ * P, g, gi, gj0);
+        sxx[r] = ld4(in + TXX * P, g, gi, gj0);
+        szz[r] = ld4(in + TZZ * P, g, gi, gj0);
+        sxz[r] = ld4(in + TXZ * P, g, gi, gj0);
+        lam[r] = masked(a.mat, gi, gj0);
+        mu[r] = masked(a.mat + P, gi, gj0);
+        b[r] = masked(a.mat + 2 * P, gi, gj0);
+        if (SM) {
+            st4s(s_mat + 4 * (r * NT + tid), lam[r]);
+            st4s(s_mat + 4 * ((RB + r) * NT + tid), mu[r]);
+            st4s(s_mat + 4 * ((2 * RB + r) * NT + tid), b[r]);
+        }
+    }
+    auto lam_of = [&](int r) { return SM ? ld4s(s_mat + 4 * (r * NT + tid)) : lam[r]; };
+    auto mu_of = [&](int r) { return SM ? ld4s(s_mat + 4 * ((RB + r) * NT + tid)) : mu[r]; };
+    auto b_of = [&](int r) { return SM ? ld4s(s_mat + 4 * ((2 * RB + r) * NT + tid)) : b[r]; };
+    const unsigned halo = halo_group<R>(g, p.tl, frame, T.slot, T.tz, T.tx, i0, th, T.q0, nq);
+    auto put = [&](int o, const uint4 (&w)[3]) {
+        auto f = [](unsigned u) { return __uint_as_float(u); };
+        st4s(s_vx + o, make_float4(f(w[0].x), f(w[0].y), f(w[0].z), f(w[1].x)));
+        st4s(s_vz + o, make_float4(f(w[1].y), f(w[1].z), f(w[2].x), f(w[2].y)));
+    };
+    __syncthreads();
+
+    // New stresses of four cells.
+    auto update = [&](float4 &xx, float4 &zz, float4 &xz, const float4 &l, const float4 &m, const float4 &dx, float dz,
+                      const float (&ex)[4], const float (&ez)[4], const float (&exz)[4]) {
+        float oxx[4], ozz[4], oxz[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float d = f4(dx, k) + dz;
+            float txx = f4(xx, k), tzz = f4(zz, k), txz = f4(xz, k);
+            txz = txz - dt * (d * txz);
+            txz = txz - dt * (f4(m, k) * exz[k]);
+            normal_pair_rev(f4(l, k), f4(m, k), ex[k], ez[k], d, dt, txx, tzz);
+            oxx[k] = txx;
+            ozz[k] = tzz;
+            oxz[k] = txz;
+        }
+        xx = mk4(oxx);
+        zz = mk4(ozz);
+        xz = mk4(oxz);
+    };
+    auto stress = [&]() {
+        const float4 dx = ld4s(s_dx + HX + 4 * bq);
+        auto row_x = [&](int r) { return ld4s(s_vx + ot + r * W); };
+        auto row_z = [&](int r) { return ld4s(s_vz + ot + r * W); };
+        ZSlide<R, true> zx(row_x);
+        ZSlide<R, false> zz(row_z);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            zx.next(row_x(r + R));
+            zz.next(row_z(r + R - 1));
+            float x[12], ex[4], ez[4], exz[4];
+            xrow<R, true>(x, zx.centre(), s_vx + ot + r * W);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ex[k] = xfwd<R>(x, k, a.k.cx);
+            xrow<R, false>(x, zz.centre(), s_vz + ot + r * W);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                exz[k] = xbwd<R>(x, k, a.k.cx) + zx.at(k, a.k.cz);
+                ez[k] = zz.at(k, a.k.cz);
+            }
+            update(sxx[r], szz[r], sxz[r], lam_of(r), mu_of(r), dx, s_dz[br + r + 2 * R], ex, ez, exz);
+            st4s(s_txx + ot + r * W, sxx[r]);
+            st4s(s_tzz + ot + r * W, szz[r]);
+            st4s(s_txz + ot + r * W, sxz[r]);
+        }
+    };
+    auto ring = [&](int e) {
+        const int r = item_row(t_ring[e]), q = item_col(t_ring[e]), c = (r + R) * W + HX - 4 + 4 * q;
+        float *s = s_ring + 20 * e;
+        float x[12], ex[4], ez[4], exz[4];
+        {
+            const ZWindow<R, 1, true> zx([&](int) { return ld4s(s_vx + c); }, s_vx + c);
+            xrow<R, true>(x, zx.w[R - 1], s_vx + c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                ex[k] = xfwd<R>(x, k, a.k.cx);
+                exz[k] = zx.at(0, k, a.k.cz);
+            }
+        }
+        const ZWindow<R, 1, false> zz([&](int) { return ld4s(s_vz + c); }, s_vz + c);
+        xrow<R, false>(x, zz.w[R], s_vz + c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            ez[k] = zz.at(0, k, a.k.cz);
+            exz[k] = xbwd<R>(x, k, a.k.cx) + exz[k];
+        }
+        float4 xx = ld4s(s), zz4 = ld4s(s + 4), xz = ld4s(s + 8);
+        update(xx, zz4, xz, ld4s(s + 12), ld4s(s + 16), ld4s(s_dx + HX - 4 + 4 * q), s_dz[r + R], ex, ez, exz);
+        st4s(s, xx);
+        st4s(s + 4, zz4);
+        st4s(s + 8, xz);
+        st4s(s_txx + c, xx);
+        st4s(s_tzz + c, zz4);
+        st4s(s_txz + c, xz);
+    };
+
+    const int rank = tid >= T.nblk ? tid - T.nblk : tid + NT - T.nblk;
+    const int t_first = p.t_hi - 1;
+    bool stop = s_stop;
+    for (int t = t_first; t >= p.t_lo && !stop; --t) {
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass == 1 && t < t_first) {
+                if (!fetch_group<3>(p.xch + (t & 1) * xpar, p.tag0 + (unsigned)(t_first - t), halo, p.err, p.limit_ns, put)) s_stop = 1;
+                __syncthreads();
+                stop = s_stop;
+                if (stop) break;
+            }
+            if (mine && inside == (pass == 0)) stress();
+        }
+        if (stop) break;
+        for (int e = rank; e < nring; e += NT) ring(e);
+        __syncthreads();
+        if (mine) {
+            uint4 *const xo = strip + ((t - 1) & 1) * xpar;
+            const unsigned tag = p.tag0 + (unsigned)(t_first - t + 1);
+            float *const o0 = p.q + (long long)(t % p.ring) * p.state + T.slot * p.q_stride + co;
+            const float4 dx = ld4s(s_dx + HX + 4 * bq);
+            {
+                auto row = [&](int r) { return ld4s(s_txz + ot + r * W); };
+                ZSlide<R, false> z(row);
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    z.next(row(r + R - 1));
+                    const float4 bb = b_of(r);
+                    const float dz = s_dz[br + r + 2 * R];
+                    float x[12], n[4];
+                    xrow<R, false>(x, sxx[r], s_txx + ot + r * W);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float d = f4(dx, k) + dz;
+                        float v = f4(vx[r], k);
+                        v = v - dt * (d * v);
+                        n[k] = v - dt * (f4(bb, k) * (xbwd<R>(x, k, a.k.cx) + z.at(k, a.k.cz)));
+                    }
+                    vx[r] = mk4(n);
+                }
+            }
+            auto row = [&](int r) { return ld4s(s_tzz + ot + r * W); };
+            ZSlide<R, true> z(row);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                z.next(row(r + R));
+                const float4 bb = b_of(r);
+                const float dz = s_dz[br + r + 2 * R];
+                float x[12], n[4];
+                xrow<R, true>(x, sxz[r], s_txz + ot + r * W);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float d = f4(dx, k) + dz;
+                    float v = f4(vz[r], k);
+                    v = v - dt * (d * v);
+                    n[k] = v - dt * (f4(bb, k) * (z.at(k, a.k.cz) + xfwd<R>(x, k, a.k.cx)));
+                }
+                vz[r] = mk4(n);
+                st4s(s_vx + ot + r * W, vx[r]);
+                st4s(s_vz + ot + r * W, vz[r]);
+                if (!inside) {
+                    const int rr = br + r;
+                    if (rr < 2 * R || rr >= th - 2 * R || bq < HG || bq >= nq - HG) {
+                        uint4 *const s = xo + 4 * frame_index(rr, bq, th, nq, 2 * R, HG);
+                        st_word(s, vx[r].x, vx[r].y, vx[r].z, tag);
+                        st_word(s + 1, vx[r].w, vz[r].x, vz[r].y, tag);
+                        st_word(s + 2, vz[r].z, vz[r].w, 0.f, tag);
+                    }
+                }
+                if (gi0 + r < g.tnz) {
+                    float *o = o0 + r * g.pitch;
+                    qst4s(o + VX * P, vx[r]);
+                    qst4s(o + VZ * P, vz[r]);
+                    qst4s(o + TXX * P, sxx[r]);
+                    qst4s(o + TZZ * P, szz[r]);
+                    qst4s(o + TXZ * P, sxz[r]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (!stop || !mine) return;
+    const float nan = __int_as_float(RES_NAN);
+    for (int t = t_first; t >= p.t_lo; --t)
+        for (int r = 0; r < RB && gi0 + r < g.tnz; ++r)
+            for (int f = 0; f < 5; ++f)
+                qst4s(p.q + (long long)(t % p.ring) * p.state + T.slot * p.q_stride + co + r * g.pitch + f * P,
+                      make_float4(nan, nan, nan, nan));
 }
 
 }  // namespace pyfwi

@@ -50,6 +50,16 @@ cudaError_t launch_exact_resident_r(AdjResArgs &a, cudaStream_t s)
 }
 
 template <int R>
+cudaError_t launch_rev_resident_r(RevResArgs &a, cudaStream_t s)
+{
+#define CASE(RB_) \
+    if (a.tl.rb == RB_) return launch_resident(reinterpret_cast<const void *>(rev_resident<R, RB_>), a, REV_RES_FLOATS<R, RB_>, s);
+    CASE(1) CASE(2) CASE(3)
+#undef CASE
+    return cudaErrorInvalidValue;
+}
+
+template <int R>
 cudaError_t launch_fwd_resident_r(FwdResArgs &a, cudaStream_t s)
 {
 #define CASE(RB_, Q_) \

@@ -73,7 +73,7 @@ def _reverse(percent, *size):
 @pytest.mark.parametrize("what,extra", [("tiny_s8", {}), ("tiny_s8", {"segment": 11}), ("c1", {"energy_balancing": True}),
                                         ("tiny_chpr", {}), ("tiny_crosswell", {}), ((10, 190, 291, 5, 200), {}),
                                         ((5, 100, 121, 3, 150), {"shot_batch": 2}), ((60, 61, 70, 2, 90), {}),
-                                        ((20, 75, 90, 2, 120, 8), {})], ids=lambda v: str(v))
+                                        ((20, 75, 90, 2, 120, 8), {}), ((10, 33, 45, 2, 2100), {}), ((4, 300, 500, 2, 75), {})], ids=lambda v: str(v))
 def test_sets_formed_from_states(what, extra):
     """Energy terms (states stored) and reconstructed states: the difference
     sets are formed a chunk of steps at a time.  The step kernels' bits."""
