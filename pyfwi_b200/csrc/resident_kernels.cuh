@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
 {
     constexpr int NT = RES_THREADS, HX = ResShape<R>::HX, HG = ResShape<R>::HG;
     extern __shared__ float4 smem4[];
-    __shared__ int s_stop, s_nslot, s_line[4][6], s_t[6];
+    __shared__ int s_stop, s_nslot, s_line[4][6], s_t[4];
     const AdjArgs &a = p.a;
     const Grid &g = a.g;
     const long long P = g.plane;
@@ -1028,7 +1028,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
         s_t[1] = T.j0;
         s_t[2] = T.th;
         s_t[3] = T.nq;
-        s_t[4] = T.slot;
     }
     const int i0 = T.i0, j0 = T.j0, th = T.th, nq = T.nq;
     constexpr int W = RES_W, PL = RES_PLANE, RING = ResShape<R>::RING;
@@ -1263,7 +1262,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) adj_resident(const __grid_cons
 
     // Difference sets of step t.  One or two rows read a row's into registers, ahead of their use, and ask for
     // those of the step after it into L2.
-    auto sets_of = [&](int t) { return p.q + (long long)(t - p.q_t0) * p.state + (RB == 3 ? s_t[4] : T.slot) * a.fwd_stride + co_of(place()); };
+    auto sets_of = [&](int t) { return p.q + (long long)(t - p.q_t0) * p.state + T.slot * a.fwd_stride + co_of(place()); };
     float4 qv[5];
     auto load_set = [&](int t, int r) {
         if (!(img >> r & 1)) return;
