@@ -238,7 +238,7 @@ def max_over_ranks(ms, world, dev):
     return float(t.item())
 
 
-def roofline(prof, ms, ncell, nint, ns, nt, steps, store, snapshot, hbm, peak_src, traffic_dir):
+def roofline(prof, ms, ncell, nint, ns, nt, steps, store, snapshot, hbm, peak_src, traffic_dir, resident=False):
     """The roofline object of the JSON line from the profiled step kernels.
 
     prof[k] = (launches, device ms, cell-shots) of kernel kind k (0 forward,
@@ -249,16 +249,24 @@ def roofline(prof, ms, ncell, nint, ns, nt, steps, store, snapshot, hbm, peak_sr
     also write every shot-step's five values once.  traffic: the ncu DRAM
     bytes per cell-shot of a one-pass capture of the benchmark's launch shape
     (traffic_dir/traffic_<kernel>_c3[_differences].json, matching store and
-    snapshot format), times this run's average launch; None without one."""
+    snapshot format), times this run's average launch; None without one.
+
+    resident: a launch runs many steps with the wavefield on chip, and what
+    has to cross memory is the imaged values alone, written once by the
+    forward loop and read once by the adjoint loop.  Latency bounds those
+    loops, not memory: frac says how little of it they use."""
     # bytes per value of what the imaging reads: FP32 states or difference
     # sets, 24-bit (BF16 + byte) or BF16 snapshots
     vb = {"fp32": 4.0, "fp24": 3.0, "bf16": 2.0}[snapshot]
     q_bytes = 5 * vb * nint * int(ns) * int(nt) * steps if store == "differences" else 0.0
-    names = {0: "fwd_step", 1: "adj_step", 2: "rev_step"}
+    names = {0: "fwd_resident", 1: "adj_resident", 2: "rev_resident"} if resident else \
+        {0: "fwd_step", 1: "adj_step", 2: "rev_step"}
 
     def kernel_roof(k):
         n_l, ms_k, cells_k = prof[k]
-        if k == 1:
+        if resident:
+            alg = q_bytes if k == 0 else cells_k / ncell * nint * 5 * vb if k == 1 else cells_k * 20.0
+        elif k == 1:
             alg = cells_k * BYTES_ADJ + (cells_k / ncell) * nint * (5 * vb + 24.0)
         else:
             alg = cells_k * BYTES_FWD + (q_bytes if k == 0 else 0.0)
@@ -289,7 +297,7 @@ def roofline(prof, ms, ncell, nint, ns, nt, steps, store, snapshot, hbm, peak_sr
     dom = max(prof, key=lambda k: prof[k][1])  # dominant kernel: the most device time
     kr = per_kernel[names[dom]]
     traffic, traffic_src = traffic_for(dom)
-    return {"bound": "hbm", "kernel": names[dom], "achieved": kr["achieved"], "peak": hbm, "unit": "GB/s",
+    return {"bound": "latency" if resident else "hbm", "kernel": names[dom], "achieved": kr["achieved"], "peak": hbm, "unit": "GB/s",
             "frac": kr["frac"], "traffic": traffic, "traffic_source": traffic_src, "peak_source": peak_src,
             "launches": kr["launches"], "avg_launch_ms": kr["avg_launch_ms"],
             "alg_bytes_per_launch": kr["alg_bytes_per_launch"],
@@ -388,10 +396,10 @@ def run_ours(args, world, rank, local):
     misfit = float(rms.item())
     batched_shots_s = int(W.ns) * args.steps / (ms_max * 1e-3)
     shape = {"ns": int(W.ns), "nt": int(W.nt), "grid": [int(W.tnz), int(W.tnx)]}
-    W_store_diffs, W_snapshot = W.plan.store_diffs, W.snapshot
+    W_store_diffs, W_snapshot, W_resident = W.plan.store_diffs, W.snapshot, W.plan.resident
     layout = {"checkpoint": W.checkpoint, "segment": W.segment, "shot_batch": W.shot_batch,
               "overlap": int(W.plan.opts.overlap), "snapshot": W.snapshot,
-              "store": "differences" if W_store_diffs else "states",
+              "store": "differences" if W_store_diffs else "states", "resident": W_resident,
               "kernels": {"forward": int(W.tile), "adjoint": int(W.adj_tile)}}
     plain = None
     if world == 1 and (args.plain_shots > 0 or args.inversion > 0 or args.uneven > 0 or args.configs):
@@ -403,7 +411,7 @@ def run_ours(args, world, rank, local):
     hbm, peak_src = peaks()
     roof = roofline(prof, ms, ncell, nint, shape["ns"], shape["nt"], args.steps,
                     "differences" if W_store_diffs else "states", W_snapshot, hbm, peak_src,
-                    os.path.join(ROOT, "profiles") if args.config == "c3" else None)
+                    os.path.join(ROOT, "profiles") if args.config == "c3" else None, W_resident)
     small = None
     if world == 1 and args.configs:
         gc.collect()
