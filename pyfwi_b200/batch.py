@@ -39,8 +39,9 @@ class SurveyBatch:
         # persistent cooperative grid per survey would compete for the SMs)
         for W in self.props:
             W.persist_allowed = False
-            if W._plan is not None and W._plan.opts.persist:
+            if W._plan is not None and W._plan.opts.persist == 1:
                 W._plan = None  # rebuilt on first use, without persistent loops
+            # (a plan with resident loops is kept, and with it the survey's state)
         self._share_memory()
         self.graph = graph
         self._graph = None

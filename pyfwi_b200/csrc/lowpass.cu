@@ -356,8 +356,10 @@ cudaError_t launch(const Job &a, int nfft)
         constexpr int pairs = LOGN <= 12 ? 4 : LOGN == 13 ? 2 : 1;
         const long long ctas = (a.ncols + 2 * pairs - 1) / (2 * pairs);
         if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        const size_t smem = n_pass(LOGN) == 1 ? 0 : ((size_t)pairs * signal_places(nfft, pairs) + roots_before(LOGN, n_pass(LOGN) - 1)) * sizeof(float2);
-        const bool vec = a.ncols % 2 == 0 && reinterpret_cast<uintptr_t>(a.in) % 8 == 0 && reinterpret_cast<uintptr_t>(a.out) % 8 == 0;
+        const size_t places = (size_t)pairs * signal_places(nfft, pairs) + roots_before(LOGN, n_pass(LOGN) - 1);
+        const size_t smem = n_pass(LOGN) == 1 ? 0 : places * sizeof(float2);
+        const bool vec = a.ncols % 2 == 0 && reinterpret_cast<uintptr_t>(a.in) % 8 == 0 &&
+                         reinterpret_cast<uintptr_t>(a.out) % 8 == 0;
         auto kern = vec ? lowpass_fft_kernel<LOGN, true> : lowpass_fft_kernel<LOGN, false>;
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

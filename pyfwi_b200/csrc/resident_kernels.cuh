@@ -17,7 +17,8 @@
 //     parity) in 16-byte words of three values and the step's tag;
 //   * reads its up to eight neighbours' words until their tags match and puts
 //     the values into its halo (a few words per thread: a warp or two of their
-//     own took 4000 to 9000 cycles a step for a tile of 81 x 52 cells).
+//     own took 4000 to 9000 cycles a step for a tile of 81 x 52 cells, and the
+//     warps of the border alone a fifth longer than all of them).
 // The tag travels with the data (one 16-byte access is a single transaction),
 // so there is neither a flag nor a fence: a release of a flag word waits until
 // everything the SM has written is in L2, the difference sets included, which
@@ -46,7 +47,7 @@ namespace pyfwi {
 
 // Threads of a CTA, a block each: 12 warps leave 168 registers a thread.
 constexpr int RES_THREADS = 384;
-constexpr int RES_HALO = RES_THREADS; // halo groups of a tile, at most: one thread fetches at most a group's words
+constexpr int RES_HALO = RES_THREADS; // halo groups of a tile, at most: a thread fetches a group's words or fewer
 constexpr int RES_MAX_CTAS = 148;     // CTAs of a launch: the SMs of a B200
 constexpr int RES_MAX_STRIPS = 65536; // strip groups of all CTAs (a word's index takes 18 bits)
 constexpr int RES_PAD = 8;            // floats before the first plane: edge groups read past a row's start

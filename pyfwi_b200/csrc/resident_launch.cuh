@@ -63,7 +63,8 @@ template <int R>
 cudaError_t launch_fwd_resident_r(FwdResArgs &a, cudaStream_t s)
 {
 #define CASE(RB_, Q_) \
-    if (a.tl.rb == RB_ && a.store == Q_) return launch_resident(reinterpret_cast<const void *>(fwd_resident<R, RB_, Q_>), a, FWD_RES_FLOATS<R, RB_>, s);
+    if (a.tl.rb == RB_ && a.store == Q_)                                                                                      \
+        return launch_resident(reinterpret_cast<const void *>(fwd_resident<R, RB_, Q_>), a, FWD_RES_FLOATS<R, RB_>, s);
     CASE(1, 0) CASE(1, 1) CASE(1, 2) CASE(1, 3) CASE(2, 0) CASE(2, 1) CASE(2, 2) CASE(2, 3) CASE(3, 0) CASE(3, 1) CASE(3, 2)
     CASE(3, 3)
 #undef CASE
