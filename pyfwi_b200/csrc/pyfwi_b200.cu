@@ -119,7 +119,6 @@ struct pyfwi_plan {
     size_t o_hdr, o_src, o_red, o_mat, o_dampx, o_dampz, o_work, o_adj, o_gacc, o_store, o_store16, o_store8, o_xch, o_sets, o_states, total;
     long long launches = 0;
     bool model_set = false, fwd_valid = false;
-    bool sets_kept = false;  // exact adjoint: the last forward pass ran on chip and kept sets where others keep states
     // per-kernel event timing (pyfwi_profile_enable)
     bool profiling = false;
     struct Ev {
@@ -827,14 +826,14 @@ int last_diffs(pyfwi_plan *p, void *ws, int m, int t_hi, int n, cudaStream_t st)
 }
 
 // ---- resident time loops -----------------------------------------------------
-// This call's time loops run with the wavefield on chip: the plan allows it,
-// the device has the SMs, and the stream is not being captured by the caller
-// (cooperative launches stay out of the caller's graphs).
-bool use_resident(pyfwi_plan *p, cudaStream_t st)
+// The plan's time loops run with the wavefield on chip: the plan allows it and
+// the device has the SMs.  The answer is the same for every call of a plan, in a
+// caller's stream capture too (a cooperative launch becomes a node of the graph):
+// what the checkpoint store holds depends on it (sets or, for the exact adjoint's
+// step kernels, states), and a graph replays between calls that know nothing of it.
+bool use_resident(pyfwi_plan *p)
 {
     if (!p->resident) return false;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
     if (!p->sms) {
         int dev = 0, sms = 0, coop = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -842,10 +841,11 @@ bool use_resident(pyfwi_plan *p, cudaStream_t st)
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return false;
         p->sms = coop ? std::min(sms, RES_MAX_CTAS) : 1;
+        ResTiles tl;
+        p->resident = resident_tiles(p->g, p->R, p->lines, p->G, p->sms, RES_FORWARD, &tl) &&
+                      resident_tiles(p->g, p->R, p->lines, p->G, p->sms, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
     }
-    ResTiles tl;
-    return resident_tiles(p->g, p->R, p->lines, p->G, p->sms, RES_FORWARD, &tl) &&
-           resident_tiles(p->g, p->R, p->lines, p->G, p->sms, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
+    return p->resident;
 }
 
 // A call's first use of the exchange buffer: no word holds a tag of this call.
@@ -1112,8 +1112,7 @@ int exact_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream
     Buf z = exact_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(z.base + q * z.stride, 0, p->state * sizeof(float), st));
     if (use_persist(p, st)) return persist_pass(p, ws, s0, n, traces, st);
-    p->sets_kept = use_resident(p, st);
-    if (p->sets_kept) return resident_pass(p, ws, s0, n, traces, st);
+    if (use_resident(p)) return resident_pass(p, ws, s0, n, traces, st);
     StepArgs a = base_step(p, ws);
     a.shot0 = s0;
     a.traces = traces;
@@ -1172,7 +1171,7 @@ int reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStre
     // states stored after the steps listed in chp (wave_propagation.py:710-727)
     Buf cur = work_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(cur.base + q * cur.stride, 0, p->state * sizeof(float), st));
-    if (use_resident(p, st)) return resident_reverse_pass(p, ws, s0, n, traces, st);
+    if (use_resident(p)) return resident_reverse_pass(p, ws, s0, n, traces, st);
     int wcur = 0;  // work buffer holding the current state (-1: a checkpoint slot)
     size_t kc = 0;
     StepArgs a = base_step(p, ws);
@@ -1506,14 +1505,13 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
             if (rc) return rc;
             rc = misfit_group(p, *mf, s0, n, st);
             if (rc) return rc;
-        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT &&
-                   (p->ngroups > 1 || !p->fwd_valid || (p->exact_adj && p->sets_kept != use_resident(p, st)))) {
+        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && (p->ngroups > 1 || !p->fwd_valid)) {
             rc = exact_pass(p, ws, s0, n, nullptr, st);  // the states of this group are gone
             if (rc) return rc;
         }
         for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(adj + 2 * q * p->state, 0, p->state * sizeof(float), st));
         int ping = 0, t_src = G.nt_ext;
-        if (p->exact_adj && use_resident(p, st)) {
+        if (p->exact_adj && use_resident(p)) {
             rc = clear_exchange(p, ws, st);
             if (rc) return rc;
             for (int m = p->M - 1; m >= 0; --m) {
@@ -1532,7 +1530,7 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
         } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && p->overlap) {
             rc = overlap_backward(p, ws, a, s0, n, t_src, ping, adj, st);
             if (rc) return rc;
-        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && use_resident(p, st)) {
+        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && use_resident(p)) {
             rc = clear_exchange(p, ws, st);
             if (rc) return rc;
             for (int m = p->M - 1; m >= 0; --m) {
@@ -1626,7 +1624,7 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
                 cur = rc ? Buf{nullptr, 0} : to;
                 return cur;
             };
-            if (use_resident(p, st)) {
+            if (use_resident(p)) {
                 rc = clear_exchange(p, ws, st);
                 if (rc) return rc;
                 const int ring = p->rchunk + 1;  // the newest state of a chunk is still read by the next one's first step
