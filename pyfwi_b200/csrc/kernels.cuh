@@ -1935,6 +1935,37 @@ struct ExactArgs {
     int add_src;
 };
 
+// The formulas above, every rounding spelled out, so that the step kernel and
+// the resident loop give the same bits.
+__device__ __forceinline__ float exact_damp(float dt, float dx, float dz) { return __fmaf_rn(-dt, __fadd_rn(dx, dz), 1.f); }
+
+// P1 .. P3 of damped stresses a.
+__device__ __forceinline__ void exact_products(float dt, float lam, float mu, float axx, float azz, float axz, float &p1, float &p2,
+                                               float &p3)
+{
+    const float l2m = __fmaf_rn(2.f, mu, lam);
+    p1 = __fmul_rn(dt, __fmaf_rn(l2m, axx, __fmul_rn(lam, azz)));
+    p2 = __fmul_rn(dt, __fmul_rn(mu, axz));
+    p3 = __fmul_rn(dt, __fmaf_rn(lam, axx, __fmul_rn(l2m, azz)));
+}
+
+// Q1 or Q2 of a damped velocity B.
+__device__ __forceinline__ float exact_q(float dt, float b, float bv) { return __fmul_rn(dt, __fmul_rn(b, bv)); }
+
+// The gradients: xp, zm, cross the differences Dx+ vx, Dz- vz, Dx- vz + Dz+ vx
+// of S_{t+1}; sx, sz the two sums of stress differences of S_t with its source.
+__device__ __forceinline__ void exact_stress_terms(float dt, float axx, float azz, float axz, float xp, float zm, float cross,
+                                                   float &glam, float &gmu)
+{
+    glam = __fmaf_rn(__fmul_rn(dt, __fadd_rn(axx, azz)), __fadd_rn(xp, zm), glam);
+    gmu = __fmaf_rn(dt, __fmaf_rn(axz, cross, __fmaf_rn(2.f * axx, xp, __fmul_rn(2.f * azz, zm))), gmu);
+}
+
+__device__ __forceinline__ void exact_velocity_terms(float dt, float bvx, float bvz, float sx, float sz, float &gb)
+{
+    gb = __fmaf_rn(dt, __fmaf_rn(bvx, sx, __fmul_rn(bvz, sz)), gb);
+}
+
 // Coefficient of f[j + o] in a backward / forward difference at j.
 template <int R>
 __device__ __forceinline__ float coef_bwd(int o, const float *c)
@@ -1986,13 +2017,9 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
         float v1 = 0.f, v2 = 0.f, v3 = 0.f;
         if (in_domain(g, R, i, j)) {
             const long long co = cell_off(g, i, j);
-            const float damp = 1.f - dt * (__ldg(a.dampx + j + XO) + __ldg(a.dampz + i + ZO));
-            const float axx = damp * __ldg(L1 + TXX * P + co), azz = damp * __ldg(L1 + TZZ * P + co),
-                        axz = damp * __ldg(L1 + TXZ * P + co);
-            const float lam = __ldg(a.mat + co), mu = __ldg(a.mat + P + co), l2m = lam + 2.f * mu;
-            v1 = dt * (l2m * axx + lam * azz);
-            v2 = dt * (mu * axz);
-            v3 = dt * (lam * axx + l2m * azz);
+            const float damp = exact_damp(dt, __ldg(a.dampx + j + XO), __ldg(a.dampz + i + ZO));
+            exact_products(dt, __ldg(a.mat + co), __ldg(a.mat + P + co), __fmul_rn(damp, __ldg(L1 + TXX * P + co)),
+                           __fmul_rn(damp, __ldg(L1 + TZZ * P + co)), __fmul_rn(damp, __ldg(L1 + TXZ * P + co)), v1, v2, v3);
         }
         p1[e] = v1;
         p2[e] = v2;
@@ -2009,10 +2036,10 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
             const int ip = (r + R) * PW + c + R;
             const float mvx = __ldg(L1 + VX * P + co) - dbwd<R>(p1, ip, 1, a.k.cx) - dbwd<R>(p2, ip, PW, a.k.cz);
             const float mvz = __ldg(L1 + VZ * P + co) - dfwd<R>(p3, ip, PW, a.k.cz) - dfwd<R>(p2, ip, 1, a.k.cx);
-            const float damp = 1.f - dt * (__ldg(a.dampx + j + XO) + __ldg(a.dampz + i + ZO));
+            const float damp = exact_damp(dt, __ldg(a.dampx + j + XO), __ldg(a.dampz + i + ZO));
             const float b = __ldg(a.mat + 2 * P + co);
-            v1 = dt * (b * (damp * mvx));
-            v2 = dt * (b * (damp * mvz));
+            v1 = exact_q(dt, b, __fmul_rn(damp, mvx));
+            v2 = exact_q(dt, b, __fmul_rn(damp, mvz));
         }
         q1[e] = v1;
         q2[e] = v2;
@@ -2027,17 +2054,17 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
         const long long co = cell_off(g, i, j);
         const int ip = (r + 2 * R) * PW + c + 2 * R, iq = (r + R) * QW + c + R;
         const bool dom = in_domain(g, R, i, j);
-        const float damp = dom ? 1.f - dt * (__ldg(a.dampx + j + XO) + __ldg(a.dampz + i + ZO)) : 1.f;
+        const float damp = dom ? exact_damp(dt, __ldg(a.dampx + j + XO), __ldg(a.dampz + i + ZO)) : 1.f;
         const float mvx = __ldg(L1 + VX * P + co) - dbwd<R>(p1, ip, 1, a.k.cx) - dbwd<R>(p2, ip, PW, a.k.cz);
         const float mvz = __ldg(L1 + VZ * P + co) - dfwd<R>(p3, ip, PW, a.k.cz) - dfwd<R>(p2, ip, 1, a.k.cx);
-        const float bvx = damp * mvx, bvz = damp * mvz;
-        const float axx = damp * __ldg(L1 + TXX * P + co), azz = damp * __ldg(L1 + TZZ * P + co),
-                    axz = damp * __ldg(L1 + TXZ * P + co);
+        const float bvx = __fmul_rn(damp, mvx), bvz = __fmul_rn(damp, mvz);
+        const float axx = __fmul_rn(damp, __ldg(L1 + TXX * P + co)), azz = __fmul_rn(damp, __ldg(L1 + TZZ * P + co)),
+                    axz = __fmul_rn(damp, __ldg(L1 + TXZ * P + co));
         L0[VX * P + co] = bvx;
         L0[VZ * P + co] = bvz;
-        L0[TXX * P + co] = axx - dfwd<R>(q1, iq, 1, a.k.cx);
-        L0[TZZ * P + co] = azz - dbwd<R>(q2, iq, QW, a.k.cz);
-        L0[TXZ * P + co] = axz - dfwd<R>(q1, iq, QW, a.k.cz) - dbwd<R>(q2, iq, 1, a.k.cx);
+        L0[TXX * P + co] = __fsub_rn(axx, dfwd<R>(q1, iq, 1, a.k.cx));
+        L0[TZZ * P + co] = __fsub_rn(azz, dbwd<R>(q2, iq, QW, a.k.cz));
+        L0[TXZ * P + co] = __fsub_rn(__fsub_rn(axz, dfwd<R>(q1, iq, QW, a.k.cz)), dbwd<R>(q2, iq, 1, a.k.cx));
         if (!dom) continue;
         const long long pz = g.pitch;
         // velocity differences of S_{t+1}, stress differences of S_t; ld(f)
@@ -2081,9 +2108,8 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
         }
         if (si == i) dxm_tx = fmaf(coef_bwd<R>(sj - j, a.k.cx), a.src.z, dxm_tx);  // S_t + source
         if (sj == j) dzp_tz = fmaf(coef_fwd<R>(si - i, a.k.cz), a.src.w, dzp_tz);
-        G[0 * P + co] += dt * (axx + azz) * (dxp_vx + dzm_vz);
-        G[1 * P + co] += dt * (2.f * axx * dxp_vx + 2.f * azz * dzm_vz + axz * (dxm_vz + dzp_vx));
-        G[2 * P + co] += dt * (bvx * (dxm_tx + dzm_txz) + bvz * (dzp_tz + dxp_txz));
+        exact_stress_terms(dt, axx, azz, axz, dxp_vx, dzm_vz, dxm_vz + dzp_vx, G[0 * P + co], G[1 * P + co]);
+        exact_velocity_terms(dt, bvx, bvz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, G[2 * P + co]);
     }
 }
 

@@ -457,7 +457,7 @@ __device__ __forceinline__ void qprefetch4(const float *q) { asm volatile("prefe
 __device__ __forceinline__ float4 mk4(const float (&v)[4]) { return make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ float4 times4(const float4 &u, const float4 &v)
 {
-    return make_float4(u.x * v.x, u.y * v.y, u.z * v.z, u.w * v.w);
+    return make_float4(__fmul_rn(u.x, v.x), __fmul_rn(u.y, v.y), __fmul_rn(u.z, v.z), __fmul_rn(u.w, v.w));
 }
 
 // Receivers k0 .. k0 + n - 1 of line l on rows [r0, r1), columns [c0, c1).
@@ -521,7 +521,7 @@ __device__ __forceinline__ void res_block(const ResTile &t, int e, int &bz, int 
 // forward steps t0 .. t1 - 1 (fwd_step's arithmetic)
 // ---------------------------------------------------------------------------
 // QD: 1 stores the difference sets of the states, 2 the states, 3 the exact
-// adjoint's sets (stress differences of S_t with step t's source, velocity
+// adjoint's sets (stress differences of S_t and its step's source, velocity
 // differences of S_{t+1}; zero outside the update domain), 0 neither.
 template <int R, int RB, int QD>
 __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_constant__ FwdResArgs p)
@@ -933,9 +933,10 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         }
         if (stop) break;
         for (int e = rank; e < nring; e += NT) ring(e);
-        if constexpr (QD == 1) {
-            // the stress differences near the source cell again, without this
-            // step's source (see fwd_step)
+        if constexpr (SETS) {
+            // the stress differences near the source cell again: without this
+            // step's source (see fwd_step), or (QD 3) with its part added to the
+            // difference, as exact_adj_step does
             if (qi && add) {
                 __syncthreads();
                 if (tid < 4 * R) {
@@ -948,8 +949,13 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                         auto lxz = [&](long long m) { return s_txz[m]; };
                         const long long c = (gi - i0 + 2 * R) * W + gj - j0 + HX;
                         const long long o = cell_off(g, gi, gj);
-                        qi[Q_TXS * P + o] = lbwd<R>(lxx, c, 1, a.k.cx) + lbwd<R>(lxz, c, W, a.k.cz);
-                        qi[Q_TZS * P + o] = lfwd<R>(lzz, c, W, a.k.cz) + lfwd<R>(lxz, c, 1, a.k.cx);
+                        float dx = lbwd<R>(lxx, c, 1, a.k.cx), dz = lfwd<R>(lzz, c, W, a.k.cz);
+                        if (QD == 3 && gi == si) dx = fmaf(coef_bwd<R>(sj - gj, a.k.cx), src.z, dx);
+                        if (QD == 3 && gj == sj) dz = fmaf(coef_fwd<R>(si - gi, a.k.cz), src.w, dz);
+                        if (QD == 1 || in_domain(g, R, gi, gj)) {
+                            qi[Q_TXS * P + o] = dx + lbwd<R>(lxz, c, W, a.k.cz);
+                            qi[Q_TZS * P + o] = dz + lfwd<R>(lxz, c, 1, a.k.cx);
+                        }
                     }
                 }
             }
@@ -1701,7 +1707,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
     auto damp4_of = [&](int r, int c) {
         const float4 dx = ld4s(s_dx + c);
         const float dz = s_dz[r];
-        return make_float4(1.f - dt * (dx.x + dz), 1.f - dt * (dx.y + dz), 1.f - dt * (dx.z + dz), 1.f - dt * (dx.w + dz));
+        return make_float4(exact_damp(dt, dx.x, dz), exact_damp(dt, dx.y, dz), exact_damp(dt, dx.z, dz), exact_damp(dt, dx.w, dz));
     };
     // P1 .. P3 of four cells
     auto products = [&](const float4 &l, const float4 &m, const float4 &d, const float4 &xx, const float4 &zz, const float4 &xz,
@@ -1709,11 +1715,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
         float v1[4], v2[4], v3[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float axx = f4(d, k) * f4(xx, k), azz = f4(d, k) * f4(zz, k), axz = f4(d, k) * f4(xz, k);
-            const float lam = f4(l, k), l2m = lam + 2.f * f4(m, k);
-            v1[k] = dt * (l2m * axx + lam * azz);
-            v2[k] = dt * (f4(m, k) * axz);
-            v3[k] = dt * (lam * axx + l2m * azz);
+            exact_products(dt, f4(l, k), f4(m, k), __fmul_rn(f4(d, k), f4(xx, k)), __fmul_rn(f4(d, k), f4(zz, k)),
+                           __fmul_rn(f4(d, k), f4(xz, k)), v1[k], v2[k], v3[k]);
         }
         p1 = mk4(v1);
         p2 = mk4(v2);
@@ -1854,11 +1857,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
             xrow<R, true>(x, ld4s(s_p2 + ot + r * W), s_p2 + ot + r * W);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                n[k] = f4(d, k) * (f4(vz[r], k) - z.at(k, a.k.cz) - xfwd<R>(x, k, a.k.cx));
-                m[k] = f4(d, k) * f4(vx[r], k);
-                u[k] = dt * (f4(b[r], k) * m[k]);
-                w[k] = dt * (f4(b[r], k) * n[k]);
-                gg[k] = f4(gb[r], k) + dt * (m[k] * f4(qx[r], k) + n[k] * f4(qz[r], k));
+                n[k] = __fmul_rn(f4(d, k), f4(vz[r], k) - z.at(k, a.k.cz) - xfwd<R>(x, k, a.k.cx));
+                m[k] = __fmul_rn(f4(d, k), f4(vx[r], k));
+                u[k] = exact_q(dt, f4(b[r], k), m[k]);
+                w[k] = exact_q(dt, f4(b[r], k), n[k]);
+                gg[k] = f4(gb[r], k);
+                exact_velocity_terms(dt, m[k], n[k], f4(qx[r], k), f4(qz[r], k), gg[k]);
             }
             vx[r] = mk4(m);
             vz[r] = mk4(n);
@@ -1882,14 +1886,14 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
         const ZWindow<R, 1, false> z2([&](int) { return ld4s(s_p2 + c); }, s_p2 + c);
         xrow<R, false>(x, ld4s(s_p1 + c), s_p1 + c);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) nx[k] = f4(d, k) * (f4(ovx, k) - xbwd<R>(x, k, a.k.cx) - z2.at(0, k, a.k.cz));
+        for (int k = 0; k < 4; ++k) nx[k] = __fmul_rn(f4(d, k), f4(ovx, k) - xbwd<R>(x, k, a.k.cx) - z2.at(0, k, a.k.cz));
         const ZWindow<R, 1, true> z3([&](int) { return ld4s(s_p3 + c); }, s_p3 + c);
         xrow<R, true>(x, ld4s(s_p2 + c), s_p2 + c);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            nz[k] = f4(d, k) * (f4(ovz, k) - z3.at(0, k, a.k.cz) - xfwd<R>(x, k, a.k.cx));
-            u[k] = dt * (f4(bb, k) * nx[k]);
-            v[k] = dt * (f4(bb, k) * nz[k]);
+            nz[k] = __fmul_rn(f4(d, k), f4(ovz, k) - z3.at(0, k, a.k.cz) - xfwd<R>(x, k, a.k.cx));
+            u[k] = exact_q(dt, f4(bb, k), nx[k]);
+            v[k] = exact_q(dt, f4(bb, k), nz[k]);
         }
         st4s(s, mk4(nx));
         st4s(s + 4, mk4(nz));
@@ -1921,18 +1925,19 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
                 xrow<R, false>(x, z.centre(), s_q2 + ot + r * W);  // Dx- Q2
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    ax[k] = f4(d, k) * f4(xx[r], k);
-                    const float az = f4(d, k) * f4(zz[r], k), axz = f4(d, k) * f4(xz[r], k);
-                    gl[k] = f4(glam[r], k) + dt * (ax[k] + az) * (f4(q0v[r], k) + f4(q1v[r], k));
-                    gm[k] = f4(gmu[r], k) + dt * (2.f * ax[k] * f4(q0v[r], k) + 2.f * az * f4(q1v[r], k) + axz * f4(q2v[r], k));
-                    oz[k] = az - z.at(k, a.k.cz);
+                    ax[k] = __fmul_rn(f4(d, k), f4(xx[r], k));
+                    const float az = __fmul_rn(f4(d, k), f4(zz[r], k)), axz = __fmul_rn(f4(d, k), f4(xz[r], k));
+                    gl[k] = f4(glam[r], k);
+                    gm[k] = f4(gmu[r], k);
+                    exact_stress_terms(dt, ax[k], az, axz, f4(q0v[r], k), f4(q1v[r], k), f4(q2v[r], k), gl[k], gm[k]);
+                    oz[k] = __fsub_rn(az, z.at(k, a.k.cz));
                     oxz[k] = xbwd<R>(x, k, a.k.cx);  // taken off after Dz+ Q1
                 }
                 xx[r] = mk4(ax);
                 zz[r] = mk4(oz);
                 glam[r] = mk4(gl);
                 gmu[r] = mk4(gm);
-                xz[r] = make_float4(d.x * xz[r].x, d.y * xz[r].y, d.z * xz[r].z, d.w * xz[r].w);
+                xz[r] = times4(d, xz[r]);
                 q2v[r] = mk4(oxz);
             }
         }
@@ -1945,8 +1950,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
             xrow<R, true>(x, z.centre(), s_q1 + ot + r * W);  // Dx+ Q1
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                ox[k] = f4(xx[r], k) - xfwd<R>(x, k, a.k.cx);
-                oxz[k] = f4(xz[r], k) - z.at(k, a.k.cz) - f4(q2v[r], k);
+                ox[k] = __fsub_rn(f4(xx[r], k), xfwd<R>(x, k, a.k.cx));
+                oxz[k] = __fsub_rn(__fsub_rn(f4(xz[r], k), z.at(k, a.k.cz)), f4(q2v[r], k));
             }
             xx[r] = mk4(ox);
             xz[r] = mk4(oxz);
