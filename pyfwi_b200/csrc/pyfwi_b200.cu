@@ -1016,6 +1016,23 @@ int resident_reverse(pyfwi_plan *p, void *ws, int n, int t_hi, int t_lo, const B
     return PYFWI_OK;
 }
 
+// Steps whose sets are formed at a time, 0: not worth it.  The more, the smaller a part the launches' own cost is:
+// 10 shots of 240 x 440 cells, reconstructed states: 48 us per step with 11, 60 with 5.  What a chunk
+// takes beside the states kept (its sets, and in reverse mode its reconstructed states and one more) is at most a
+// quarter of them, up to a half while that is below 256 MB, or 64 MB, which no plan misses.
+int sets_chunk(const pyfwi_plan *p)
+{
+    constexpr size_t MB = 1ull << 20;
+    constexpr int LEAST = 4;
+    const bool reverse = p->opt.checkpoint != PYFWI_CKPT_EXACT;
+    const size_t step = (size_t)p->state * sizeof(float) * p->G,
+                 kept = step * (reverse ? p->chp.size() * p->geom.ns / p->G : (size_t)p->seg);
+    const size_t steps = std::max({kept / 4, std::min(kept / 2, 256 * MB), 64 * MB}) / step;
+    // every step of a segment is kept: few only where segments are short
+    const size_t n = reverse ? (steps ? (steps - 1) / 2 : 0) : std::max<size_t>(LEAST, steps);
+    return n < LEAST ? 0 : (int)std::min<size_t>(SETS_STEPS, n);
+}
+
 // The same with the sets formed from the states, a chunk of steps at a time;
 // state(t, lo): where S_{t+1} is, called for each step of a chunk (whose last
 // is lo) in backward order before any of the chunk's sets are formed.
@@ -1911,14 +1928,11 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     p->resident = opt->persist == 2 && (p->qd == 1 || from_states) && !p->overlap && src_in &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, RES_FORWARD, &tl) &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
-    if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
     if (p->resident && !p->qd && !p->exact_adj) {
-        // long enough that the launches' own cost is a small part, in a quarter of the memory of the states kept
-        // or, up to half of it, 256 MB
-        const size_t kept = opt->checkpoint == PYFWI_CKPT_EXACT ? (size_t)p->seg : p->chp.size() * G.ns / p->G;
-        const size_t room = (256ull << 20) / ((size_t)p->state * sizeof(float) * p->G);
-        p->rchunk = (int)std::min<size_t>(SETS_STEPS, std::max<size_t>({4, kept / 4, std::min(kept / 2, room)}));
+        p->rchunk = sets_chunk(p);
+        p->resident = p->rchunk > 0;
     }
+    if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
 
     const size_t pf = (size_t)p->g.plane * sizeof(float), sb = (size_t)p->state * sizeof(float);
     // regions holding planes start on a row of the workspace (a multiple of

@@ -1,0 +1,63 @@
+"""What plans with resident time loops reserve and refuse, decided on the host
+when a plan is created: no GPU needed."""
+import ctypes
+
+import numpy as np
+import pytest
+
+RESIDENT = 8  # pyfwi_plan_flags
+
+
+@pytest.fixture(scope="module")
+def native():
+    from pyfwi_b200 import build
+    build.build()
+    from pyfwi_b200 import _native
+    return _native
+
+
+def _plan(native, nz, nx, ns, nt, persist=2, half=2, npml=20, kept=None, **options):
+    """(workspace bytes, resident) of a plan; kept: reverse checkpoints, so many."""
+    g = native.Geometry()
+    g.nz, g.nx, g.npml, g.half_order = nz, nx, npml, half
+    g.nt, g.nt_ext, g.dt_scale = nt, nt, 1
+    g.dt, g.dh = 0.0004, 2.0
+    for q, c in enumerate((1.125, -0.041667, 0.0, 0.0)):
+        g.c[q] = c
+    g.ns, g.nr, g.n_lines = ns, nx, 1
+    g.lines[0] = native.RecLine(npml + 2, npml, 0, 1, nx, 0, 0)
+    g.mask_row0, g.mask_row1, g.mask_col0, g.mask_col1 = 0, nz, 0, nx
+    o = native.Options()
+    o.persist = persist
+    for k, v in options.items():
+        setattr(o, k, v)
+    if kept:
+        chp = np.ascontiguousarray(np.round(np.linspace(nt / kept - 1, nt - 1, kept)), np.int32)
+        o.checkpoint, o.nchp, o.chp = native.CKPT_REVERSE, kept, chp.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
+    src = np.full(ns, npml + 3, np.int32).ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
+    L, h, size, flags = native.lib(), ctypes.c_void_p(), ctypes.c_size_t(), ctypes.c_int32()
+    assert L.pyfwi_plan_create(ctypes.byref(g), src, src, ctypes.byref(o), ctypes.byref(h)) == 0, L.pyfwi_last_error()
+    L.pyfwi_workspace_size(h, ctypes.byref(size))
+    L.pyfwi_plan_flags(h, ctypes.byref(flags))
+    L.pyfwi_plan_destroy(h)
+    return size.value, bool(flags.value & RESIDENT)
+
+
+def _store(native, *a, kept, **kw):
+    """(bytes of one kept step of all shots, bytes the resident loops add to a reverse plan)."""
+    steps, _ = _plan(native, *a, persist=0, kept=kept, **kw)
+    fewer, _ = _plan(native, *a, persist=0, kept=kept - 1, **kw)
+    return steps - fewer, _plan(native, *a, kept=kept, **kw)[0] - steps
+
+
+EXCHANGE = 8 << 20  # the loops' exchange buffer and alignment
+
+
+@pytest.mark.parametrize("nz,nx,ns,nt,kept", [(150, 250, 5, 500, 50), (150, 250, 5, 500, 5), (500, 1000, 1, 400, 40),
+                                              (500, 1000, 4, 400, 40), (500, 1000, 16, 300, 6), (100, 100, 64, 300, 30),
+                                              (33, 45, 1, 200, 4)])
+def test_reverse_checkpoints_stay_a_low_memory_scheme(native, nz, nx, ns, nt, kept):
+    """The sets and reconstructed states of a chunk take at most half of what
+    the checkpoints take, or 64 MB."""
+    step, extra = _store(native, nz, nx, ns, nt, kept=kept)
+    assert extra <= max(kept * step // 2, 64 << 20) + EXCHANGE + (1 << 20)
