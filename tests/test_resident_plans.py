@@ -61,3 +61,18 @@ def test_reverse_checkpoints_stay_a_low_memory_scheme(native, nz, nx, ns, nt, ke
     the checkpoints take, or 64 MB."""
     step, extra = _store(native, nz, nx, ns, nt, kept=kept)
     assert extra <= max(kept * step // 2, 64 << 20) + EXCHANGE + (1 << 20)
+
+
+@pytest.mark.parametrize("ns", [1, 700, 1024, 4096, 20000, 65535])
+def test_a_chunk_of_every_shot_is_one_launch(native, ns):
+    """Shots x steps of a chunk are a grid's z extent: at most 65,535.  Plans
+    that would need more keep the step kernels."""
+    nt, kept = 600, 300
+    step, extra = _store(native, 5, 5, ns, nt, npml=4, kept=kept)
+    _, resident = _plan(native, 5, 5, ns, nt, npml=4, kept=kept)
+    chunk = (extra - EXCHANGE) / step  # sets, reconstructed states and one more
+    assert resident == (ns <= 65535 // 4)
+    if resident:
+        assert 4 <= round((chunk - 1) / 2) <= 65535 // ns
+    else:
+        assert extra == 0
