@@ -286,6 +286,10 @@ int pyfwi_launch_count(const pyfwi_plan *plan, int64_t *count);
  * (options.persist 2).  No reference counterpart. */
 int pyfwi_plan_flags(const pyfwi_plan *plan, int32_t *flags);
 
+/* Byte offset of the device error word (int32) in a workspace, for callers that
+ * copy it to the host themselves without a synchronisation. */
+#define PYFWI_ERROR_WORD 128
+
 /* Read and clear the workspace's device error word after the work queued on
  * `stream` (synchronises that stream).  *code: 0 none, 1 a streaming kernel
  * gave up waiting (one second) for a row copy and left its rows unwritten,

@@ -32,6 +32,7 @@ class Geometry(ctypes.Structure):
 
 ABI_VERSION = 8  # PYFWI_ABI_VERSION of include/pyfwi_b200.h
 REDUCE_SLOTS = 2368  # PYFWI_REDUCE_SLOTS
+ERROR_WORD = 128  # PYFWI_ERROR_WORD
 
 
 class Options(ctypes.Structure):

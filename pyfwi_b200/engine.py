@@ -57,6 +57,11 @@ class Plan:
         self.ws = ctypes.c_void_p((base + 255) // 256 * 256)
         self.nz, self.nx, self.npml = geom.nz, geom.nx, geom.npml
         self.ns, self.nr, self.nt_ext = geom.ns, geom.nr, geom.nt_ext
+        self._watched = self._report = None
+        if self.resident:
+            word = self.ws.value - base + N.ERROR_WORD
+            self._error = self._ws[word:word + 4].view(torch.int32)
+            self._report = torch.empty(1, dtype=torch.int32, pin_memory=True)
 
     def __del__(self):
         h = getattr(self, "handle", None)
@@ -124,6 +129,7 @@ class Plan:
         """pyfwi_misfit_gradient: observed / adjoint are lists of 5 device
         tensors [nt_ext, ns*nr] or None.  Returns (grad [3, nz, nx], misfit
         0-d float64 tensor, traces [5, nt_ext, ns*nr])."""
+        self._raise_if_gave_up()
         sv = np.ascontiguousarray(src_vals, np.float32).reshape(-1, 4)
         if traces is None:
             traces = torch.empty((5, self.nt_ext, self.ns * self.nr), dtype=torch.float32, device=self.device)
@@ -152,6 +158,7 @@ class Plan:
                                                int(param), _ptr(traces), _ptr(grad), _ptr(misfit),
                                                _stream(self.device)))
         self._keep = (observed, adjoint)
+        self._watch_device()
         if graph:
             for a, b in zip(adjoint, adj_in):
                 if a is not None:
@@ -159,10 +166,31 @@ class Plan:
             return grad.clone(), misfit.clone(), traces
         return grad, misfit, traces
 
+    # A resident loop may give up a wait as well, but calls on tensors must not
+    # synchronise to find out: the error word is copied to the host behind a
+    # call, and a later call that finds the copy done raises and clears the word.
+    def _watch_device(self):
+        """Have the error word of the call just queued looked at."""
+        if self._report is None or self._watched is not None or torch.cuda.is_current_stream_capturing():
+            return
+        self._report.copy_(self._error, non_blocking=True)
+        self._watched = torch.cuda.Event()
+        self._watched.record(torch.cuda.current_stream(self.device))
+
+    def _raise_if_gave_up(self):
+        """Raise NativeError if a resident loop of an earlier call gave up."""
+        if self._watched is None or torch.cuda.is_current_stream_capturing() or not self._watched.query():
+            return
+        self._watched = None
+        if int(self._report):
+            self.check_device()
+
     def check_device(self):
         """Synchronise the device stream and raise NativeError if a streaming
-        kernel gave up waiting for a row copy, or a persistent kernel at a
-        grid barrier, since the last check."""
+        kernel gave up waiting for a row copy, a persistent kernel at a grid
+        barrier or a resident loop for a neighbour's halo, since the last
+        check."""
+        self._watched = None
         code = ctypes.c_int32()
         N.check(self.lib.pyfwi_device_error(self.handle, self.ws, self.ws_bytes, ctypes.byref(code),
                                             _stream(self.device)))
@@ -212,6 +240,7 @@ class Plan:
         return n.value, ms.value, cells.value
 
     def set_model(self, vp, vs, rho, damp_x, damp_z):
+        self._raise_if_gave_up()
         args = [t.to(self.device, torch.float32).contiguous() for t in (vp, vs, rho, damp_x, damp_z)]
         N.check(self.lib.pyfwi_set_model(self.handle, self.ws, self.ws_bytes, *[_ptr(t) for t in args],
                                          _stream(self.device)))
@@ -219,12 +248,14 @@ class Plan:
 
     def forward(self, src_vals, traces=None):
         """Run all shots; returns traces [5, nt_ext, ns*nr] (float32, device)."""
+        self._raise_if_gave_up()
         sv = np.ascontiguousarray(src_vals, np.float32).reshape(-1, 4)
         if traces is None:
             traces = torch.empty((5, self.nt_ext, self.ns * self.nr), dtype=torch.float32, device=self.device)
         N.check(self.lib.pyfwi_forward(self.handle, self.ws, self.ws_bytes,
                                        sv.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), int(sv.shape[0]),
                                        _ptr(traces), _stream(self.device)))
+        self._watch_device()
         return traces
 
     def gradient(self, residual, param, grad=None, raw=None):
@@ -234,6 +265,7 @@ class Plan:
         With graph replay on, the residual is copied into buffers the plan
         keeps, so every call presents the same pointers to the captured
         graph."""
+        self._raise_if_gave_up()
         res = []
         for q, r in enumerate(residual):
             if r is None:
@@ -260,6 +292,7 @@ class Plan:
         N.check(self.lib.pyfwi_gradient(self.handle, self.ws, self.ws_bytes, arr, int(param), _ptr(grad), _ptr(raw),
                                         _stream(self.device)))
         self._res_keep = res
+        self._watch_device()
         return grad.clone() if self.opts.graph else grad
 
 

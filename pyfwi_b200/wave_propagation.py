@@ -549,7 +549,8 @@ class WavePropagator(WavePreparation):
         """Raise if a streaming or persistent kernel stopped early.  Reading
         the error word synchronises, so it is done where the call synchronises
         anyway (host results) or where such a kernel may have run, never
-        inside a CUDA-graph capture."""
+        inside a CUDA-graph capture.  A resident loop of a call on tensors that
+        stopped early leaves NaN; a later call on the plan raises."""
         if torch.cuda.is_current_stream_capturing():
             return
         o = self.plan.opts
