@@ -1019,7 +1019,7 @@ int resident_reverse(pyfwi_plan *p, void *ws, int n, int t_hi, int t_lo, const B
 // Steps whose sets are formed at a time, 0: not worth it.  The more, the smaller a part the launches' own cost is:
 // 10 shots of 240 x 440 cells, reconstructed states: 48 us per step with 11, 60 with 5.  What a chunk
 // takes beside the states kept (its sets, and in reverse mode its reconstructed states and one more) is at most a
-// quarter of them, up to a half while that is below 256 MB, or 64 MB, which no plan misses.
+// quarter of them, up to a half while that is below 256 MB, or 96 MB, which no plan misses.
 // Without energy terms a launch has shots times steps in blockIdx.z.
 int sets_chunk(const pyfwi_plan *p)
 {
@@ -1028,7 +1028,7 @@ int sets_chunk(const pyfwi_plan *p)
     const bool reverse = p->opt.checkpoint != PYFWI_CKPT_EXACT;
     const size_t step = (size_t)p->state * sizeof(float) * p->G,
                  kept = step * (reverse ? p->chp.size() * p->geom.ns / p->G : (size_t)p->seg);
-    const size_t steps = std::max({kept / 4, std::min(kept / 2, 256 * MB), 64 * MB}) / step;
+    const size_t steps = std::max({kept / 4, std::min(kept / 2, 256 * MB), 96 * MB}) / step;
     // every step of a segment is kept: few only where segments are short
     const size_t n = reverse ? (steps ? (steps - 1) / 2 : 0) : std::max<size_t>(LEAST, steps);
     const size_t most = p->nacc == 6 ? SETS_STEPS : std::min<size_t>(SETS_STEPS, 65535 / p->G);

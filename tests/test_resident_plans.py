@@ -58,9 +58,9 @@ EXCHANGE = 8 << 20  # the loops' exchange buffer and alignment
                                               (33, 45, 1, 200, 4)])
 def test_reverse_checkpoints_stay_a_low_memory_scheme(native, nz, nx, ns, nt, kept):
     """The sets and reconstructed states of a chunk take at most half of what
-    the checkpoints take, or 64 MB."""
+    the checkpoints take, or 96 MB."""
     step, extra = _store(native, nz, nx, ns, nt, kept=kept)
-    assert extra <= max(kept * step // 2, 64 << 20) + EXCHANGE + (1 << 20)
+    assert extra <= max(kept * step // 2, 96 << 20) + EXCHANGE + (1 << 20)
 
 
 @pytest.mark.parametrize("ns", [1, 700, 1024, 4096, 20000, 65535])
