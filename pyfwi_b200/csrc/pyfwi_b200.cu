@@ -77,7 +77,7 @@ constexpr int FWD_TMA[] = {0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 0};
 constexpr int ADJ_PREFETCH[] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1};
 constexpr int N_TILES = 12;
 constexpr int FWD_PF = 4, ADJ_PF = 2;  // rows the streaming kernels fetch ahead
-constexpr size_t ERR_OFF = 128;         // byte offset of the device error word in the header
+constexpr size_t ERR_OFF = PYFWI_ERROR_WORD;  // byte offset of the device error word in the header
 constexpr size_t CHECK_OFF = 192;       // byte offset of the frame-check counter (uint64) in the header
 constexpr size_t BAR_OFF = 224;         // byte offset of the persistent kernels' grid barrier (2 x uint32)
 
@@ -2073,7 +2073,8 @@ int pyfwi_device_error(pyfwi_plan *p, void *ws, size_t bytes, int32_t *code, voi
     *code = v;
     if (v)
         return fail(PYFWI_E_TIMEOUT, "device error word %d: %s", v,
-                    v == 3 ? "a persistent kernel gave up at a grid barrier" : "a streaming kernel stopped early");
+                    v == 3 ? "a persistent kernel gave up at a grid barrier, or a resident one for a neighbour's halo"
+                           : "a streaming kernel stopped early");
     return PYFWI_OK;
 }
 
