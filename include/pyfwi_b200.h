@@ -144,7 +144,7 @@ typedef struct pyfwi_options {
                                segments hold difference sets in FP32 (store_diffs), or the sets
                                can be formed from FP32 states (energy terms, reverse checkpoints;
                                a chunk of sets more in the workspace), or for the exact adjoint
-                               with FP32 states; no overlap is on, every source lies in the update domain and the
+                               with FP32 states; no overlap is on, every source lies in the update domain, every receiver in the grid and the
                                grid fits on the SMs (up to about 600,000 cells); the step kernels
                                otherwise.  A caller's stream capture takes the resident loops too:
                                graph replays and direct calls of a plan may be mixed */

@@ -1966,19 +1966,6 @@ __device__ __forceinline__ void exact_velocity_terms(float dt, float bvx, float 
     gb = __fmaf_rn(dt, __fmaf_rn(bvx, sx, __fmul_rn(bvz, sz)), gb);
 }
 
-// Coefficient of f[j + o] in a backward / forward difference at j.
-template <int R>
-__device__ __forceinline__ float coef_bwd(int o, const float *c)
-{
-    return (o >= 0 && o < R) ? c[o] : ((o < 0 && o >= -R) ? -c[-o - 1] : 0.f);
-}
-
-template <int R>
-__device__ __forceinline__ float coef_fwd(int o, const float *c)
-{
-    return (o >= 1 && o <= R) ? c[o - 1] : ((o <= 0 && o > -R) ? -c[-o] : 0.f);
-}
-
 template <int R, int TZ>
 struct ExactShape {
     static constexpr int PW = TX + 4 * R, PH = TZ + 4 * R;  // P fields: tile +- 2R
@@ -2047,7 +2034,8 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
     __syncthreads();
 
     // the tile: L_t and the gradients
-    const int si = a.add_src ? a.srcz[shot] : -(1 << 30), sj = a.srcx[shot];
+    const int si = a.add_src ? a.srcz[shot] : -1, sj = a.srcx[shot];
+    const long long sc = cell_off(g, si, sj);
     for (int e = threadIdx.x; e < TZ * TX; e += NTHREADS) {
         const int r = e / TX, c = e - r * TX, i = i0 + r, j = j0 + c;
         if (i >= g.tnz || j >= g.tnx) continue;
@@ -2076,9 +2064,11 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
             zp_vx = lfwd<R>(ld(VX), co, pz, a.k.cz);
         };
         auto sdiffs = [&](auto ld, float &xm_tx, float &zm_txz, float &zp_tz, float &xp_txz) {
-            xm_tx = lbwd<R>(ld(TXX), co, 1, a.k.cx);
+            // of S_t with its step's source, added to the stress as the forward step adds it
+            auto with = [&](auto f, float v) { return [=](long long m) { return m == sc ? __fadd_rn(f(m), v) : f(m); }; };
+            xm_tx = si == i ? lbwd<R>(with(ld(TXX), a.src.z), co, 1, a.k.cx) : lbwd<R>(ld(TXX), co, 1, a.k.cx);
             zm_txz = lbwd<R>(ld(TXZ), co, pz, a.k.cz);
-            zp_tz = lfwd<R>(ld(TZZ), co, pz, a.k.cz);
+            zp_tz = sj == j && si >= 0 ? lfwd<R>(with(ld(TZZ), a.src.w), co, pz, a.k.cz) : lfwd<R>(ld(TZZ), co, pz, a.k.cz);
             xp_txz = lfwd<R>(ld(TXZ), co, 1, a.k.cx);
         };
         auto f32 = [&](const float *S) {
@@ -2106,8 +2096,6 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
             vdiffs(f32(S1), dxp_vx, dzm_vz, dxm_vz, dzp_vx);
             sdiffs(f32(S0), dxm_tx, dzm_txz, dzp_tz, dxp_txz);
         }
-        if (si == i) dxm_tx = fmaf(coef_bwd<R>(sj - j, a.k.cx), a.src.z, dxm_tx);  // S_t + source
-        if (sj == j) dzp_tz = fmaf(coef_fwd<R>(si - i, a.k.cz), a.src.w, dzp_tz);
         exact_stress_terms(dt, axx, azz, axz, dxp_vx, dzm_vz, dxm_vz + dzp_vx, G[0 * P + co], G[1 * P + co]);
         exact_velocity_terms(dt, bvx, bvz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, G[2 * P + co]);
     }

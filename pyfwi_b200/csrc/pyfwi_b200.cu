@@ -1918,16 +1918,21 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     p->qd = qd ? (opt->snapshot == PYFWI_SNAP_FP24 ? 2 : 1) : 0;
     // resident time loops: difference sets on one stream, tiles that fit on chip
     ResTiles tl;
-    bool src_in = true;  // every source inside the update domain
+    bool all_in = true;  // every source inside the update domain, every receiver inside the grid
     for (int s = 0; s < G.ns; ++s)
-        src_in = src_in && srcz[s] >= p->R && srcz[s] <= tnz - p->R && srcx[s] >= p->R && srcx[s] <= tnx - p->R;
+        all_in = all_in && srcz[s] >= p->R && srcz[s] <= tnz - p->R && srcx[s] >= p->R && srcx[s] <= tnx - p->R;
+    for (int l = 0; l < G.n_lines; ++l) {
+        const pyfwi_rec_line &L = G.lines[l];
+        const long long last = std::max(L.count - 1, 0);
+        all_in = all_in && L.row0 >= 0 && L.col0 >= 0 && L.row0 + last * L.drow < tnz && L.col0 + last * L.dcol < tnx;
+    }
     // (FP32, the reference adjoint, the plain tile kernels), or states that the
     // sets can be formed from: energy terms, reconstructed states
     // (or the exact adjoint, whose resident form keeps sets where its step kernels keep states)
     const bool from_states = !p->qd && (p->nacc == 6 || opt->checkpoint != PYFWI_CKPT_EXACT || p->exact_adj) &&
                              opt->snapshot == PYFWI_SNAP_FP32 && !p->persist && !p->st_w && !p->ftma &&
                              !p->ast_w && p->ans == 1 && !p->apf && G.npml + p->R >= 4;
-    p->resident = opt->persist == 2 && (p->qd == 1 || from_states) && !p->overlap && src_in &&
+    p->resident = opt->persist == 2 && (p->qd == 1 || from_states) && !p->overlap && all_in &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, RES_FORWARD, &tl) &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
     if (p->resident && !p->qd && !p->exact_adj) {

@@ -521,7 +521,7 @@ __device__ __forceinline__ void res_block(const ResTile &t, int e, int &bz, int 
 // forward steps t0 .. t1 - 1 (fwd_step's arithmetic)
 // ---------------------------------------------------------------------------
 // QD: 1 stores the difference sets of the states, 2 the states, 3 the exact
-// adjoint's sets (stress differences of S_t and its step's source, velocity
+// adjoint's sets (stress differences of S_t with step t's source, velocity
 // differences of S_{t+1}; zero outside the update domain), 0 neither.
 template <int R, int RB, int QD>
 __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_constant__ FwdResArgs p)
@@ -933,10 +933,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
         }
         if (stop) break;
         for (int e = rank; e < nring; e += NT) ring(e);
-        if constexpr (SETS) {
-            // the stress differences near the source cell again: without this
-            // step's source (see fwd_step), or (QD 3) with its part added to the
-            // difference, as exact_adj_step does
+        if constexpr (QD == 1) {
+            // the stress differences near the source cell again, without this
+            // step's source (see fwd_step)
             if (qi && add) {
                 __syncthreads();
                 if (tid < 4 * R) {
@@ -949,13 +948,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) fwd_resident(const __grid_cons
                         auto lxz = [&](long long m) { return s_txz[m]; };
                         const long long c = (gi - i0 + 2 * R) * W + gj - j0 + HX;
                         const long long o = cell_off(g, gi, gj);
-                        float dx = lbwd<R>(lxx, c, 1, a.k.cx), dz = lfwd<R>(lzz, c, W, a.k.cz);
-                        if (QD == 3 && gi == si) dx = fmaf(coef_bwd<R>(sj - gj, a.k.cx), src.z, dx);
-                        if (QD == 3 && gj == sj) dz = fmaf(coef_fwd<R>(si - gi, a.k.cz), src.w, dz);
-                        if (QD == 1 || in_domain(g, R, gi, gj)) {
-                            qi[Q_TXS * P + o] = dx + lbwd<R>(lxz, c, W, a.k.cz);
-                            qi[Q_TZS * P + o] = dz + lfwd<R>(lxz, c, 1, a.k.cx);
-                        }
+                        qi[Q_TXS * P + o] = lbwd<R>(lxx, c, 1, a.k.cx) + lbwd<R>(lxz, c, W, a.k.cz);
+                        qi[Q_TZS * P + o] = lfwd<R>(lzz, c, W, a.k.cz) + lfwd<R>(lxz, c, 1, a.k.cx);
                     }
                 }
             }
