@@ -146,8 +146,10 @@ typedef struct pyfwi_options {
                                a chunk of sets more in the workspace), or for the exact adjoint
                                with FP32 states; no overlap is on, every source lies in the update domain, every receiver in the grid and the
                                grid fits on the SMs (up to about 600,000 cells); the step kernels
-                               otherwise.  A caller's stream capture takes the resident loops too:
-                               graph replays and direct calls of a plan may be mixed */
+                               otherwise, and for a pass that they run faster (many shots of
+                               eighth order, many shots with states or checkpoints).  A caller's
+                               stream capture takes the resident loops too: graph replays and
+                               direct calls of a plan may be mixed */
     int32_t overlap;        /* 1: exact checkpoints in FP32 with recompute segments: recompute
                                segment m-1 on a second stream of the plan while the adjoint of
                                segment m runs (two segment buffers in the workspace) */

@@ -104,7 +104,8 @@ struct pyfwi_plan {
     int R, tz, st_w, ftma, atz, ast_w, ans, apf, chunk_opt, nacc, G, ngroups, seg, M, n_inj;  // a*: adjoint step variant
     bool exact_adj = false;  // PYFWI_ADJOINT_EXACT
     bool persist = false;    // time loops as persistent kernels (options.persist, where the layout allows)
-    bool resident = false;   // time loops with the wavefield on chip (options.persist 2, where it fits)
+    bool resident = false;   // time loops with the wavefield on chip (options.persist 2, where it fits): one of
+    bool res_fwd = true, res_bwd = true;  // the forward pass and the backward one, or both
     int rchunk = 0;          // resident without sets in the store: steps whose sets are formed from their states at a time
     int sms = 0;             // SMs of the device the resident launches run on (0: not asked yet)
     unsigned tag = 1;        // next unused tag of the exchange buffer in this call
@@ -1131,7 +1132,7 @@ int exact_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStream
     Buf z = exact_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(z.base + q * z.stride, 0, p->state * sizeof(float), st));
     if (use_persist(p, st)) return persist_pass(p, ws, s0, n, traces, st);
-    if (use_resident(p)) return resident_pass(p, ws, s0, n, traces, st);
+    if (use_resident(p) && p->res_fwd) return resident_pass(p, ws, s0, n, traces, st);
     StepArgs a = base_step(p, ws);
     a.shot0 = s0;
     a.traces = traces;
@@ -1190,7 +1191,7 @@ int reverse_pass(pyfwi_plan *p, void *ws, int s0, int n, float *traces, cudaStre
     // states stored after the steps listed in chp (wave_propagation.py:710-727)
     Buf cur = work_state(p, ws, 0);
     for (int q = 0; q < n; ++q) CK(cudaMemsetAsync(cur.base + q * cur.stride, 0, p->state * sizeof(float), st));
-    if (use_resident(p)) return resident_reverse_pass(p, ws, s0, n, traces, st);
+    if (use_resident(p) && p->res_fwd) return resident_reverse_pass(p, ws, s0, n, traces, st);
     int wcur = 0;  // work buffer holding the current state (-1: a checkpoint slot)
     size_t kc = 0;
     StepArgs a = base_step(p, ws);
@@ -1549,7 +1550,7 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
         } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && p->overlap) {
             rc = overlap_backward(p, ws, a, s0, n, t_src, ping, adj, st);
             if (rc) return rc;
-        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && use_resident(p)) {
+        } else if (p->opt.checkpoint == PYFWI_CKPT_EXACT && use_resident(p) && p->res_bwd) {
             rc = clear_exchange(p, ws, st);
             if (rc) return rc;
             for (int m = p->M - 1; m >= 0; --m) {
@@ -1643,7 +1644,7 @@ int gradient_enqueue(pyfwi_plan *p, void *ws, const float *const *residual, int3
                 cur = rc ? Buf{nullptr, 0} : to;
                 return cur;
             };
-            if (use_resident(p)) {
+            if (use_resident(p) && p->res_bwd) {
                 rc = clear_exchange(p, ws, st);
                 if (rc) return rc;
                 const int ring = p->rchunk + 1;  // the newest state of a chunk is still read by the next one's first step
@@ -1935,9 +1936,13 @@ int pyfwi_plan_create(const pyfwi_geometry *geom, const int32_t *srcx, const int
     p->resident = opt->persist == 2 && (p->qd == 1 || from_states) && !p->overlap && all_in &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, RES_FORWARD, &tl) &&
                   resident_tiles(p->g, p->R, p->lines, p->G, RES_MAX_CTAS, p->exact_adj ? RES_EXACT : RES_ADJOINT, &tl);
-    if (p->resident && !p->qd && !p->exact_adj) {
-        p->rchunk = sets_chunk(p);
-        p->resident = p->rchunk > 0;
+    if (p->resident && !p->exact_adj) {  // whose adjoint is about twice as fast on chip at any size
+        const ResStore store = p->qd ? RES_OF_SETS : opt->checkpoint == PYFWI_CKPT_EXACT ? RES_OF_STATES : RES_OF_CHECKPOINTS;
+        const int chunk = p->qd ? 0 : sets_chunk(p);
+        resident_pays(p->g, p->R, p->lines, G.ns, p->tz, store, chunk, p->nacc == 6, &p->res_fwd, &p->res_bwd);
+        if (store != RES_OF_SETS) p->res_bwd = p->res_bwd && chunk > 0;
+        p->rchunk = p->res_bwd ? chunk : 0;
+        p->resident = p->res_fwd || p->res_bwd;
     }
     if (p->resident) p->opt.graph = 0;  // a few launches per call: nothing to replay
 

@@ -45,7 +45,7 @@ static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_
 // shots of 240 x 440 take 12.6 / 16.0 us with 1 row and two shots at a time,
 // 13.6 / 17.1 with 2 rows and two, 10.8 / 17.0 with 3 rows and four; 8 of 140 x
 // 140 in one launch 3.15 / 3.36 with 1 row, 4.31 / 7.47 with 3.
-bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms, ResLoop loop, ResTiles *out)
+bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms, ResLoop loop, ResTiles *out, double *us)
 {
     struct Cost {
         double step, row, warp_row, ring, row3;  // fixed; per row; per warp of blocks and row; per warp of ring items; with 3 rows
@@ -76,7 +76,43 @@ bool resident_tiles(const Grid &g, int R, const Lines &lines, int shots, int sms
             }
         }
     }
+    if (us) *us = best;
     return best > 0;
+}
+
+// With many shots in a launch the step kernels run at the memory's rate, while a
+// resident launch holds so few shots that its latency does not shrink with their
+// number.  So the time of a step (us) is modelled for both: the resident loops' as
+// resident_tiles does, the step kernels' as a fixed part and a rate in
+// ps per cell and shot of whole tiles, which measured (64 shots unless said, us per step, step kernels / on chip):
+//   sets, eighth order, forward and backward: 340 x 540 602 / 647, 300 x 500 475 / 587, 190 x 940 555 / 603; tiles
+//     of 8 rows 240 x 440 430 / 313, 280 x 440 505 / 515.  Fourth order is always faster on chip: 340 x 540
+//     436 / 313, 8 shots of 560 x 1060 181 / 121, and the model finds no grid where it would not be.
+//   states, forward: fourth order 520 x 560 216 / 250, 340 x 540 148 / 147, eighth 340 x 540 255 / 300; tiles of
+//     8 rows 240 x 440 102 / 82 and 206 / 152.  Backward with energy terms always on chip: 1204 / 594, 1655 / 569.
+//   checkpoints, backward, fourth order: 520 x 560 735 / 1053, 16 shots of it 211 / 267, of 240 x 440
+//     82 / 87, 4 of 560 x 1060 110 / 112, 1 of it 31 / 26, 10 of 240 x 440 53 / 48; eighth order 340 x 540
+//     1487 / 1016.
+void resident_pays(const Grid &g, int R, const Lines &lines, int shots, int rows, ResStore store, int chunk, bool energy,
+                   bool *fwd, bool *bwd)
+{
+    const bool eighth = R > 2, large = rows > 8;
+    const double cells = 1e-6 * g.tnz * g.tnx * shots,
+                 tiles = 1e-6 * ((g.tnx + 31) / 32 * 32) * ((g.tnz + rows - 1) / rows * rows) * shots;
+    ResTiles tl;
+    double f = 0, b = 0;
+    *fwd = resident_tiles(g, R, lines, shots, RES_MAX_CTAS, RES_FORWARD, &tl, &f);
+    *bwd = resident_tiles(g, R, lines, shots, RES_MAX_CTAS, RES_ADJOINT, &tl, &b);
+    if (store == RES_OF_SETS) {  // both passes or neither
+        if (eighth) *fwd = *bwd = *fwd && *bwd && f + b <= 8 + (large ? 46.5 : 62.5) * tiles;
+        return;
+    }
+    // a loop that writes every state takes 6 % more than one with sets, one that writes few 10 % less
+    *fwd = *fwd && f * (store == RES_OF_STATES ? 1.06 : 0.9) <= 4 + (eighth ? (large ? 20.8 : 30) : (large ? 11.6 : 14.8)) * tiles;
+    if (store == RES_OF_STATES || energy) return;
+    // reverse-time loop, forming the sets and the launches of a chunk, adjoint loop
+    *bwd = *bwd && chunk > 0 &&
+           f + b + (12 + 60.0 / chunk) * cells + 8.0 / chunk <= 9 + (eighth ? 120 : large ? 38 : 42) * tiles;
 }
 
 cudaError_t launch_fwd_resident(FwdResArgs &a, int R, cudaStream_t s)

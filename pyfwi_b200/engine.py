@@ -158,7 +158,6 @@ class Plan:
                                                int(param), _ptr(traces), _ptr(grad), _ptr(misfit),
                                                _stream(self.device)))
         self._keep = (observed, adjoint)
-        self._watch_device()
         if graph:
             for a, b in zip(adjoint, adj_in):
                 if a is not None:
@@ -169,8 +168,8 @@ class Plan:
     # A resident loop may give up a wait as well, but calls on tensors must not
     # synchronise to find out: the error word is copied to the host behind a
     # call, and a later call that finds the copy done raises and clears the word.
-    def _watch_device(self):
-        """Have the error word of the call just queued looked at."""
+    def watch_device(self):
+        """Have the error word of the calls queued so far looked at."""
         if self._report is None or self._watched is not None or torch.cuda.is_current_stream_capturing():
             return
         self._report.copy_(self._error, non_blocking=True)
@@ -255,7 +254,6 @@ class Plan:
         N.check(self.lib.pyfwi_forward(self.handle, self.ws, self.ws_bytes,
                                        sv.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), int(sv.shape[0]),
                                        _ptr(traces), _stream(self.device)))
-        self._watch_device()
         return traces
 
     def gradient(self, residual, param, grad=None, raw=None):
@@ -292,7 +290,6 @@ class Plan:
         N.check(self.lib.pyfwi_gradient(self.handle, self.ws, self.ws_bytes, arr, int(param), _ptr(grad), _ptr(raw),
                                         _stream(self.device)))
         self._res_keep = res
-        self._watch_device()
         return grad.clone() if self.opts.graph else grad
 
 

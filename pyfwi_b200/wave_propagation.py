@@ -556,6 +556,8 @@ class WavePropagator(WavePreparation):
         o = self.plan.opts
         if synchronous or 3 <= o.tile <= 5 or 4 <= o.adj_tile <= 6 or o.persist == 1:
             self.plan.check_device()
+        else:
+            self.plan.watch_device()
 
     def _section(self, traces):
         """acquisition.seismic_section on device traces [5][nt_ext][ns*nr]."""

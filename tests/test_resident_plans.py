@@ -71,8 +71,28 @@ def test_a_chunk_of_every_shot_is_one_launch(native, ns):
     step, extra = _store(native, 5, 5, ns, nt, npml=4, kept=kept)
     _, resident = _plan(native, 5, 5, ns, nt, npml=4, kept=kept)
     chunk = (extra - EXCHANGE) / step  # sets, reconstructed states and one more
-    assert resident == (ns <= 65535 // 4)
-    if resident:
+    if ns > 65535 // 4:
+        assert chunk < 1
+    elif resident and chunk > 1:
         assert 4 <= round((chunk - 1) / 2) <= 65535 // ns
-    else:
-        assert extra == 0
+
+
+# (half order, nz, nx, shots, steps kept, energy, tile variant): passes on chip, as measured
+FASTER = [(2, 300, 500, 64, 0, 0, 0, True), (2, 500, 1000, 16, 0, 0, 0, True), (2, 400, 700, 64, 0, 0, 0, True),
+          (4, 300, 500, 16, 0, 0, 1, True), (4, 260, 460, 48, 0, 0, 1, True), (4, 2000, 60, 64, 0, 0, 0, True),
+          (4, 300, 500, 64, 0, 0, 0, False), (4, 260, 460, 64, 0, 0, 0, False), (4, 150, 900, 64, 0, 0, 0, False),
+          (4, 240, 400, 64, 0, 0, 1, False)]
+
+
+@pytest.mark.parametrize("half,nz,nx,ns,kept,energy,tile,resident", FASTER)
+def test_sets_stay_on_chip_where_that_is_faster(native, half, nz, nx, ns, kept, energy, tile, resident):
+    assert _plan(native, nz, nx, ns, 40, half=half, tile=tile, energy=energy, store_diffs=1)[1] == resident
+
+
+@pytest.mark.parametrize("nz,nx,ns,tile,backward", [(100, 100, 4, 1, True), (200, 400, 1, 1, True), (500, 1000, 1, 1, True),
+                                                    (300, 500, 64, 0, False), (480, 520, 16, 1, False), (480, 520, 64, 0, False)])
+def test_reconstruction_stays_on_chip_where_that_is_faster(native, nz, nx, ns, tile, backward):
+    """A backward pass on chip reserves a chunk; the forward pass stays on chip either way."""
+    step, extra = _store(native, nz, nx, ns, 400, kept=40, tile=tile)
+    assert (extra > step + EXCHANGE) == backward
+    assert _plan(native, nz, nx, ns, 400, kept=40, tile=tile)[1]
