@@ -78,12 +78,13 @@ class Plan:
         return Plan.query(geom, opts)[0]
 
     @staticmethod
-    def query(geom, opts):
+    def query(geom, opts, srcx=None, srcz=None):
         """(workspace bytes, pyfwi_plan_flags) of a plan with these settings."""
         L = N.lib()
-        # sources in the middle of the model: some options apply only to sources in the update domain
-        srcx = np.full(geom.ns, geom.npml + geom.nx // 2, np.int32)
-        srcz = np.full(geom.ns, geom.npml + geom.nz // 2, np.int32)
+        # sources in the middle of the model where none are given: some options apply only to
+        # sources in the update domain
+        srcx = np.ascontiguousarray(np.full(geom.ns, geom.npml + geom.nx // 2) if srcx is None else srcx, np.int32)
+        srcz = np.ascontiguousarray(np.full(geom.ns, geom.npml + geom.nz // 2) if srcz is None else srcz, np.int32)
         h = ctypes.c_void_p()
         N.check(L.pyfwi_plan_create(ctypes.byref(geom), srcx.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
                                     srcz.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), ctypes.byref(opts),

@@ -478,7 +478,9 @@ class WavePreparation:
             # ((M - 1) * s) in a smaller store
             return -(-nt // (-(-nt // lo)))
 
-        resident = Plan.query(geom, opts(nt, 1))[1] & 8
+        # (with overlap a plan of several segments has the step kernels)
+        o = opts(nt, 1)
+        resident = not o.overlap and Plan.query(geom, o, self.srcx, self.srcz)[1] & 8
 
         def group_cost(s, b):
             m = -(-nt // s)

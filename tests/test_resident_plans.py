@@ -96,3 +96,28 @@ def test_reconstruction_stays_on_chip_where_that_is_faster(native, nz, nx, ns, t
     step, extra = _store(native, nz, nx, ns, 400, kept=40, tile=tile)
     assert (extra > step + EXCHANGE) == backward
     assert _plan(native, nz, nx, ns, 400, kept=40, tile=tile)[1]
+
+
+@pytest.mark.parametrize("why", ["overlap", "a source in the frame"])
+def test_layouts_of_plans_without_resident_loops(native, monkeypatch, why):
+    """A survey whose plan will have the step kernels gets their layout, also
+    when the resident loops were asked for."""
+    import torch
+    import cases
+    from helpers import product
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d=None: (60 << 30, 180 << 30))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda d=None: 0)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda d=None: 0)
+    W = product(cases.c3(), cuda_device="cpu")
+    if why != "overlap":
+        W.srcz = np.array(W.srcz)
+        W.srcz[0] = 1  # above the update domain
+
+    def layout(persist):
+        def opts(seg, batch):
+            o = native.Options()
+            o.segment, o.shot_batch, o.persist, o.store_diffs = int(seg), int(batch), persist, 1
+            o.overlap = int(why == "overlap")
+            return o
+        return W._auto_layout(W._geometry(), opts, 0, 0)
+    assert layout(2) == layout(0)
