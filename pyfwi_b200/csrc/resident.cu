@@ -101,10 +101,12 @@ void resident_pays(const Grid &g, int R, const Lines &lines, int shots, int rows
                  tiles = 1e-6 * ((g.tnx + 31) / 32 * 32) * ((g.tnz + rows - 1) / rows * rows) * shots;
     ResTiles tl;
     double f = 0, b = 0;
+    *fwd = *bwd = true;
+    if (store == RES_OF_SETS && !eighth) return;
     *fwd = resident_tiles(g, R, lines, shots, RES_MAX_CTAS, RES_FORWARD, &tl, &f);
     *bwd = resident_tiles(g, R, lines, shots, RES_MAX_CTAS, RES_ADJOINT, &tl, &b);
     if (store == RES_OF_SETS) {  // both passes or neither
-        if (eighth) *fwd = *bwd = *fwd && *bwd && f + b <= 8 + (large ? 46.5 : 62.5) * tiles;
+        *fwd = *bwd = *fwd && *bwd && f + b <= 8 + (large ? 46.5 : 62.5) * tiles;
         return;
     }
     // a loop that writes every state takes 6 % more than one with sets, one that writes few 10 % less
