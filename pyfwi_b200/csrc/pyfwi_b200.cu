@@ -1009,7 +1009,7 @@ int resident_reverse(pyfwi_plan *p, void *ws, int n, int t_hi, int t_lo, const B
         r.q = slot_of(out, c0).base;
         r.tag0 = p->tag;
         p->tag += (unsigned)(t_hi - t_lo) + 1;
-        ProfileScope prof(p, st, 0, tl.nslots * (t_hi - t_lo));
+        ProfileScope prof(p, st, 2, tl.nslots * (t_hi - t_lo));
         cudaError_t e = launch_rev_resident(r, p->R, st);
         if (e != cudaSuccess) return fail(PYFWI_E_CUDA, "resident reverse-time launch: %s", cudaGetErrorString(e));
         p->launches++;
