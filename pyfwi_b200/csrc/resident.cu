@@ -17,8 +17,6 @@ extern template cudaError_t launch_exact_resident_r<4>(AdjResArgs &a, cudaStream
 
 namespace {
 
-constexpr size_t MAX_FLOATS = (232448 - 1024) / sizeof(float);  // 227 KB per CTA less the static words
-
 template <int R>
 bool fits(int th, int nq, int rb, int ctas, const Lines &lines, ResLoop loop)
 {
@@ -27,11 +25,11 @@ bool fits(int th, int nq, int rb, int ctas, const Lines &lines, ResLoop loop)
     return th <= S::TH && nq <= S::NQ && (th / rb) * nq <= RES_THREADS && halo <= RES_HALO &&
            ctas * frame_count(th, nq, 2 * R, S::HG) <= RES_MAX_STRIPS && slots <= RES_MAX_SLOTS &&
            (loop == RES_FORWARD ||
-            (loop == RES_EXACT ? exact_res_floats<R>(rb) : adj_res_floats<R>(rb)) + RES_SLOT_FLOATS * (size_t)slots <= MAX_FLOATS);
+            (loop == RES_EXACT ? exact_res_floats<R>(rb) : adj_res_floats<R>(rb)) + RES_SLOT_FLOATS * (size_t)slots <= RES_MAX_FLOATS);
 }
 
-static_assert(FWD_RES_FLOATS<2, 3> <= MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= MAX_FLOATS && REV_RES_FLOATS<2, 3> <= MAX_FLOATS &&
-                  REV_RES_FLOATS<4, 3> <= MAX_FLOATS,
+static_assert(FWD_RES_FLOATS<2, 3> <= RES_MAX_FLOATS && FWD_RES_FLOATS<4, 3> <= RES_MAX_FLOATS && REV_RES_FLOATS<2, 3> <= RES_MAX_FLOATS &&
+                  REV_RES_FLOATS<4, 3> <= RES_MAX_FLOATS,
               "the forward and reverse-time loops fit on an SM");
 
 }  // namespace

@@ -5,11 +5,15 @@
 
 namespace pyfwi {
 
+constexpr size_t RES_MAX_FLOATS = (232448 - 1024) / sizeof(float);  // 227 KB per CTA less the static words
+
+// The limit that is set is the same for every launch: it belongs to the kernel, and plans
+// of other sizes may be launching the same one on other threads.
 template <class Args>
 static cudaError_t launch_resident(const void *kern, const Args &a, size_t floats, cudaStream_t s)
 {
     const size_t smem = floats * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_MAX_FLOATS * sizeof(float));
     if (e != cudaSuccess) return e;
     void *args[] = {const_cast<Args *>(&a)};
     return cudaLaunchCooperativeKernel(kern, dim3(a.tl.gz * a.tl.gx * a.tl.nslots), dim3(RES_THREADS), args, smem, s);

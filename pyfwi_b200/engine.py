@@ -57,11 +57,12 @@ class Plan:
         self.ws = ctypes.c_void_p((base + 255) // 256 * 256)
         self.nz, self.nx, self.npml = geom.nz, geom.nx, geom.npml
         self.ns, self.nr, self.nt_ext = geom.ns, geom.nr, geom.nt_ext
-        self._watched = self._report = None
+        self._watched, self._report = False, None
         if self.resident:
             word = self.ws.value - base + N.ERROR_WORD
             self._error = self._ws[word:word + 4].view(torch.int32)
             self._report = torch.empty(1, dtype=torch.int32, pin_memory=True)
+            self._reported = torch.cuda.Event()
 
     def __del__(self):
         h = getattr(self, "handle", None)
@@ -171,17 +172,17 @@ class Plan:
     # call, and a later call that finds the copy done raises and clears the word.
     def watch_device(self):
         """Have the error word of the calls queued so far looked at."""
-        if self._report is None or self._watched is not None or torch.cuda.is_current_stream_capturing():
+        if self._report is None or self._watched or torch.cuda.is_current_stream_capturing():
             return
         self._report.copy_(self._error, non_blocking=True)
-        self._watched = torch.cuda.Event()
-        self._watched.record(torch.cuda.current_stream(self.device))
+        self._reported.record(torch.cuda.current_stream(self.device))
+        self._watched = True
 
     def _raise_if_gave_up(self):
         """Raise NativeError if a resident loop of an earlier call gave up."""
-        if self._watched is None or torch.cuda.is_current_stream_capturing() or not self._watched.query():
+        if not self._watched or torch.cuda.is_current_stream_capturing() or not self._reported.query():
             return
-        self._watched = None
+        self._watched = False
         if int(self._report):
             self.check_device()
 
@@ -190,7 +191,7 @@ class Plan:
         kernel gave up waiting for a row copy, a persistent kernel at a grid
         barrier or a resident loop for a neighbour's halo, since the last
         check."""
-        self._watched = None
+        self._watched = False
         code = ctypes.c_int32()
         N.check(self.lib.pyfwi_device_error(self.handle, self.ws, self.ws_bytes, ctypes.byref(code),
                                             _stream(self.device)))
