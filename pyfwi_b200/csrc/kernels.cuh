@@ -1966,6 +1966,19 @@ __device__ __forceinline__ void exact_velocity_terms(float dt, float bvx, float 
     gb = __fmaf_rn(dt, __fmaf_rn(bvx, sx, __fmul_rn(bvz, sz)), gb);
 }
 
+// Coefficient of f[j + o] in a backward / forward difference at j.
+template <int R>
+__device__ __forceinline__ float coef_bwd(int o, const float *c)
+{
+    return (o >= 0 && o < R) ? c[o] : ((o < 0 && o >= -R) ? -c[-o - 1] : 0.f);
+}
+
+template <int R>
+__device__ __forceinline__ float coef_fwd(int o, const float *c)
+{
+    return (o >= 1 && o <= R) ? c[o - 1] : ((o <= 0 && o > -R) ? -c[-o] : 0.f);
+}
+
 template <int R, int TZ>
 struct ExactShape {
     static constexpr int PW = TX + 4 * R, PH = TZ + 4 * R;  // P fields: tile +- 2R
@@ -2034,8 +2047,9 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
     __syncthreads();
 
     // the tile: L_t and the gradients
-    const int si = a.add_src ? a.srcz[shot] : -1, sj = a.srcx[shot];
-    const long long sc = cell_off(g, si, sj);
+    const int si = a.add_src ? a.srcz[shot] : -(1 << 30), sj = a.srcx[shot];
+    // cells whose stress differences reach the source cell
+    auto near_src = [&](int i, int j) { return (i == si && abs(j - sj) <= R) || (j == sj && abs(i - si) <= R); };
     for (int e = threadIdx.x; e < TZ * TX; e += NTHREADS) {
         const int r = e / TX, c = e - r * TX, i = i0 + r, j = j0 + c;
         if (i >= g.tnz || j >= g.tnx) continue;
@@ -2046,13 +2060,13 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
         const float mvx = __ldg(L1 + VX * P + co) - dbwd<R>(p1, ip, 1, a.k.cx) - dbwd<R>(p2, ip, PW, a.k.cz);
         const float mvz = __ldg(L1 + VZ * P + co) - dfwd<R>(p3, ip, PW, a.k.cz) - dfwd<R>(p2, ip, 1, a.k.cx);
         const float bvx = __fmul_rn(damp, mvx), bvz = __fmul_rn(damp, mvz);
-        const float axx = __fmul_rn(damp, __ldg(L1 + TXX * P + co)), azz = __fmul_rn(damp, __ldg(L1 + TZZ * P + co)),
-                    axz = __fmul_rn(damp, __ldg(L1 + TXZ * P + co));
+        const float lxx = __ldg(L1 + TXX * P + co), lzz = __ldg(L1 + TZZ * P + co), lxz = __ldg(L1 + TXZ * P + co);
+        const float axx = __fmul_rn(damp, lxx), azz = __fmul_rn(damp, lzz), axz = __fmul_rn(damp, lxz);
         L0[VX * P + co] = bvx;
         L0[VZ * P + co] = bvz;
-        L0[TXX * P + co] = __fsub_rn(axx, dfwd<R>(q1, iq, 1, a.k.cx));
-        L0[TZZ * P + co] = __fsub_rn(azz, dbwd<R>(q2, iq, QW, a.k.cz));
-        L0[TXZ * P + co] = __fsub_rn(__fsub_rn(axz, dfwd<R>(q1, iq, QW, a.k.cz)), dbwd<R>(q2, iq, 1, a.k.cx));
+        L0[TXX * P + co] = __fmaf_rn(damp, lxx, -dfwd<R>(q1, iq, 1, a.k.cx));
+        L0[TZZ * P + co] = __fmaf_rn(damp, lzz, -dbwd<R>(q2, iq, QW, a.k.cz));
+        L0[TXZ * P + co] = __fsub_rn(__fmaf_rn(damp, lxz, -dfwd<R>(q1, iq, QW, a.k.cz)), dbwd<R>(q2, iq, 1, a.k.cx));
         if (!dom) continue;
         const long long pz = g.pitch;
         // velocity differences of S_{t+1}, stress differences of S_t; ld(f)
@@ -2064,11 +2078,9 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
             zp_vx = lfwd<R>(ld(VX), co, pz, a.k.cz);
         };
         auto sdiffs = [&](auto ld, float &xm_tx, float &zm_txz, float &zp_tz, float &xp_txz) {
-            // of S_t with its step's source, added to the stress as the forward step adds it
-            auto with = [&](auto f, float v) { return [=](long long m) { return m == sc ? __fadd_rn(f(m), v) : f(m); }; };
-            xm_tx = si == i ? lbwd<R>(with(ld(TXX), a.src.z), co, 1, a.k.cx) : lbwd<R>(ld(TXX), co, 1, a.k.cx);
+            xm_tx = lbwd<R>(ld(TXX), co, 1, a.k.cx);
             zm_txz = lbwd<R>(ld(TXZ), co, pz, a.k.cz);
-            zp_tz = sj == j && si >= 0 ? lfwd<R>(with(ld(TZZ), a.src.w), co, pz, a.k.cz) : lfwd<R>(ld(TZZ), co, pz, a.k.cz);
+            zp_tz = lfwd<R>(ld(TZZ), co, pz, a.k.cz);
             xp_txz = lfwd<R>(ld(TXZ), co, 1, a.k.cx);
         };
         auto f32 = [&](const float *S) {
@@ -2097,7 +2109,36 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
             sdiffs(f32(S0), dxm_tx, dzm_txz, dzp_tz, dxp_txz);
         }
         exact_stress_terms(dt, axx, azz, axz, dxp_vx, dzm_vz, dxm_vz + dzp_vx, G[0 * P + co], G[1 * P + co]);
-        exact_velocity_terms(dt, bvx, bvz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, G[2 * P + co]);
+        if (BF) {  // S_t + source
+            if (si == i) dxm_tx = fmaf(coef_bwd<R>(sj - j, a.k.cx), a.src.z, dxm_tx);
+            if (sj == j) dzp_tz = fmaf(coef_fwd<R>(si - i, a.k.cz), a.src.w, dzp_tz);
+        }
+        if (BF || !near_src(i, j)) exact_velocity_terms(dt, bvx, bvz, dxm_tx + dzm_txz, dzp_tz + dxp_txz, G[2 * P + co]);
+    }
+    if (BF || !a.add_src) return;
+    // Near the source the differences of S_t with its step's source added to the stress, as the forward step
+    // adds it (in the loop above this took 14 registers and a third of a step's time).
+    __syncthreads();
+    if (threadIdx.x <= 4 * R) {
+        const int e = threadIdx.x, k = e <= 2 * R ? e - R : e <= 3 * R ? e - 3 * R - 1 : e - 3 * R;
+        const int i = e <= 2 * R ? si : si + k, j = e <= 2 * R ? sj + k : sj;
+        if (i < i0 || i >= i0 + TZ || j < j0 || j >= j0 + TX || !in_domain(g, R, i, j)) return;
+        const long long co = cell_off(g, i, j), sc = cell_off(g, si, sj);
+        // lbwd / lfwd of field f, v added at the source cell, one pair of values at a time: few registers
+        auto diff = [&](int f, float v, long long step, const float *c, int fwd) {
+            auto at = [&](int o) {
+                const long long m = co + o * step;
+                const float x = __ldg(S0 + f * P + m);
+                return m == sc ? __fadd_rn(x, v) : x;
+            };
+            float d = c[0] * (at(fwd) - at(fwd - 1));
+#pragma unroll 1
+            for (int q = 1; q < R; ++q) d = fmaf(c[q], at(q + fwd) - at(fwd - 1 - q), d);
+            return d;
+        };
+        const float sx = diff(TXX, a.src.z, 1, a.k.cx, 0) + diff(TXZ, 0.f, g.pitch, a.k.cz, 0);
+        const float sz = diff(TZZ, a.src.w, g.pitch, a.k.cz, 1) + diff(TXZ, 0.f, 1, a.k.cx, 1);
+        exact_velocity_terms(dt, L0[VX * P + co], L0[VZ * P + co], sx, sz, G[2 * P + co]);
     }
 }
 
