@@ -4,7 +4,12 @@
 different grids, record lengths, shot counts and receiver layouts — together
 on one GPU.  Each survey's plan runs on its own CUDA stream, so the step
 kernels of small surveys overlap instead of leaving the GPU idle between
-launches.  Surveys whose plans are not built yet share the free device
+launches.  The plans that a batch builds have the step kernels: a survey whose
+grid fits on chip is faster by itself, with the resident time loops, so a loop
+over ``WavePropagator.misfit_gradient`` beats a batch of such surveys (32
+uneven surveys: 16.9 s one after another, 25.4 s on streams, 25.5 s as one
+graph); a batch pays where grids are too large for them or where one call or
+one graph launch for all surveys is wanted.  Surveys whose plans are not built yet share the free device
 memory in proportion to their every-step storage (cells x steps x shots),
 so the first survey's layout does not take the memory the others need.
 With ``graph=True`` the whole batch (every survey's forward,
@@ -15,8 +20,10 @@ into that graph, whatever their number: the 32-survey uneven batch of the
 benchmark, about 1.8 million launches, runs this way).
 
 The reference evaluates one survey at a time (one ``WavePropagator`` per
-model, wave_propagation.py:594-938); results here are the same as evaluating
-each survey alone with ``WavePropagator.misfit_gradient``.
+model, wave_propagation.py:594-938); results here are those of evaluating each
+survey alone with ``WavePropagator.misfit_gradient``: the same bits where the
+layouts agree, and to rounding of the sums over shots where the memory share or
+the kernels give another number of shots per group.
 """
 import numpy as np
 import torch
@@ -41,7 +48,7 @@ class SurveyBatch:
             W.persist_allowed = False
             if W._plan is not None and W._plan.opts.persist == 1:
                 W._plan = None  # rebuilt on first use, without persistent loops
-            # (a plan with resident loops is kept, and with it the survey's state)
+            # (a plan with resident loops that was built before is kept, and with it the survey's state)
         self._share_memory()
         self.graph = graph
         self._graph = None
@@ -89,6 +96,8 @@ class SurveyBatch:
             return self._run(models, observed, parameterization)
         if self._graph is None:
             self._capture(models, observed, parameterization)
+        for W in self.props:
+            W.plan.raise_if_gave_up()
         with torch.no_grad():
             for (m_buf, o_buf), m, o in zip(self._inputs, models, observed):
                 for k in m_buf:
@@ -96,6 +105,8 @@ class SurveyBatch:
                 for k in o_buf:
                     o_buf[k].copy_(o[k])
         self._graph.replay()
+        for W in self.props:
+            W.plan.watch_device()
         return [(rms.clone(), {k: v.clone() for k, v in g.items()}) for rms, g in self._outputs]
 
     def _capture(self, models, observed, param):

@@ -131,7 +131,7 @@ class Plan:
         """pyfwi_misfit_gradient: observed / adjoint are lists of 5 device
         tensors [nt_ext, ns*nr] or None.  Returns (grad [3, nz, nx], misfit
         0-d float64 tensor, traces [5, nt_ext, ns*nr])."""
-        self._raise_if_gave_up()
+        self.raise_if_gave_up()
         sv = np.ascontiguousarray(src_vals, np.float32).reshape(-1, 4)
         if traces is None:
             traces = torch.empty((5, self.nt_ext, self.ns * self.nr), dtype=torch.float32, device=self.device)
@@ -178,7 +178,7 @@ class Plan:
         self._reported.record(torch.cuda.current_stream(self.device))
         self._watched = True
 
-    def _raise_if_gave_up(self):
+    def raise_if_gave_up(self):
         """Raise NativeError if a resident loop of an earlier call gave up."""
         if not self._watched or torch.cuda.is_current_stream_capturing() or not self._reported.query():
             return
@@ -241,7 +241,7 @@ class Plan:
         return n.value, ms.value, cells.value
 
     def set_model(self, vp, vs, rho, damp_x, damp_z):
-        self._raise_if_gave_up()
+        self.raise_if_gave_up()
         args = [t.to(self.device, torch.float32).contiguous() for t in (vp, vs, rho, damp_x, damp_z)]
         N.check(self.lib.pyfwi_set_model(self.handle, self.ws, self.ws_bytes, *[_ptr(t) for t in args],
                                          _stream(self.device)))
@@ -249,7 +249,7 @@ class Plan:
 
     def forward(self, src_vals, traces=None):
         """Run all shots; returns traces [5, nt_ext, ns*nr] (float32, device)."""
-        self._raise_if_gave_up()
+        self.raise_if_gave_up()
         sv = np.ascontiguousarray(src_vals, np.float32).reshape(-1, 4)
         if traces is None:
             traces = torch.empty((5, self.nt_ext, self.ns * self.nr), dtype=torch.float32, device=self.device)
@@ -265,7 +265,7 @@ class Plan:
         With graph replay on, the residual is copied into buffers the plan
         keeps, so every call presents the same pointers to the captured
         graph."""
-        self._raise_if_gave_up()
+        self.raise_if_gave_up()
         res = []
         for q, r in enumerate(residual):
             if r is None:

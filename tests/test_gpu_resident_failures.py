@@ -122,3 +122,23 @@ def test_receivers_outside_the_grid_add_nothing(adjoint):
         grads.append(plan.gradient([t.contiguous() + 1.0 for t in traces], 1))
         assert plan.frame_check() == 0, persist
     assert torch.equal(*grads)
+
+
+def test_a_replayed_batch_reports_a_loop_that_gave_up():
+    """The graph of a batch whose plan was built with resident loops."""
+    import torch
+    from pyfwi_b200._native import NativeError
+    from pyfwi_b200.batch import SurveyBatch
+    W, model, obs = _setup()
+    batch = SurveyBatch([W], graph=True)
+    clean = {k: v.clone() for k, v in batch.misfit_gradient([model], [obs])[0][1].items()}
+    torch.cuda.synchronize()
+    W.plan.barrier_selftest(20_000_000)
+    batch.misfit_gradient([model], [obs])
+    torch.cuda.synchronize()
+    with pytest.raises(NativeError, match="device error word 3"):
+        for _ in range(3):
+            batch.misfit_gradient([model], [obs])
+            torch.cuda.synchronize()
+    again = batch.misfit_gradient([model], [obs])[0][1]
+    assert all(torch.equal(again[k], clean[k]) for k in clean)
