@@ -142,10 +142,11 @@ typedef struct pyfwi_options {
                                2: resident time loops, one cooperative launch per run of steps
                                and few shots with the wavefield kept on chip, where checkpoint
                                segments hold difference sets in FP32 (store_diffs), or the sets
-                               can be formed from FP32 states (energy terms, reverse checkpoints;
-                               a chunk of sets more in the workspace), or for the exact adjoint
-                               with FP32 states; no overlap is on, every source lies in the update domain, every receiver in the grid and the
-                               grid fits on the SMs (up to about 600,000 cells); the step kernels
+                               can be formed from FP32 states (energy terms, reverse checkpoints: a
+                               chunk of sets, and in reverse mode of reconstructed states, more in
+                               the workspace, at most half of the states kept or 96 MB), or for the exact adjoint
+                               with FP32 states; no overlap is on, every source lies in the
+                               update domain, every receiver in the grid and the grid fits on the SMs (up to about 600,000 cells); the step kernels
                                otherwise, and for a pass that they run faster (many shots of
                                eighth order, many shots with states or checkpoints).  A caller's
                                stream capture takes the resident loops too: graph replays and

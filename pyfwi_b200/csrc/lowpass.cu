@@ -26,7 +26,7 @@
 //
 // What bounds it: a radix-2 transform (24 sweeps over shared memory for 4096
 // points, a barrier each) took 842 us for 8000 traces of 2000 samples, 20 us of
-// which are the memory traffic; four sweeps are left here, and it takes 119 us.
+// which are the memory traffic; four sweeps are left here, and it takes 117 us.
 #include "pyfwi_b200.h"
 
 #include <cuda_runtime.h>

@@ -27,12 +27,14 @@
 // bytes per imaged cell, written forward, read backward).
 //
 // Measured, forward / adjoint per step of all shots, against one launch per
-// step: 500 x 1000 cells and 4 shots 50.8 / 59.2 -> 22.9 / 37.6 us; whole
-// gradients of 100 x 100 cells, 4 shots, 500 steps 7.1 -> 2.6 ms, and of 200 x
-// 400 cells, 10 shots, 1000 steps 48.4 -> 30.7 ms.
+// step: 500 x 1000 cells and 4 shots 50.8 / 59.2 -> 20.9 / 37.0 us; whole
+// gradients of 100 x 100 cells, 4 shots, 500 steps 7.1 -> 2.5 ms, and of 200 x
+// 400 cells, 10 shots, 1000 steps 48.4 -> 29.5 ms.
 //
-// The arithmetic is that of fwd_step / adj_step, operation for operation:
-// the results are the step kernels' bits, whatever the tiling.
+// The arithmetic is that of fwd_step / adj_step / exact_adj_step, operation
+// for operation: the results are the step kernels' bits, whatever the tiling.
+// (After an overflow the same samples are finite; where the damping is zero an
+// infinity stays one here and becomes NaN there.)
 //
 // Every wait is bounded by p.limit_ns of the global timer: a CTA that gives
 // up sets the workspace error word to 3 and stops, and so does every CTA that

@@ -31,8 +31,9 @@ on where a step carries at most 2 M cell-shots; absent, with ``tile`` and
 ``adj_tile`` absent and ``graph`` not True: the resident time loops, which keep
 the wavefield on chip for whole runs of steps, where a grid fits and exact
 checkpoints hold difference sets in FP32, energy terms are asked for or states
-are reconstructed -- the same bits as False -- and for the exact adjoint with
-FP32 states, up to rounding),
+are reconstructed, and for the exact adjoint with FP32 states: the same bits as
+False in the same layout.  Passes that the step kernels run faster keep them:
+many shots of eighth order, of stored states or of reconstructed ones),
 ``overlap`` (exact checkpoints in FP32 with recompute segments: recompute
 segment m - 1 on a second CUDA stream while the adjoint of segment m runs,
 with two segment buffers), ``store`` ('differences', the default: in exact
