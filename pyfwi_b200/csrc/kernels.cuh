@@ -1944,7 +1944,7 @@ __device__ __forceinline__ void exact_products(float dt, float lam, float mu, fl
                                                float &p3)
 {
     const float l2m = __fmaf_rn(2.f, mu, lam);
-    p1 = __fmul_rn(dt, __fmaf_rn(l2m, axx, __fmul_rn(lam, azz)));
+    p1 = __fmul_rn(dt, __fmaf_rn(lam, azz, __fmul_rn(l2m, axx)));
     p2 = __fmul_rn(dt, __fmul_rn(mu, axz));
     p3 = __fmul_rn(dt, __fmaf_rn(lam, axx, __fmul_rn(l2m, azz)));
 }
@@ -1958,7 +1958,7 @@ __device__ __forceinline__ void exact_stress_terms(float dt, float axx, float az
                                                    float &glam, float &gmu)
 {
     glam = __fmaf_rn(__fmul_rn(dt, __fadd_rn(axx, azz)), __fadd_rn(xp, zm), glam);
-    gmu = __fmaf_rn(dt, __fmaf_rn(axz, cross, __fmaf_rn(2.f * axx, xp, __fmul_rn(2.f * azz, zm))), gmu);
+    gmu = __fmaf_rn(dt, __fmaf_rn(axz, cross, __fmaf_rn(2.f * azz, zm, __fmul_rn(2.f * axx, xp))), gmu);
 }
 
 __device__ __forceinline__ void exact_velocity_terms(float dt, float bvx, float bvz, float sx, float sz, float &gb)
@@ -2060,13 +2060,13 @@ __global__ void __launch_bounds__(NTHREADS) exact_adj_step(const __grid_constant
         const float mvx = __ldg(L1 + VX * P + co) - dbwd<R>(p1, ip, 1, a.k.cx) - dbwd<R>(p2, ip, PW, a.k.cz);
         const float mvz = __ldg(L1 + VZ * P + co) - dfwd<R>(p3, ip, PW, a.k.cz) - dfwd<R>(p2, ip, 1, a.k.cx);
         const float bvx = __fmul_rn(damp, mvx), bvz = __fmul_rn(damp, mvz);
-        const float lxx = __ldg(L1 + TXX * P + co), lzz = __ldg(L1 + TZZ * P + co), lxz = __ldg(L1 + TXZ * P + co);
-        const float axx = __fmul_rn(damp, lxx), azz = __fmul_rn(damp, lzz), axz = __fmul_rn(damp, lxz);
+        const float axx = __fmul_rn(damp, __ldg(L1 + TXX * P + co)), azz = __fmul_rn(damp, __ldg(L1 + TZZ * P + co)),
+                    axz = __fmul_rn(damp, __ldg(L1 + TXZ * P + co));
         L0[VX * P + co] = bvx;
         L0[VZ * P + co] = bvz;
-        L0[TXX * P + co] = __fmaf_rn(damp, lxx, -dfwd<R>(q1, iq, 1, a.k.cx));
-        L0[TZZ * P + co] = __fmaf_rn(damp, lzz, -dbwd<R>(q2, iq, QW, a.k.cz));
-        L0[TXZ * P + co] = __fsub_rn(__fmaf_rn(damp, lxz, -dfwd<R>(q1, iq, QW, a.k.cz)), dbwd<R>(q2, iq, 1, a.k.cx));
+        L0[TXX * P + co] = __fsub_rn(axx, dfwd<R>(q1, iq, 1, a.k.cx));
+        L0[TZZ * P + co] = __fsub_rn(azz, dbwd<R>(q2, iq, QW, a.k.cz));
+        L0[TXZ * P + co] = __fsub_rn(__fsub_rn(axz, dfwd<R>(q1, iq, QW, a.k.cz)), dbwd<R>(q2, iq, 1, a.k.cx));
         if (!dom) continue;
         const long long pz = g.pitch;
         // velocity differences of S_{t+1}, stress differences of S_t; ld(f)

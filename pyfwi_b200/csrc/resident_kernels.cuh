@@ -1917,20 +1917,23 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
             for (int r = 0; r < RB; ++r) {
                 z.next(row(r + R - 1));
                 const float4 d = damp4_of(br + r + 2 * R, HX + 4 * bq);
-                float x[12], oz[4], oxz[4], gl[4], gm[4];
+                float x[12], oz[4], oxz[4], gl[4], gm[4], ax[4];
                 xrow<R, false>(x, z.centre(), s_q2 + ot + r * W);  // Dx- Q2
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const float ax = __fmul_rn(f4(d, k), f4(xx[r], k)), az = __fmul_rn(f4(d, k), f4(zz[r], k)), axz = __fmul_rn(f4(d, k), f4(xz[r], k));
+                    ax[k] = __fmul_rn(f4(d, k), f4(xx[r], k));
+                    const float az = __fmul_rn(f4(d, k), f4(zz[r], k)), axz = __fmul_rn(f4(d, k), f4(xz[r], k));
                     gl[k] = f4(glam[r], k);
                     gm[k] = f4(gmu[r], k);
-                    exact_stress_terms(dt, ax, az, axz, f4(q0v[r], k), f4(q1v[r], k), f4(q2v[r], k), gl[k], gm[k]);
-                    oz[k] = __fmaf_rn(f4(d, k), f4(zz[r], k), -z.at(k, a.k.cz));
+                    exact_stress_terms(dt, ax[k], az, axz, f4(q0v[r], k), f4(q1v[r], k), f4(q2v[r], k), gl[k], gm[k]);
+                    oz[k] = __fsub_rn(az, z.at(k, a.k.cz));
                     oxz[k] = xbwd<R>(x, k, a.k.cx);  // taken off after Dz+ Q1
                 }
+                xx[r] = mk4(ax);
                 zz[r] = mk4(oz);
                 glam[r] = mk4(gl);
                 gmu[r] = mk4(gm);
+                xz[r] = times4(d, xz[r]);
                 q2v[r] = mk4(oxz);
             }
         }
@@ -1939,13 +1942,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
             z.next(row(r + R));
-            const float4 d = damp4_of(br + r + 2 * R, HX + 4 * bq);
             float x[12], ox[4], oxz[4];
             xrow<R, true>(x, z.centre(), s_q1 + ot + r * W);  // Dx+ Q1
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                ox[k] = __fmaf_rn(f4(d, k), f4(xx[r], k), -xfwd<R>(x, k, a.k.cx));
-                oxz[k] = __fsub_rn(__fmaf_rn(f4(d, k), f4(xz[r], k), -z.at(k, a.k.cz)), f4(q2v[r], k));
+                ox[k] = __fsub_rn(f4(xx[r], k), xfwd<R>(x, k, a.k.cx));
+                oxz[k] = __fsub_rn(__fsub_rn(f4(xz[r], k), z.at(k, a.k.cz)), f4(q2v[r], k));
             }
             xx[r] = mk4(ox);
             xz[r] = mk4(oxz);
@@ -1957,7 +1959,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) exact_resident(const __grid_co
                 inject(xz[r], t, TXZ, rs[r]);
             }
             float4 p1, p2, p3;
-            products(ld4s(s_lam + 4 * (r * NT + tid)), ld4s(s_mu + 4 * (r * NT + tid)), d, xx[r], zz[r], xz[r], p1, p2, p3);
+            products(ld4s(s_lam + 4 * (r * NT + tid)), ld4s(s_mu + 4 * (r * NT + tid)), damp4_of(br + r + 2 * R, HX + 4 * bq),
+                     xx[r], zz[r], xz[r], p1, p2, p3);
             st4s(s_p1 + ot + r * W, p1);
             st4s(s_p2 + ot + r * W, p2);
             st4s(s_p3 + ot + r * W, p3);
